@@ -7,12 +7,16 @@
 #include <cuda_runtime_api.h>
 #include <torch/extension.h>
 
+#include <stdlib.h>
+#include <string.h>
+
 #include <map>
 #include <memory>
 #include <atomic>
 #include <mutex>
 #include <thread>
 
+#include "kernels/gemv_local.h"
 #include "kernels/launch.h"
 #include "oracle/cpu_reference.h"
 #include "symm/allocator.h"
@@ -616,6 +620,41 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   }, py::arg("x"), py::arg("w"), py::arg("out"), py::arg("workspace"), py::arg("ws_offset"),
      py::arg("timeout_ns"), py::arg("tensor_core") = false, py::arg("num_sms") = 148, py::arg("tagged") = false,
      py::arg("weights_nk") = false);
+
+  // Rank-local x @ w (decode batch): checks, output and launch in one call, because the kernel takes less time
+  // than a Python-side check of its operands.  None when the operands are not what the tcgen05 kernel takes
+  // (or SMR_GEMV_ALGO asks for the CUDA-core kernel): the caller's full path then serves them or says why not.
+  m.def("gemv_local", [](const torch::Tensor& x, const torch::Tensor& w, const c10::optional<torch::Tensor>& out,
+                         bool weights_nk, uint64_t timeout_ns) -> c10::optional<torch::Tensor> {
+    auto ok2d = [](const torch::Tensor& t) { return t.is_cuda() && t.dim() == 2 && t.scalar_type() == torch::kBFloat16; };
+    if (!ok2d(x) || !ok2d(w) || !w.is_contiguous()) return c10::nullopt;
+    const int64_t B = x.size(0), K = x.size(1), N = w.size(weights_nk ? 0 : 1);
+    if (w.size(weights_nk ? 1 : 0) != K || B < 1 || B > 16 || K < 8 || K % 8 != 0 || N < 8 || N % 8 != 0)
+      return c10::nullopt;
+    const int dev = x.get_device();
+    if (w.get_device() != dev) return c10::nullopt;
+    if (out.has_value() && (!ok2d(*out) || !out->is_contiguous() || out->get_device() != dev || out->size(0) != B ||
+                            out->size(1) != N || (uintptr_t)out->data_ptr() % 8 != 0))
+      return c10::nullopt;
+    if (const char* algo = getenv("SMR_GEMV_ALGO"))
+      if (strcmp(algo, "simt") == 0) return c10::nullopt;
+    c10::cuda::CUDAGuard guard(dev);
+    const torch::Tensor xc = x.contiguous();
+    if (((uintptr_t)xc.data_ptr() | (uintptr_t)w.data_ptr()) % 16 != 0) return c10::nullopt;
+    torch::Tensor y = out.has_value() ? *out : at::empty({B, N}, x.options());
+    GemvLocalArgs args{};
+    args.x = xc.data_ptr();
+    args.w = w.data_ptr();
+    args.out = y.data_ptr();
+    args.batch = (int)B; args.K = (int)K; args.N = (int)N;
+    args.weights_nk = weights_nk;
+    args.overlap = true;
+    args.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+    args.timeout_ns = timeout_ns;
+    args.status = status_for(dev);
+    rt_check(launch_gemv_local(args, current_stream(dev)), "gemv");
+    return y;
+  }, py::arg("x"), py::arg("w"), py::arg("out"), py::arg("weights_nk"), py::arg("timeout_ns"));
 
   m.def("matmul_rs_workspace_bytes", &matmul_rs_workspace_bytes);
   m.def("matmul_reduce_scatter", [](torch::Tensor a, torch::Tensor b, torch::Tensor out,

@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include "mbarrier.cuh"
+#include "vec.cuh"
 
 namespace smr {
 
@@ -30,6 +31,16 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
+__device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar,
+                                            int32_t x, int32_t y, int32_t z, int32_t w) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)),
+        "r"(x), "r"(y), "r"(z), "r"(w)
+      : "memory");
+}
+
 // 2-D tile shared -> global, tracked by bulk async-groups.  Parts of the box outside the tensor
 // are not written.  The shared-memory writes that filled the tile must be followed by
 // fence_proxy_async_smem() before the issuing thread is signalled.
@@ -44,6 +55,23 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 }
 __device__ __forceinline__ void st_shared_16(uint32_t smem_addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(smem_addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+
+__device__ __forceinline__ Vec16 ld_shared_16(uint32_t smem_addr) {
+  Vec16 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(smem_addr) : "memory");
+  return v;
+}
+// 16 bytes global -> shared by this thread, tracked by its cp.async groups (generic proxy: follow the wait
+// with fence_proxy_async_smem() before the async proxy reads them).
+__device__ __forceinline__ void cp_async_16(uint32_t smem_addr, const void* gmem_src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr), "l"(gmem_src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 // Untiled bulk copy global -> shared (both 16-byte aligned, size % 16 == 0).

@@ -24,8 +24,8 @@
 // partial [16 b x 128 n] in its own shared memory, the cluster meets, and CTA
 // kh sums the partials of its share of the tile's columns (128 / splits) over
 // the cluster's shared memories (distributed shared memory, split order): the
-// K reduction never touches global memory.  With one rank that sum is the
-// result.  With several, the CTA pushes it into slot `rank` of every rank's
+// K reduction never touches global memory.  (A rank with nobody to reduce with
+// runs gemv_local.cu instead.)  The CTA pushes the sum into slot `rank` of every rank's
 // inbox for those columns, raises the slot's flag (st.release.sys), waits
 // (bounded) for the WS flags of its columns and adds the slots in rank order,
 // so every rank produces the same bits.
@@ -102,16 +102,6 @@ __device__ __forceinline__ uint64_t umma_smem_desc_mn_sw128(uint32_t smem_addr) 
   return d;
 }
 
-__device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
-
 __device__ __forceinline__ void group_sync_128() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // Cluster-wide barrier (every thread of every CTA of the cluster) and a 16-byte load from the
@@ -153,11 +143,7 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
 
   char* my_ws = static_cast<char*>(p.buffers[rank]);
   uint32_t* my_counter = reinterpret_cast<uint32_t*>(my_ws + p.counters_offset) + blockIdx.x;
-  uint32_t epoch = 0, parity = 0;
-  if (ws > 1) {                          // a world of one exchanges nothing: no call number needed
-    epoch = ld_relaxed_gpu(my_counter) + 1u;
-    parity = epoch & 1u;
-  }
+  const uint32_t epoch = ld_relaxed_gpu(my_counter) + 1u, parity = epoch & 1u;
 
   const int kb_total = (p.K + kBK - 1) / kBK;
   const int kb_per = (kb_total + p.ksplit - 1) / p.ksplit;
@@ -207,7 +193,7 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
   const int etid = (int)threadIdx.x - 64;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t stage = (uint32_t)(n_first % kStages), phase = n_first == kStages ? 1u : 0u;
       for (int i = n_first; i < n_kb; ++i) {
         if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.timeout_ns)) {
@@ -220,7 +206,7 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // kind::f16, bf16 x bf16 -> fp32, A MN-major (bit 15), B K-major, M = 128, N = 16
       constexpr uint32_t idesc = umma_idesc_bf16_f32(kTileN, kBatchN) | (kWeightsNK ? 0u : (1u << 15));
       uint32_t stage = 0, phase = 0;
@@ -279,130 +265,114 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     // item = (batch row b, four consecutive columns of this CTA's share); at most 16 * 32 items
     const int n_items = p.batch * (share / 4);
     const uint32_t part_addr = smem_u32(part);
-    if (ws == 1) {
-      for (int item = etid; item < n_items; item += 128) {
-        const int b = item / (share / 4), c = c_share0 + (item % (share / 4)) * 4;
-        if (n0 + c >= p.N) continue;                                      // N % 8 == 0
-        float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int j = 0; j < p.ksplit; ++j) {                              // split order: deterministic
-          const float4 v = ld_dsmem_f4(part_addr + (uint32_t)(b * kTileN + c) * 4u, (uint32_t)j);
-          s4.x += v.x; s4.y += v.y; s4.z += v.z; s4.w += v.w;
+    const size_t slot_stride = (size_t)kBatchN * p.N;                   // floats (or words) per slot
+    const size_t parity_off = (size_t)parity * ws * slot_stride;
+    // ---- push this rank's sum of the share into slot `rank` of every rank's inbox ----
+    for (int item = etid; item < n_items && !failed; item += 128) {
+      const int b = item / (share / 4), c = c_share0 + (item % (share / 4)) * 4;
+      if (n0 + c >= p.N) continue;
+      float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int j = 0; j < p.ksplit; ++j) {
+        const float4 v = ld_dsmem_f4(part_addr + (uint32_t)(b * kTileN + c) * 4u, (uint32_t)j);
+        s4.x += v.x; s4.y += v.y; s4.z += v.z; s4.w += v.w;
+      }
+      const size_t off = parity_off + (size_t)rank * slot_stride + (size_t)b * p.N + n0 + c;
+      if constexpr (kTagged) {
+        const Vec16 w0{__float_as_uint(s4.x), epoch, __float_as_uint(s4.y), epoch};
+        const Vec16 w1{__float_as_uint(s4.z), epoch, __float_as_uint(s4.w), epoch};
+        for (int j = 1; j <= ws; ++j) {                                 // own inbox last
+          int peer = rank + j;
+          if (peer >= ws) peer -= ws;
+          char* dst = static_cast<char*>(p.buffers[peer]) + p.inbox_offset + off * 8;
+          st_16(dst, w0);
+          st_16(dst + 16, w1);
         }
+      } else {
+        const Vec16 v{__float_as_uint(s4.x), __float_as_uint(s4.y), __float_as_uint(s4.z), __float_as_uint(s4.w)};
+        for (int j = 1; j <= ws; ++j) {
+          int peer = rank + j;
+          if (peer >= ws) peer -= ws;
+          float* inbox = reinterpret_cast<float*>(static_cast<char*>(p.buffers[peer]) + p.inbox_offset);
+          st_16(inbox + off, v);
+        }
+      }
+    }
+    if constexpr (kTagged) {
+      // ---- poll the own inbox until every rank's words for an item carry this call's number ----
+      const char* inbox = my_ws + p.inbox_offset;
+      for (int item = etid; item < n_items && !failed && flags_ok; item += 128) {
+        const int b = item / (share / 4), c = c_share0 + (item % (share / 4)) * 4;
+        if (n0 + c >= p.N) continue;
+        float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        Deadline d(p.timeout_ns);
+        for (int sl = 0; sl < ws; ++sl) {                               // rank order: same bits on every rank
+          const char* src = inbox + (parity_off + (size_t)sl * slot_stride + (size_t)b * p.N + n0 + c) * 8;
+          Vec16 a, g;
+          bool got = false;
+          while (!got) {
+            asm volatile("ld.relaxed.sys.global.v4.u32 {%0,%1,%2,%3}, [%4];"
+                         : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w) : "l"(src) : "memory");
+            asm volatile("ld.relaxed.sys.global.v4.u32 {%0,%1,%2,%3}, [%4];"
+                         : "=r"(g.x), "=r"(g.y), "=r"(g.z), "=r"(g.w) : "l"(src + 16) : "memory");
+            got = a.y == epoch && a.w == epoch && g.y == epoch && g.w == epoch;
+            if (!got && !d.alive()) {
+              report_status(p.status, kTimeoutFlag, rank, tile, sl, kWhereGemvArrive, epoch);
+              flags_ok = 0;
+              break;
+            }
+          }
+          if (!got) break;
+          s4.x += __uint_as_float(a.x); s4.y += __uint_as_float(a.z);
+          s4.z += __uint_as_float(g.x); s4.w += __uint_as_float(g.z);
+        }
+        if (!flags_ok) break;
         uint2 o;
         o.x = pack_bf16x2(s4.x, s4.y);
         o.y = pack_bf16x2(s4.z, s4.w);
         *reinterpret_cast<uint2*>(p.out + (size_t)b * p.N + n0 + c) = o;
       }
     } else {
-      const size_t slot_stride = (size_t)kBatchN * p.N;                   // floats (or words) per slot
-      const size_t parity_off = (size_t)parity * ws * slot_stride;
-      // ---- push this rank's sum of the share into slot `rank` of every rank's inbox ----
-      for (int item = etid; item < n_items && !failed; item += 128) {
-        const int b = item / (share / 4), c = c_share0 + (item % (share / 4)) * 4;
-        if (n0 + c >= p.N) continue;
-        float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int j = 0; j < p.ksplit; ++j) {
-          const float4 v = ld_dsmem_f4(part_addr + (uint32_t)(b * kTileN + c) * 4u, (uint32_t)j);
-          s4.x += v.x; s4.y += v.y; s4.z += v.z; s4.w += v.w;
-        }
-        const size_t off = parity_off + (size_t)rank * slot_stride + (size_t)b * p.N + n0 + c;
-        if constexpr (kTagged) {
-          const Vec16 w0{__float_as_uint(s4.x), epoch, __float_as_uint(s4.y), epoch};
-          const Vec16 w1{__float_as_uint(s4.z), epoch, __float_as_uint(s4.w), epoch};
-          for (int j = 1; j <= ws; ++j) {                                 // own inbox last
-            int peer = rank + j;
-            if (peer >= ws) peer -= ws;
-            char* dst = static_cast<char*>(p.buffers[peer]) + p.inbox_offset + off * 8;
-            st_16(dst, w0);
-            st_16(dst + 16, w1);
-          }
-        } else {
-          const Vec16 v{__float_as_uint(s4.x), __float_as_uint(s4.y), __float_as_uint(s4.z), __float_as_uint(s4.w)};
-          for (int j = 1; j <= ws; ++j) {
-            int peer = rank + j;
-            if (peer >= ws) peer -= ws;
-            float* inbox = reinterpret_cast<float*>(static_cast<char*>(p.buffers[peer]) + p.inbox_offset);
-            st_16(inbox + off, v);
+      group_sync_128();   // the group's pushes precede the releases below
+      const size_t flag_idx = ((size_t)parity * p.tiles + tile) * kFlagStride + (size_t)kh * ws;
+      if (etid < ws && !failed) {
+        uint32_t* peer_flags = reinterpret_cast<uint32_t*>(static_cast<char*>(p.buffers[etid]) + p.flags_offset);
+        st_release_sys(peer_flags + flag_idx + rank, epoch);
+      }
+      if (etid < ws) {
+        const uint32_t* mine = reinterpret_cast<const uint32_t*>(my_ws + p.flags_offset) + flag_idx + etid;
+        Deadline d(p.timeout_ns);
+        while (ld_acquire_sys(mine) != epoch) {
+          if (!d.alive()) {
+            report_status(p.status, kTimeoutFlag, rank, tile, etid, kWhereGemvArrive, epoch);
+            flags_ok = 0;
+            break;
           }
         }
       }
-      if constexpr (kTagged) {
-        // ---- poll the own inbox until every rank's words for an item carry this call's number ----
-        const char* inbox = my_ws + p.inbox_offset;
-        for (int item = etid; item < n_items && !failed && flags_ok; item += 128) {
+      group_sync_128();
+      if (flags_ok && !failed) {
+        const float* inbox = reinterpret_cast<const float*>(my_ws + p.inbox_offset) + parity_off;
+        for (int item = etid; item < n_items; item += 128) {
           const int b = item / (share / 4), c = c_share0 + (item % (share / 4)) * 4;
           if (n0 + c >= p.N) continue;
+          const float* src = inbox + (size_t)b * p.N + n0 + c;
           float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
-          Deadline d(p.timeout_ns);
-          for (int sl = 0; sl < ws; ++sl) {                               // rank order: same bits on every rank
-            const char* src = inbox + (parity_off + (size_t)sl * slot_stride + (size_t)b * p.N + n0 + c) * 8;
-            Vec16 a, g;
-            bool got = false;
-            while (!got) {
-              asm volatile("ld.relaxed.sys.global.v4.u32 {%0,%1,%2,%3}, [%4];"
-                           : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w) : "l"(src) : "memory");
-              asm volatile("ld.relaxed.sys.global.v4.u32 {%0,%1,%2,%3}, [%4];"
-                           : "=r"(g.x), "=r"(g.y), "=r"(g.z), "=r"(g.w) : "l"(src + 16) : "memory");
-              got = a.y == epoch && a.w == epoch && g.y == epoch && g.w == epoch;
-              if (!got && !d.alive()) {
-                report_status(p.status, kTimeoutFlag, rank, tile, sl, kWhereGemvArrive, epoch);
-                flags_ok = 0;
-                break;
+          for (int sl0 = 0; sl0 < ws; sl0 += 8) {                       // 8 independent loads in flight
+            Vec16 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              if (sl0 + u < ws) v[u] = ld_16_stream(src + (size_t)(sl0 + u) * slot_stride);
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              if (sl0 + u < ws) {
+                s4.x += __uint_as_float(v[u].x); s4.y += __uint_as_float(v[u].y);
+                s4.z += __uint_as_float(v[u].z); s4.w += __uint_as_float(v[u].w);
               }
-            }
-            if (!got) break;
-            s4.x += __uint_as_float(a.x); s4.y += __uint_as_float(a.z);
-            s4.z += __uint_as_float(g.x); s4.w += __uint_as_float(g.z);
           }
-          if (!flags_ok) break;
           uint2 o;
           o.x = pack_bf16x2(s4.x, s4.y);
           o.y = pack_bf16x2(s4.z, s4.w);
           *reinterpret_cast<uint2*>(p.out + (size_t)b * p.N + n0 + c) = o;
-        }
-      } else {
-        group_sync_128();   // the group's pushes precede the releases below
-        const size_t flag_idx = ((size_t)parity * p.tiles + tile) * kFlagStride + (size_t)kh * ws;
-        if (etid < ws && !failed) {
-          uint32_t* peer_flags = reinterpret_cast<uint32_t*>(static_cast<char*>(p.buffers[etid]) + p.flags_offset);
-          st_release_sys(peer_flags + flag_idx + rank, epoch);
-        }
-        if (etid < ws) {
-          const uint32_t* mine = reinterpret_cast<const uint32_t*>(my_ws + p.flags_offset) + flag_idx + etid;
-          Deadline d(p.timeout_ns);
-          while (ld_acquire_sys(mine) != epoch) {
-            if (!d.alive()) {
-              report_status(p.status, kTimeoutFlag, rank, tile, etid, kWhereGemvArrive, epoch);
-              flags_ok = 0;
-              break;
-            }
-          }
-        }
-        group_sync_128();
-        if (flags_ok && !failed) {
-          const float* inbox = reinterpret_cast<const float*>(my_ws + p.inbox_offset) + parity_off;
-          for (int item = etid; item < n_items; item += 128) {
-            const int b = item / (share / 4), c = c_share0 + (item % (share / 4)) * 4;
-            if (n0 + c >= p.N) continue;
-            const float* src = inbox + (size_t)b * p.N + n0 + c;
-            float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int sl0 = 0; sl0 < ws; sl0 += 8) {                       // 8 independent loads in flight
-              Vec16 v[8];
-#pragma unroll
-              for (int u = 0; u < 8; ++u)
-                if (sl0 + u < ws) v[u] = ld_16_stream(src + (size_t)(sl0 + u) * slot_stride);
-#pragma unroll
-              for (int u = 0; u < 8; ++u)
-                if (sl0 + u < ws) {
-                  s4.x += __uint_as_float(v[u].x); s4.y += __uint_as_float(v[u].y);
-                  s4.z += __uint_as_float(v[u].z); s4.w += __uint_as_float(v[u].w);
-                }
-            }
-            uint2 o;
-            o.x = pack_bf16x2(s4.x, s4.y);
-            o.y = pack_bf16x2(s4.z, s4.w);
-            *reinterpret_cast<uint2*>(p.out + (size_t)b * p.N + n0 + c) = o;
-          }
         }
       }
     }
@@ -415,7 +385,7 @@ gemv_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
   __syncthreads();
   tcgen05_fence_after_thread_sync();
   if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
-  if (ws > 1 && threadIdx.x == 0) *my_counter = epoch;   // this CTA has made its call; read by its next launch
+  if (threadIdx.x == 0) *my_counter = epoch;   // this CTA has made its call; read by its next launch
   // no CTA of the cluster leaves while another may still read its shared memory
   __syncwarp();
   cluster_barrier();
@@ -452,14 +422,11 @@ int launch_gemv_tc(Kernel kernel, const CUtensorMap& tw, const CUtensorMap& tx, 
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTotal);
   if (e != cudaSuccess) return (int)e;
   // The largest split (cluster size) not above the planned one whose clusters are all resident at
-  // once: one wave streams the weights fastest, and with several ranks it is required, because the
-  // CTAs of a tile wait for the same tile's CTAs on the peers (every rank arrives at the same split:
-  // same shape, same GPU).  A world of one whose tiles alone exceed the GPU runs in waves.
+  // once: the CTAs of a tile wait for the same tile's CTAs on the peers (every rank arrives at the
+  // same split: same shape, same GPU).
   int ks = p.ksplit;
   while (ks > 1 && check_co_resident(kernel, p.tiles * ks, kThreads, kSmemTotal, ks) != 0) ks >>= 1;
-  if (p.world_size > 1) {
-    if (int rc = check_co_resident(kernel, p.tiles * ks, kThreads, kSmemTotal, ks)) return rc;
-  }
+  if (int rc = check_co_resident(kernel, p.tiles * ks, kThreads, kSmemTotal, ks)) return rc;
   p.ksplit = ks;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(p.tiles * p.ksplit), 1, 1);
@@ -500,7 +467,8 @@ size_t gemv_tc_workspace_bytes(int N, int K, int world_size, int num_sms, size_t
 }
 
 int launch_gemv_all_reduce_tc(const GemvArgs& a, int num_sms, cudaStream_t stream, bool tagged, bool weights_nk) {
-  if (a.batch < 1 || a.batch > kBatchN || a.N % 8 != 0 || a.K % 8 != 0 || a.ws_offset != 0)
+  if (a.batch < 1 || a.batch > kBatchN || a.N % 8 != 0 || a.K % 8 != 0 || a.ws_offset != 0 ||
+      a.pv.world_size < 2)
     return cudaErrorInvalidValue;
   GemvTcParams p{};
   p.out = static_cast<__nv_bfloat16*>(a.out);
@@ -527,125 +495,3 @@ int launch_gemv_all_reduce_tc(const GemvArgs& a, int num_sms, cudaStream_t strea
 }
 
 }  // namespace smr
-
-// ---------------------------------------------------------------------------
-// Allocation-free C entry point (see gemv_noalloc.h).  The global memory that the
-// kernel above needs besides its operands lives in this array: offset 0 holds the
-// one-entry "workspace base of every rank" table the kernel reads, offset 64 the
-// 32-byte Status record its bounded waits report into; a (here unused) workspace
-// would start at offset 256.  In a world of one the K splits of a tile meet in
-// shared memory, so nothing else is kept in global memory between or during calls.
-// ---------------------------------------------------------------------------
-#include <mutex>
-#include <stdio.h>
-
-#include "gemv_noalloc.h"
-
-namespace {
-
-static __device__ __align__(256) unsigned char g_gemv_noalloc_scratch[SMR_GEMV_NOALLOC_SCRATCH_BYTES];
-
-constexpr int kMaxDevices = 64;
-std::mutex g_noalloc_mu;
-unsigned char* g_noalloc_base[kMaxDevices] = {};   // device address of the array, per device
-int g_noalloc_sms[kMaxDevices] = {};
-constexpr size_t kNoallocStatusOffset = 64;
-
-int noalloc_fail(int code, char* err, int err_len, const char* what, const char* detail = "") {
-  if (err != nullptr && err_len > 0) snprintf(err, (size_t)err_len, "smr_gemv_bf16_noalloc: %s%s", what, detail);
-  return code;
-}
-
-}  // namespace
-
-extern "C" int smr_gemv_bf16_noalloc(const void* x, const void* w, void* out, int batch, int K, int N,
-                                     void* stream_ptr, char* err, int err_len) {
-  using namespace smr;
-  if (batch < 1 || batch > SMR_GEMV_NOALLOC_MAX_BATCH)
-    return noalloc_fail(1, err, err_len, "batch must be between 1 and 16");
-  if (N < 8 || N > SMR_GEMV_NOALLOC_MAX_N || N % 8 != 0)
-    return noalloc_fail(1, err, err_len, "N must be a multiple of 8 and at most 8192 (the limit of this entry point)");
-  if (K < 8 || K % 8 != 0) return noalloc_fail(1, err, err_len, "K must be a positive multiple of 8");
-  if (x == nullptr || w == nullptr || out == nullptr || ((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) % 16 != 0)
-    return noalloc_fail(2, err, err_len, "x, w and out must be non-null and 16-byte aligned");
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-
-  int dev = -1;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return noalloc_fail(3, err, err_len, "cudaGetDevice: ", cudaGetErrorString(e));
-  if (dev < 0 || dev >= kMaxDevices) return noalloc_fail(3, err, err_len, "device ordinal out of range");
-  unsigned char* base;
-  int sms;
-  {
-    // Once per device, with that device current: the array's name is only a
-    // host-side handle; the kernel needs the address the symbol has on THIS GPU.
-    std::lock_guard<std::mutex> lock(g_noalloc_mu);
-    if (g_noalloc_base[dev] == nullptr) {
-      void* p = nullptr;
-      e = cudaGetSymbolAddress(&p, g_gemv_noalloc_scratch);
-      if (e != cudaSuccess) return noalloc_fail(3, err, err_len, "cudaGetSymbolAddress: ", cudaGetErrorString(e));
-      void* ws_base = static_cast<unsigned char*>(p) + 256;
-      e = cudaMemcpy(p, &ws_base, sizeof(void*), cudaMemcpyHostToDevice);   // the one-entry base table
-      if (e != cudaSuccess) return noalloc_fail(3, err, err_len, "cudaMemcpy(base table): ", cudaGetErrorString(e));
-      int n = 0;
-      e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-      if (e != cudaSuccess) return noalloc_fail(3, err, err_len, "cudaDeviceGetAttribute: ", cudaGetErrorString(e));
-      g_noalloc_sms[dev] = n;
-      g_noalloc_base[dev] = static_cast<unsigned char*>(p);
-    }
-    base = g_noalloc_base[dev];
-    sms = g_noalloc_sms[dev];
-  }
-
-  GemvTcParams p{};
-  p.out = static_cast<__nv_bfloat16*>(out);
-  p.batch = batch; p.K = K; p.N = N;
-  p.rank = 0; p.world_size = 1;
-  p.buffers = reinterpret_cast<void* const*>(base);
-  p.timeout_ns = 2000000000ull;
-  p.status = reinterpret_cast<Status*>(base + kNoallocStatusOffset);
-  // tiles and K splits of this shape; the offsets describe a workspace that a world of one never touches
-  gemv_tc_workspace_bytes(N, K, 1, sms, &p.flags_offset, &p.inbox_offset, &p.tiles, &p.ksplit, false,
-                          &p.counters_offset);
-  CUtensorMap tw, tx;
-  try {
-    if (encode(&tw, w, (uint64_t)N, (uint64_t)K, 64, kBK) || encode(&tx, x, (uint64_t)K, (uint64_t)batch, kBK, kBatchN))
-      return noalloc_fail(3, err, err_len, "cuTensorMapEncodeTiled rejected the operands");
-  } catch (const std::exception& ex) {
-    return noalloc_fail(3, err, err_len, "CUDA driver: ", ex.what());
-  }
-  int rc = launch_gemv_tc(gemv_tc_kernel<false>, tw, tx, p, stream);
-  if (rc != 0) return noalloc_fail(3, err, err_len, "kernel launch: ", cudaGetErrorString((cudaError_t)rc));
-  return 0;
-}
-
-extern "C" int smr_gemv_bf16_noalloc_status(void* stream_ptr, unsigned int record[6], char* err, int err_len) {
-  using namespace smr;
-  int dev = -1;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return noalloc_fail(3, err, err_len, "cudaGetDevice: ", cudaGetErrorString(e));
-  if (dev < 0 || dev >= kMaxDevices) return noalloc_fail(3, err, err_len, "device ordinal out of range");
-  unsigned char* base;
-  {
-    std::lock_guard<std::mutex> lock(g_noalloc_mu);
-    base = g_noalloc_base[dev];
-  }
-  if (record != nullptr)
-    for (int i = 0; i < 6; ++i) record[i] = 0u;
-  if (base == nullptr) return 0;                 // no call on this device yet: nothing can have failed
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  e = cudaStreamSynchronize(stream);
-  if (e != cudaSuccess) return noalloc_fail(3, err, err_len, "cudaStreamSynchronize: ", cudaGetErrorString(e));
-  Status st{};
-  e = cudaMemcpy(&st, base + kNoallocStatusOffset, sizeof(Status), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return noalloc_fail(3, err, err_len, "cudaMemcpy(status): ", cudaGetErrorString(e));
-  if (record != nullptr) {
-    record[0] = st.code; record[1] = st.rank; record[2] = st.block;
-    record[3] = st.peer; record[4] = st.where; record[5] = st.aux;
-  }
-  if (st.code == kOk) return 0;
-  e = cudaMemset(base + kNoallocStatusOffset, 0, sizeof(Status));    // reported once
-  if (e != cudaSuccess) return noalloc_fail(3, err, err_len, "cudaMemset(status): ", cudaGetErrorString(e));
-  return noalloc_fail(4, err, err_len, "a wait inside an earlier call ran out after 2 s (the CTAs of the kernel were "
-                                       "not all resident at once?); that call left `out` unwritten");
-}

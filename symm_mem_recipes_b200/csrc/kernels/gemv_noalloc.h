@@ -28,13 +28,11 @@
 //  * x is [batch, K], w is [K, N], out is [batch, N]; contiguous bf16 in device
 //    memory of the current device, 16-byte aligned.  The caller owns them.
 //  * The first call on each device resolves the device address of the array
-//    (cudaGetSymbolAddress) and writes one pointer into it with a blocking
-//    copy.  Make that first call before any stream capture and outside any
-//    region that must not synchronise.  Later calls only enqueue work on
-//    `stream`.
+//    (cudaGetSymbolAddress) and the launch limits of the kernel.  Make that first
+//    call before any stream capture.  Later calls only enqueue work on `stream`.
 //  * No call allocates: no cudaMalloc, no cudaFree, no framework allocator.
 //  * All calls on a device share the one array, which keeps whatever the
-//    previous call left in it (the pointer table, and the status record of a
+//    previous call left in it (the status record of a
 //    failed call until it is queried).  Two calls that overlap in time on the
 //    same GPU — different streams, or two host threads — would share the status
 //    record; order them on one stream or with events.

@@ -50,6 +50,12 @@ def _workspace(batch_tile: int, N: int, K: int, device: torch.device, group, ten
     return t
 
 
+def _gemv_local(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor], weights_nk: bool,
+                timeout_ms: int) -> Optional[torch.Tensor]:
+    """The rank-local tcgen05 kernel, or None when these operands are not for it."""
+    return C.gemv_local(x, w, out, weights_nk, timeout_ms * 1_000_000)
+
+
 @traced("smr.gemv_all_reduce")
 def gemv_all_reduce(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
                     group=None, timeout_ms: int = _TIMEOUT_MS, algo: Optional[str] = None,
@@ -69,6 +75,10 @@ def gemv_all_reduce(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor
     `weights_nk=True`: `w` is [N, K] (K contiguous), the layout
     `matmul_reduce_scatter` takes, so that one copy of a row-parallel weight
     serves prefill and decode (tcgen05 kernels only)."""
+    if x.is_cuda and algo != "simt" and (group is _LOCAL or not dist.is_initialized() or dist.get_world_size(group) == 1):
+        y = _gemv_local(x, w, out, weights_nk, timeout_ms) if algo in (None, "tc", "tc_tagged") else None
+        if y is not None:
+            return y
     k_dim, n_dim = (1, 0) if weights_nk else (0, 1)
     if x.dim() != 2 or w.dim() != 2 or x.shape[1] != w.shape[k_dim]:
         raise SymmMemError("need x[B, K] and w[K, N]" + (" given as [N, K]" if weights_nk else ""))
@@ -102,7 +112,12 @@ def gemv(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, w
     """Rank-local `x @ w` for a decode batch (1..16 rows) on the same kernels as `gemv_all_reduce`, with
     nobody to reduce with: the column-parallel projections of a decode step (QKV, gate / up), whose
     weights are streamed once from HBM.  `weights_nk=True`: `w` is [N, K], the layout of the prefill
-    GEMMs' B operand.  Not collective; its scratch is a private world of one."""
+    GEMMs' B operand.  Not collective.  Operands the tcgen05 kernel does not take go through
+    `gemv_all_reduce` in a private world of one."""
+    if x.is_cuda:
+        y = _gemv_local(x, w, out, weights_nk, timeout_ms)
+        if y is not None:
+            return y
     return gemv_all_reduce(x, w, out, group=_LOCAL, timeout_ms=timeout_ms, weights_nk=weights_nk)
 
 
