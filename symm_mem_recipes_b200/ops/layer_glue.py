@@ -95,6 +95,18 @@ def silu_mul(gate_up: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch
 _attn_scratch: dict[tuple, torch.Tensor] = {}
 
 
+def attention_scratch(k_cache: torch.Tensor) -> torch.Tensor:
+    """Scratch of the decode attention kernel for caches of this shape, kept between calls."""
+    B, s_max, hkv, D = k_cache.shape
+    key = (k_cache.device.type, k_cache.device.index, B, hkv, D, s_max)
+    scratch = _attn_scratch.get(key)
+    if scratch is None:
+        scratch = torch.zeros(C.decode_attention_scratch_bytes(B, hkv, D, s_max), dtype=torch.uint8,
+                              device=k_cache.device)
+        _attn_scratch[key] = scratch
+    return scratch
+
+
 @traced("smr.decode_attention_")
 def decode_attention_(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, n_q_heads: int,
                       pos: Union[int, torch.Tensor], out: Optional[torch.Tensor] = None,
@@ -126,11 +138,7 @@ def decode_attention_(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.T
         raise SymmMemError("rope_theta must be 0 (no rotation) or larger than 1")
     if out is None:
         out = torch.empty(B, n_q_heads * D, dtype=torch.bfloat16, device=qkv.device)
-    key = (qkv.device.type, qkv.device.index, B, hkv, D, s_max)
-    scratch = _attn_scratch.get(key)
-    if scratch is None:
-        scratch = torch.zeros(C.decode_attention_scratch_bytes(B, hkv, D, s_max), dtype=torch.uint8, device=qkv.device)
-        _attn_scratch[key] = scratch
+    scratch = attention_scratch(k_cache)
     if isinstance(pos, torch.Tensor):
         if pos.dtype != torch.int32 or pos.numel() != 1 or pos.device != qkv.device:
             raise SymmMemError("a position tensor must be int32, of one element, on qkv's device")
