@@ -63,6 +63,35 @@ py::tuple read_status(int device) {
 
 cudaStream_t current_stream(int device) { return c10::cuda::getCurrentCUDAStream(device).stream(); }
 
+// ---- which symmetric allocation an address belongs to ----------------------
+// Looked up on every all-reduce, so it lives here and not in a Python dictionary: an ordered map from payload
+// base to allocation.  Entries die with their allocation (weak pointers, pruned on insertion).
+std::mutex g_allocs_mu;
+std::map<char*, std::weak_ptr<CudaSymmAllocation>> g_allocs;
+
+std::shared_ptr<CudaSymmAllocation> new_cuda_allocation(int device, size_t nbytes) {
+  auto a = std::make_shared<CudaSymmAllocation>(device, nbytes);
+  std::lock_guard<std::mutex> lock(g_allocs_mu);
+  for (auto it = g_allocs.begin(); it != g_allocs.end();) it = it->second.expired() ? g_allocs.erase(it) : std::next(it);
+  g_allocs[static_cast<char*>(a->local_ptr())] = a;
+  return a;
+}
+
+// The rendezvoused allocation whose payload holds [p, p + nbytes), or nullptr.
+std::shared_ptr<CudaSymmAllocation> allocation_of(const void* p, size_t nbytes) {
+  char* q = static_cast<char*>(const_cast<void*>(p));
+  std::shared_ptr<CudaSymmAllocation> a;
+  {
+    std::lock_guard<std::mutex> lock(g_allocs_mu);
+    auto it = g_allocs.upper_bound(q);
+    if (it == g_allocs.begin()) return nullptr;
+    a = std::prev(it)->second.lock();
+  }
+  if (a == nullptr || a->local_ptr() == nullptr || !a->rendezvoused()) return nullptr;
+  char* base = static_cast<char*>(a->local_ptr());
+  return q >= base && q + nbytes <= base + a->payload_bytes() ? a : nullptr;
+}
+
 PeerView view_of(const CudaSymmAllocation& a) {
   TORCH_CHECK(a.rendezvoused(), "symmetric allocation has not been rendezvoused");
   PeerView pv;
@@ -215,7 +244,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
            });
 
   py::class_<CudaSymmAllocation, std::shared_ptr<CudaSymmAllocation>>(m, "CudaSymmAllocation")
-      .def(py::init<int, size_t>())
+      .def(py::init(&new_cuda_allocation))
       .def_property_readonly("device", &CudaSymmAllocation::device)
       .def_property_readonly("payload_bytes", &CudaSymmAllocation::payload_bytes)
       .def_property_readonly("block_bytes", &CudaSymmAllocation::block_bytes)
@@ -450,6 +479,29 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
              "one_shot_all_reduce");
   }, py::arg("alloc"), py::arg("offset_bytes"), py::arg("out"), py::arg("numel"), py::arg("max_blocks"),
      py::arg("exit_barrier"), py::arg("timeout_ns"), py::arg("write_back") = false);
+  // The same for a tensor of an allocation that has been rendezvoused already: looks the allocation up, makes the
+  // output and launches.  None when it is not such a call: the caller's full path then serves it or raises.
+  m.def("one_shot_all_reduce_of", [](const torch::Tensor& t, const c10::optional<torch::Tensor>& out, int max_blocks,
+                                     bool exit_barrier, bool write_back,
+                                     uint64_t timeout_ns) -> c10::optional<torch::Tensor> {
+    auto ok = [](const torch::Tensor& x) {
+      return x.is_cuda() && x.is_contiguous() && x.scalar_type() == torch::kBFloat16;
+    };
+    if (!ok(t) || t.numel() % 8 != 0) return c10::nullopt;
+    if (out.has_value() && (!ok(*out) || out->numel() != t.numel() || (uintptr_t)out->data_ptr() % 16 != 0))
+      return c10::nullopt;
+    const auto a = allocation_of(t.data_ptr(), t.nbytes());
+    if (a == nullptr) return c10::nullopt;
+    const size_t offset = (size_t)(static_cast<char*>(t.data_ptr()) - static_cast<char*>(a->local_ptr()));
+    if (offset % 16 != 0) return c10::nullopt;
+    c10::cuda::CUDAGuard guard(a->device());
+    torch::Tensor y = out.has_value() ? *out : at::empty_like(t);
+    rt_check(launch_one_shot_all_reduce(view_of(*a), ptrs_of(*a), offset, y.data_ptr(), (size_t)t.numel(), max_blocks,
+                                        exit_barrier, write_back, timeout_ns, status_for(a->device()),
+                                        current_stream(a->device())), "one_shot_all_reduce");
+    return y;
+  }, py::arg("t"), py::arg("out"), py::arg("max_blocks"), py::arg("exit_barrier"), py::arg("write_back"),
+     py::arg("timeout_ns"));
   m.def("ll_all_reduce_workspace_bytes", &ll_all_reduce_workspace_bytes);
   m.def("ll_all_reduce", [](const std::shared_ptr<CudaSymmAllocation>& workspace, torch::Tensor in,
                             torch::Tensor out, int64_t capacity_numel, int max_blocks, uint64_t timeout_ns) {

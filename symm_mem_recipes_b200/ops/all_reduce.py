@@ -48,11 +48,15 @@ def one_shot_all_reduce(t: torch.Tensor, *, exit_barrier: bool = False,
     group proves it), or pass `exit_barrier=True`.  `write_back=True` (implies
     the exit barrier) also stores the sum into `t` once all peers have read it.
     """
+    t_ns = config.timeout_ms * 1_000_000
+    exit_barrier = exit_barrier or write_back
+    if t.is_cuda:
+        y = C.one_shot_all_reduce_of(t, out, config.one_shot_max_blocks, exit_barrier, write_back, t_ns)
+        if y is not None:
+            return y
     hdl, offset = _prepare(t)
     if out is None:
         out = torch.empty_like(t)
-    t_ns = config.timeout_ms * 1_000_000
-    exit_barrier = exit_barrier or write_back
     if hdl.kind == "cuda":
         C.one_shot_all_reduce(hdl.native, offset, out, t.numel(), config.one_shot_max_blocks,
                               exit_barrier, t_ns, write_back)
