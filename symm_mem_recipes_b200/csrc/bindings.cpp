@@ -49,6 +49,8 @@ Status* status_for(int device) {
   return s;
 }
 
+void clear_tail_counters(int device);
+
 // Synchronises the device, returns (code, rank, block, peer, where, aux) and
 // clears the record.
 py::tuple read_status(int device) {
@@ -57,11 +59,59 @@ py::tuple read_status(int device) {
   Status h{};
   rt_check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
   rt_check(cudaMemcpy(&h, s, sizeof(Status), cudaMemcpyDeviceToHost), "cudaMemcpy(status)");
-  if (h.code != 0) rt_check(cudaMemset(s, 0, sizeof(Status)), "cudaMemset(status)");
+  if (h.code != 0) {
+    rt_check(cudaMemset(s, 0, sizeof(Status)), "cudaMemset(status)");
+    clear_tail_counters(device);
+  }
   return py::make_tuple(h.code, h.rank, h.block, h.peer, h.where, h.aux);
 }
 
 cudaStream_t current_stream(int device) { return c10::cuda::getCurrentCUDAStream(device).stream(); }
+
+// ---- arrival counters of the GEMM's split-K tail -----------------------------
+// 4 KiB per (device, stream), zero between launches (the kernel resets them), so that calls on different
+// streams never share one.  At most kMaxCounterBuffers of them; a call beyond that, or one that is being
+// captured (its graph may be replayed beside anything), takes its counters from the framework's allocator
+// and clears them in the stream.
+constexpr size_t kTailCounterSlots = 1024;
+constexpr size_t kMaxCounterBuffers = 64;
+std::mutex g_counters_mu;
+std::map<std::pair<int, cudaStream_t>, uint32_t*> g_counters;
+
+uint32_t* tail_counters(int device, cudaStream_t stream, torch::Tensor& own) {
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  rt_check(cudaStreamIsCapturing(stream, &capturing), "cudaStreamIsCapturing");
+  if (capturing == cudaStreamCaptureStatusNone) {
+    std::lock_guard<std::mutex> lock(g_counters_mu);
+    auto it = g_counters.find({device, stream});
+    if (it != g_counters.end()) return it->second;
+    if (g_counters.size() < kMaxCounterBuffers) {
+      uint32_t* c = nullptr;
+      rt_check(cudaMalloc(reinterpret_cast<void**>(&c), kTailCounterSlots * 4), "cudaMalloc(counters)");
+      rt_check(cudaMemset(c, 0, kTailCounterSlots * 4), "cudaMemset(counters)");
+      return g_counters[{device, stream}] = c;
+    }
+  }
+  own = at::empty({(int64_t)kTailCounterSlots}, torch::TensorOptions().dtype(torch::kInt32).device(torch::kCUDA, device));
+  rt_check(cudaMemsetAsync(own.data_ptr(), 0, kTailCounterSlots * 4, stream), "cudaMemsetAsync(counters)");
+  return reinterpret_cast<uint32_t*>(own.data_ptr());
+}
+
+// After a kernel gave up on a wait its counters hold whatever they held: back to zero (the device is idle).
+void clear_tail_counters(int device) {
+  std::lock_guard<std::mutex> lock(g_counters_mu);
+  for (auto& kv : g_counters)
+    if (kv.first.first == device) rt_check(cudaMemset(kv.second, 0, kTailCounterSlots * 4), "cudaMemset(counters)");
+}
+
+void release_tail_counters() {
+  std::lock_guard<std::mutex> lock(g_counters_mu);
+  for (auto& kv : g_counters) {
+    c10::cuda::CUDAGuard guard(kv.first.first);
+    cudaFree(kv.second);
+  }
+  g_counters.clear();
+}
 
 // ---- which symmetric allocation an address belongs to ----------------------
 // Looked up on every all-reduce, so it lives here and not in a Python dictionary: an ordered map from payload
@@ -618,6 +668,62 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
      py::arg("trace") = py::none(), py::arg("lead") = -1,
      py::arg("push_ahead") = 0, py::arg("push_plain_stores") = false,
      py::arg("push_pieces") = 0, py::arg("panel_w") = 0);
+
+  // The GEMM alone (no gather): checks, output, scratch and launch in one call.  None when the operands are not
+  // what the kernel takes: the caller's full path then says why.  epilogue: see AgMatmulArgs.
+  m.def("matmul_local", [](const torch::Tensor& a, const torch::Tensor& b, const c10::optional<torch::Tensor>& out,
+                           int epilogue, const c10::optional<torch::Tensor>& residual, int block_n, int num_sms,
+                           bool split_k, int panel_w, uint64_t timeout_ns, int max_splits) -> c10::optional<torch::Tensor> {
+    const auto dtype = a.scalar_type();
+    const bool fp8 = dtype == at::kFloat8_e4m3fn;
+    if ((!fp8 && dtype != torch::kBFloat16) || !a.is_cuda()) return c10::nullopt;
+    const int dev = a.get_device();
+    auto ok = [dtype, dev](const torch::Tensor& t) {
+      return t.is_cuda() && t.get_device() == dev && t.dim() == 2 && t.is_contiguous() && t.scalar_type() == dtype &&
+             (uintptr_t)t.data_ptr() % 16 == 0;
+    };
+    if (!ok(a) || !ok(b) || a.size(1) != b.size(1)) return c10::nullopt;
+    const int64_t M = a.size(0), N = b.size(0), K = a.size(1), align = fp8 ? 16 : 8;
+    const bool swiglu = epilogue != 0;
+    if (M < 1 || N < 1 || K < 1 || N % align != 0 || K % align != 0 || epilogue < 0 || epilogue > 2) return c10::nullopt;
+    if (swiglu && (fp8 || N % (epilogue == 1 ? 256 : 16) != 0 || (block_n != 0 && block_n != 256))) return c10::nullopt;
+    const int64_t n_out = swiglu ? N / 2 : N;
+    if (out.has_value() && (!ok(*out) || out->size(0) != M || out->size(1) != n_out)) return c10::nullopt;
+    if (residual.has_value() && (fp8 || swiglu || !ok(*residual) || residual->size(0) != M || residual->size(1) != N))
+      return c10::nullopt;
+    c10::cuda::CUDAGuard guard(dev);
+    cudaStream_t stream = current_stream(dev);
+    torch::Tensor c = out.has_value() ? *out : at::empty({M, n_out}, a.options());
+    AgMatmulArgs args{};
+    args.a_local = a.data_ptr();
+    args.b = b.data_ptr();
+    args.c = c.data_ptr();
+    args.M = (int)M; args.N = (int)N; args.K = (int)K;
+    args.elem_bytes = fp8 ? 1 : 2;
+    args.epilogue = epilogue;
+    args.residual = residual ? residual->data_ptr() : nullptr;
+    args.num_sms = num_sms > 0 ? num_sms : at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+    args.timeout_ns = timeout_ns;
+    args.status = status_for(dev);
+    args.panel_w = panel_w;
+    args.overlap = true;
+    const MatmulPlan plan = plan_matmul((int)M, (int)N, (int)K, args.elem_bytes, epilogue, block_n, args.num_sms,
+                                        split_k ? max_splits : 1);
+    args.block_n = plan.block_n;
+    torch::Tensor scratch, own_counters;
+    if (plan.tail_bytes > 0) {
+      scratch = at::empty({(int64_t)plan.tail_bytes}, a.options().dtype(torch::kUInt8));
+      args.tail_scratch = scratch.data_ptr();
+      args.tail_scratch_bytes = plan.tail_bytes;
+      args.tail_counters = tail_counters(dev, stream, own_counters);
+      args.tail_counter_slots = kTailCounterSlots;
+      args.tail_splits = plan.tail_splits;
+    }
+    rt_check(launch_ag_matmul_2cta(args, stream), "matmul");
+    return c;
+  }, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("epilogue"), py::arg("residual"), py::arg("block_n"),
+     py::arg("num_sms"), py::arg("split_k"), py::arg("panel_w"), py::arg("timeout_ns"), py::arg("max_splits") = 0);
+  m.def("release_tail_counters", &release_tail_counters);
 
   m.def("check_push_schedule", &check_push_schedule);
   m.def("check_pair_work", &check_pair_work);

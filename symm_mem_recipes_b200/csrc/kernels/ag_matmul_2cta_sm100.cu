@@ -19,11 +19,14 @@
 //   tmem_empty[b]  leader only, 8 arrivals: the four epilogue warps of each CTA
 //                  (the peer's arrive through a shared::cluster address).
 // Tail of the static schedule: when the last wave would fill only a few pairs
-// (896 tiles on 74 pairs leave 8), each of its tiles is cut along K into 2, 4
-// or 8 parts that run on as many pairs at once.  Every part stores its fp32
-// partial accumulator to scratch memory, bumps the tile's arrival counter,
+// (896 tiles on 74 pairs leave 8; a short prompt has fewer tiles than the GPU has
+// pairs to begin with), each of its tiles is cut along K into 2 to 8 parts that run
+// on as many pairs at once.  Every part stores its fp32
+// partial accumulator to scratch memory (four columns x 128 rows contiguous, so
+// that a warp's accesses are whole lines), bumps the tile's arrival counter,
 // waits (bounded) for the other parts and then reduces ITS share of the tile's
-// columns in part order, so the result does not depend on timing.
+// columns in part order, so the result does not depend on timing.  The last part
+// to leave puts the counter back to zero: no memset in front of the kernel.
 // The two 128-row blocks of a pair are two consecutive positions of the M
 // schedule, not necessarily neighbours in memory: each CTA loads, waits for and
 // stores its own block.
@@ -39,6 +42,7 @@
 // this library used to carry): 1940 µs against 705-724 µs on 4 GPUs at the
 // Llama-3-70B shape; an ordinary (non-symmetric) a_out is therefore served by this
 // kernel through the internal symmetric buffer plus one local copy.
+#include "../device/pdl.cuh"
 #include "../device/tcgen05_pair.cuh"
 #include "ag_matmul_common.cuh"
 #include "residency.h"
@@ -49,14 +53,16 @@ using namespace agmm;
 
 namespace {
 
-// Whether an instantiation's epilogue leaves through shared memory and TMA stores: plain bf16
-// output in whole boxes of 64 columns (a 224-wide tile would spill into its neighbour's columns).
+// Bytes of C that a tile has per row, and whether they leave through shared memory and TMA stores: in whole
+// boxes of 128 bytes (a bf16 tile of 224 columns, or an fp8 tile of 192 or 224, would spill into its neighbour).
 template <int BN, bool kFp8, bool kSwiGlu>
-constexpr bool pair_tma_store() { return !kFp8 && !kSwiGlu && BN % 64 == 0; }
+constexpr int pair_row_bytes() { return kFp8 ? BN : (kSwiGlu ? BN : 2 * BN); }
+template <int BN, bool kFp8, bool kSwiGlu>
+constexpr bool pair_tma_store() { return pair_row_bytes<BN, kFp8, kSwiGlu>() % 128 == 0; }
 
-// kOut: the plain bf16 epilogue leaves through shared memory: each epilogue warp owns two
-// 4 KB boxes (32 rows x 64 columns, 128-byte swizzle) that it fills from its accumulator rows
-// and hands to a TMA store while it converts the next 64 columns into the other box.
+// kOut: the epilogue leaves through shared memory: each epilogue warp owns two 4 KB boxes (32 rows x 128
+// bytes, 128-byte swizzle) that it fills from its accumulator rows and hands to a TMA store while it
+// converts the next columns into the other box.
 template <int BN, int STAGES, bool kOut = false>
 struct PairSmem {
   static constexpr uint32_t kABytes = kBM * kBK * 2;
@@ -80,14 +86,18 @@ struct PairSmem {
 // 256-column tile holds 128 gate columns followed by the 128 matching up columns;
 // the epilogue writes SiLU(gate) * up, i.e. C is [M, N / 2] and tile ni covers its
 // columns [128 ni, 128 ni + 128).  The activation never makes a round trip through
-// memory and C is half as wide.  The split-K tail is not used with it.
-template <int BN, int STAGES, bool kFp8, bool kSwiGlu = false>
+// memory and C is half as wide.  Since each CTA of a pair loads half of the tile's rows of
+// B, gate and up rows may as well come from two separate halves of B (`b_pair`).
+// kResidual (bf16, plain): C = bf16(bf16(A B^T) + residual), the residual add of a decoder layer without a pass of
+// its own over C.
+template <int BN, int STAGES, bool kFp8, bool kSwiGlu = false, bool kResidual = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
                       const __grid_constant__ CUtensorMap tmap_a_out,
                       const __grid_constant__ CUtensorMap tmap_b,
                       const __grid_constant__ CUtensorMap tmap_c, const AgMatmulParams p) {
   constexpr bool kTmaStore = pair_tma_store<BN, kFp8, kSwiGlu>();
+  static_assert(!kResidual || (kTmaStore && !kFp8 && !kSwiGlu), "the residual belongs to the plain bf16 epilogue");
   using L = PairSmem<BN, STAGES, kTmaStore>;
   extern __shared__ uint8_t smem_raw[];
   // same offset in both CTAs: the dynamic window starts at the same shared address
@@ -134,6 +144,7 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
   cluster_sync_all();                 // barriers of both CTAs initialised, TMEM allocated
   tcgen05_fence_after_thread_sync();
   const uint32_t tmem_base = *tmem_slot;
+  if (threadIdx.x == 0) pdl_launch_dependents();
   const bool tr = p.trace != nullptr;
   uint64_t* trc = tr ? p.trace + (size_t)blockIdx.x * ag_trace::kTraceSlots : nullptr;
   if (tr && threadIdx.x == 0) trc[ag_trace::kStart] = globaltimer_ns();
@@ -149,11 +160,12 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t stage = 0, phase = 0;
       PairWork w;
       uint64_t t_flag = 0, t_stage = 0, t_first = 0;
       bool first_remote = true;
+      pdl_wait();
       for (int wi = 0; !failed && pair_work(p, pair, n_pairs, total_tiles, k_blocks, wi, w); ++wi) {
         const int t = w.tile;
         int prow, ni;
@@ -201,7 +213,7 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
           if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2u * L::kStageBytes);
           const uint32_t full_leader = map_to_cta(smem_u32(&full_bar[stage]), 0);
           tma_load_2d_pair(sa, amap, full_leader, kb * kBKE, row0);
-          tma_load_2d_pair(sb, &tmap_b, full_leader, kb * kBKE, ni * BN + (int)cta_rank * (BN / 2));
+          tma_load_2d_pair(sb, &tmap_b, full_leader, kb * kBKE, ni * p.b_step + (int)cta_rank * p.b_pair);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -213,7 +225,7 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
-    if (leader && lane == 0) {
+    if (leader && elect_one()) {
       constexpr uint32_t idesc = kFp8 ? umma_idesc_e4m3_f32(2 * kBM, BN) : umma_idesc_bf16_f32(2 * kBM, BN);
       uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
       PairWork w;
@@ -273,6 +285,7 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
     const int etid = (int)threadIdx.x - 64;
     int next_piece = (int)blockIdx.x, round = 0;
     const int all_pieces = p.blocks_per_rank * p.pieces;
+    pdl_wait();
     [[maybe_unused]] int out_box = 0;                  // which of this warp's two output boxes is filled next
     if (p.mode == 2 && !push_entry_barrier(p, (int)blockIdx.x, etid)) failed = true;
     const bool trt = tr && etid == 0;
@@ -307,15 +320,23 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
       }
       tcgen05_fence_after_thread_sync();
       const int row = mblk * kBM + quarter * 32 + lane;
+      const bool row_ok = valid && row < p.M;
       const uint32_t taddr = tmem_base + acc * 256u + ((uint32_t)(quarter * 32) << 16);
-      __nv_bfloat16* crow = p.c + (size_t)row * p.N + (size_t)ni * BN;
-      uint8_t* crow8 = reinterpret_cast<uint8_t*>(p.c) + (size_t)row * p.N + (size_t)ni * BN;   // kFp8
+      auto release_accumulator = [&]() {
+        tcgen05_fence_before_thread_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
+      };
+      constexpr int kOutCols = kSwiGlu ? BN / 2 : BN;                // columns of C in this tile
+      const int n_out = kSwiGlu ? p.N >> 1 : p.N;                    // columns of C
+      const int col0 = ni * kOutCols;
+      uint8_t* crow = reinterpret_cast<uint8_t*>(p.c) + ((size_t)row * n_out + col0) * (kFp8 ? 1 : 2);
+      [[maybe_unused]] const __nv_bfloat16* rrow = kResidual ? p.residual + (size_t)row * n_out + col0 : nullptr;
       if (w.part >= 0) {
         // ---- split-K tail: park the fp32 partial, meet the other parts, reduce my columns ----
+        const size_t blk = (size_t)kBM * BN;                         // floats per CTA block
         const int r = quarter * 32 + lane;
-        const size_t blk = (size_t)kBM * BN;                       // floats per CTA block
-        float* mine = p.tail_scratch + (((size_t)w.tail_idx * p.tail_splits + w.part) * 2 + cta_rank) * blk +
-                      (size_t)r * BN;
+        float* mine = p.tail_scratch + (((size_t)w.tail_idx * p.tail_splits + w.part) * 2 + cta_rank) * blk + r * 4;
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
           uint32_t v[32];
@@ -328,11 +349,9 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
           }
 #pragma unroll
           for (int q = 0; q < 8; ++q)
-            st_16(mine + c * 32 + q * 4, Vec16{v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]});
+            st_16(mine + (size_t)(c * 8 + q) * (kBM * 4), Vec16{v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]});
         }
-        tcgen05_fence_before_thread_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
+        release_accumulator();
         __threadfence();
         if (etid == 0) tail_ok = 1;
         epilogue_group_sync();
@@ -343,161 +362,180 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
             report_status(p.status, kTimeoutFlag, p.rank, blockIdx.x, w.tail_idx, kWhereGemmTmemFull, w.part);
             tail_ok = 0;
           }
+          // every part counts twice; the one that brings the counter to 2 x parts is the last to have seen it
+          if (atomicAdd(counter, 1u) == 2u * (uint32_t)p.tail_splits - 1u) *counter = 0u;
         }
         epilogue_group_sync();
         if (!tail_ok) { failed = true; break; }
-        const int cw = BN / p.tail_splits;                         // my share of the tile's columns
-        const float* base = p.tail_scratch + ((size_t)w.tail_idx * p.tail_splits * 2 + cta_rank) * blk +
-                            (size_t)r * BN + (size_t)w.part * cw;
-        for (int c8 = 0; c8 < cw; c8 += 8) {
-          float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-          for (int sp = 0; sp < p.tail_splits; ++sp) {             // part order: deterministic
-            const float* src = base + (size_t)sp * 2 * blk + c8;
-            Vec16 lo = ld_16_stream(src), hi = ld_16_stream(src + 4);
-            s[0] += __uint_as_float(lo.x); s[1] += __uint_as_float(lo.y);
-            s[2] += __uint_as_float(lo.z); s[3] += __uint_as_float(lo.w);
-            s[4] += __uint_as_float(hi.x); s[5] += __uint_as_float(hi.y);
-            s[6] += __uint_as_float(hi.z); s[7] += __uint_as_float(hi.w);
-          }
-          const int col = ni * BN + w.part * cw + c8;
-          if (valid && row < p.M && col < p.N) {
-            if constexpr (kFp8) {
-              st_8(crow8 + w.part * cw + c8, pack_e4m3x4(s[0], s[1], s[2], s[3]),
-                   pack_e4m3x4(s[4], s[5], s[6], s[7]));
-            } else {
-              Vec16 o;
-              o.x = pack_bf16x2(s[0], s[1]); o.y = pack_bf16x2(s[2], s[3]);
-              o.z = pack_bf16x2(s[4], s[5]); o.w = pack_bf16x2(s[6], s[7]);
-              st_16(crow + w.part * cw + c8, o);
-            }
-          }
-        }
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1;
-        continue;
-      }
-      if constexpr (kSwiGlu) {
-        const int F = p.N >> 1;                            // output columns
-        __nv_bfloat16* orow = p.c + (size_t)row * F + (size_t)ni * (BN / 2);
+        // My share of the tile's columns of C, in groups of eight.  Four groups of accumulator columns (with
+        // SwiGLU two of gate and the matching two of up) times two parts are in flight at once, because one
+        // group at a time would pay the L2's latency for each.
+        constexpr int kGroups = kOutCols / 8, kBatch = kSwiGlu ? 2 : 4;
+        const int g0 = w.part * kGroups / p.tail_splits, g1 = (w.part + 1) * kGroups / p.tail_splits;
+        const float* base = p.tail_scratch + ((size_t)w.tail_idx * p.tail_splits * 2 + cta_rank) * blk + r * 4;
 #pragma unroll 1
-        for (int c = 0; c < BN / 64; ++c) {
-          uint32_t g[32], u[32];
-          tmem_ld_32x32b_x32(taddr + (uint32_t)(c * 32), g);                 // gate columns
-          tmem_ld_32x32b_x32(taddr + (uint32_t)(BN / 2 + c * 32), u);        // the matching up columns
-          tmem_ld_wait();
-          const int col0 = ni * (BN / 2) + c * 32;
-          if (valid && row < p.M) {
+        for (int g = g0; g < g1; g += kBatch) {
+          float s[4][8];
+          const float* src[4];
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              if (col0 + v * 8 < F) {
-                float y[8];
+          for (int i = 0; i < 4; ++i) {
+            const int col = kSwiGlu ? (i >> 1) * (BN / 2) + (g + (i & 1)) * 8 : (g + i) * 8;
+            src[i] = base + (size_t)(col / 4) * (kBM * 4);
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                  const float gv = __uint_as_float(g[v * 8 + q]);
-                  y[q] = gv / (1.0f + __expf(-gv)) * __uint_as_float(u[v * 8 + q]);
+            for (int q = 0; q < 8; ++q) s[i][q] = 0.f;
+          }
+#pragma unroll 1
+          for (int sp = 0; sp < p.tail_splits; sp += 2) {             // parts in order: deterministic
+            Vec16 v[2][4][2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (sp + u < p.tail_splits && g + (kSwiGlu ? i & 1 : i) < g1) {
+                  v[u][i][0] = ld_16_stream(src[i] + (size_t)(sp + u) * 2 * blk);
+                  v[u][i][1] = ld_16_stream(src[i] + (size_t)(sp + u) * 2 * blk + kBM * 4);
                 }
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (sp + u < p.tail_splits && g + (kSwiGlu ? i & 1 : i) < g1) {
+                  s[i][0] += __uint_as_float(v[u][i][0].x); s[i][1] += __uint_as_float(v[u][i][0].y);
+                  s[i][2] += __uint_as_float(v[u][i][0].z); s[i][3] += __uint_as_float(v[u][i][0].w);
+                  s[i][4] += __uint_as_float(v[u][i][1].x); s[i][5] += __uint_as_float(v[u][i][1].y);
+                  s[i][6] += __uint_as_float(v[u][i][1].z); s[i][7] += __uint_as_float(v[u][i][1].w);
+                }
+          }
+#pragma unroll
+          for (int i = 0; i < kBatch; ++i) {
+            if constexpr (kSwiGlu) {
+#pragma unroll
+              for (int q = 0; q < 8; ++q) s[i][q] = s[i][q] / (1.0f + __expf(-s[i][q])) * s[i + 2][q];
+            }
+            const int col = (g + i) * 8;
+            if (row_ok && g + i < g1 && col0 + col < n_out) {
+              if constexpr (kFp8) {
+                st_8(crow + col, pack_e4m3x4(s[i][0], s[i][1], s[i][2], s[i][3]), pack_e4m3x4(s[i][4], s[i][5], s[i][6], s[i][7]));
+              } else {
                 Vec16 o;
-                o.x = pack_bf16x2(y[0], y[1]); o.y = pack_bf16x2(y[2], y[3]);
-                o.z = pack_bf16x2(y[4], y[5]); o.w = pack_bf16x2(y[6], y[7]);
-                st_16(orow + c * 32 + v * 8, o);
+                o.x = pack_bf16x2(s[i][0], s[i][1]); o.y = pack_bf16x2(s[i][2], s[i][3]);
+                o.z = pack_bf16x2(s[i][4], s[i][5]); o.w = pack_bf16x2(s[i][6], s[i][7]);
+                if constexpr (kResidual) o = add_bf16x8(o, ld_16(rrow + col));
+                st_16(crow + col * 2, o);
               }
             }
           }
         }
       } else if constexpr (kTmaStore) {
-        // 64 columns at a time: two TMEM loads in flight, bf16 into this warp's free box
-        // (16-byte chunk j of row r sits at chunk j ^ (r & 7): the 128-byte swizzle of the
-        // tensor map, and conflict-free for the warp's stores), then one TMA store.
+        // One box (128 bytes of every row) at a time: accumulator columns -> packed words -> this warp's free
+        // box (16-byte chunk j of row r sits at chunk j ^ (r & 7): the 128-byte swizzle of the tensor map,
+        // conflict-free for the warp's stores) -> one TMA store.
+        constexpr int kBoxes = pair_row_bytes<BN, kFp8, kSwiGlu>() / 128;
+        constexpr int kBoxCols = kOutCols / kBoxes;                  // columns of C per box
         const uint32_t box0 = smem_u32(smem + L::kOutOffset) + (uint32_t)quarter * 2u * L::kOutBoxBytes;
         const bool store_ok = valid && mblk * kBM + quarter * 32 < p.M;
-#pragma unroll 1
-        for (int c = 0; c < BN / 64; ++c) {
-          uint32_t r0[32], r1[32];
-          tmem_ld_32x32b_x32(taddr + (uint32_t)(c * 64), r0);
-          tmem_ld_32x32b_x32(taddr + (uint32_t)(c * 64 + 32), r1);
-          if (lane == 0) bulk_wait_group_read<1>();      // the store that last read this box is done with it
-          __syncwarp();
-          tmem_ld_wait();
-          if (c == BN / 64 - 1) {
-            // the accumulator is in registers: hand it back before the stores
-            tcgen05_fence_before_thread_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
+        Vec16 res[kResidual ? 8 : 1];
+        auto fetch_residual = [&](int c) {
+          if constexpr (kResidual) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              res[j] = row_ok && col0 + c * kBoxCols + j * 8 < n_out ? ld_16(rrow + c * kBoxCols + j * 8) : Vec16{0u, 0u, 0u, 0u};
           }
+        };
+        fetch_residual(0);
+#pragma unroll 1
+        for (int c = 0; c < kBoxes; ++c) {
+          // 64 accumulator columns in flight: the whole box, or half of it where two go into one of C's bytes (fp8)
+          // or columns (SwiGLU)
+          constexpr int kPasses = kFp8 || kSwiGlu ? 2 : 1;
           const uint32_t box = box0 + (uint32_t)out_box * L::kOutBoxBytes;
           const uint32_t rowaddr = box + (uint32_t)lane * 128u;
           const uint32_t sw = (uint32_t)(lane & 7);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            st_shared_16(rowaddr + ((((uint32_t)j) ^ sw) << 4),
-                         pack_bf16x2(__uint_as_float(r0[j * 8 + 0]), __uint_as_float(r0[j * 8 + 1])),
-                         pack_bf16x2(__uint_as_float(r0[j * 8 + 2]), __uint_as_float(r0[j * 8 + 3])),
-                         pack_bf16x2(__uint_as_float(r0[j * 8 + 4]), __uint_as_float(r0[j * 8 + 5])),
-                         pack_bf16x2(__uint_as_float(r0[j * 8 + 6]), __uint_as_float(r0[j * 8 + 7])));
-            st_shared_16(rowaddr + ((((uint32_t)(j + 4)) ^ sw) << 4),
-                         pack_bf16x2(__uint_as_float(r1[j * 8 + 0]), __uint_as_float(r1[j * 8 + 1])),
-                         pack_bf16x2(__uint_as_float(r1[j * 8 + 2]), __uint_as_float(r1[j * 8 + 3])),
-                         pack_bf16x2(__uint_as_float(r1[j * 8 + 4]), __uint_as_float(r1[j * 8 + 5])),
-                         pack_bf16x2(__uint_as_float(r1[j * 8 + 6]), __uint_as_float(r1[j * 8 + 7])));
+          for (int h = 0; h < kPasses; ++h) {
+            uint32_t v[2][32];
+            if constexpr (kSwiGlu) {
+              tmem_ld_32x32b_x32(taddr + (uint32_t)(c * 64 + h * 32), v[0]);             // gate columns
+              tmem_ld_32x32b_x32(taddr + (uint32_t)(BN / 2 + c * 64 + h * 32), v[1]);    // the matching up columns
+            } else {
+              tmem_ld_32x32b_x32(taddr + (uint32_t)(c * kBoxCols + h * 64), v[0]);
+              tmem_ld_32x32b_x32(taddr + (uint32_t)(c * kBoxCols + h * 64 + 32), v[1]);
+            }
+            if (h == 0) {
+              if (lane == 0) bulk_wait_group_read<1>();      // the store that last read this box is done with it
+              __syncwarp();
+            }
+            tmem_ld_wait();
+            // the accumulator is in registers: hand it back before the stores
+            if (c == kBoxes - 1 && h == kPasses - 1) release_accumulator();
+#pragma unroll
+            for (int j = 0; j < 8 / kPasses; ++j) {
+              Vec16 o;
+              if constexpr (kFp8) {
+                const uint32_t* q = v[j / 2] + (j & 1) * 16;
+                auto f = [q](int i) { return __uint_as_float(q[i]); };
+                o.x = pack_e4m3x4(f(0), f(1), f(2), f(3)); o.y = pack_e4m3x4(f(4), f(5), f(6), f(7));
+                o.z = pack_e4m3x4(f(8), f(9), f(10), f(11)); o.w = pack_e4m3x4(f(12), f(13), f(14), f(15));
+              } else {
+                const uint32_t* q = v[kSwiGlu ? 0 : j / 4] + (j & 3) * 8;
+                float y[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                  y[i] = __uint_as_float(q[i]);
+                  if constexpr (kSwiGlu) y[i] = y[i] / (1.0f + __expf(-y[i])) * __uint_as_float(v[1][j * 8 + i]);
+                }
+                o.x = pack_bf16x2(y[0], y[1]); o.y = pack_bf16x2(y[2], y[3]);
+                o.z = pack_bf16x2(y[4], y[5]); o.w = pack_bf16x2(y[6], y[7]);
+                if constexpr (kResidual) o = add_bf16x8(o, res[j]);
+              }
+              st_shared_16(rowaddr + (((uint32_t)(h * (8 / kPasses) + j) ^ sw) << 4), o.x, o.y, o.z, o.w);
+            }
           }
+          if (c + 1 < kBoxes) fetch_residual(c + 1);
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            if (store_ok && ni * BN + c * 64 < p.N) {
+            if (store_ok && col0 + c * kBoxCols < n_out) {
               uint8_t* src = smem + L::kOutOffset + ((size_t)quarter * 2 + out_box) * L::kOutBoxBytes;
-              tma_store_2d(&tmap_c, src, ni * BN + c * 64, mblk * kBM + quarter * 32);
+              tma_store_2d(&tmap_c, src, col0 + c * kBoxCols, mblk * kBM + quarter * 32);
             }
             bulk_commit_group();
           }
           out_box ^= 1;
         }
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1;
-        continue;
       } else {
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(taddr + (uint32_t)(c * 32), r);
-        tmem_ld_wait();
-        const int col0 = ni * BN + c * 32;
-        if constexpr (kFp8) {
-          if (valid && row < p.M) {
+        for (int c = 0; c < BN / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(taddr + (uint32_t)(c * 32), r);
+          tmem_ld_wait();
+          if constexpr (kFp8) {
 #pragma unroll
             for (int v = 0; v < 2; ++v) {
-              if (col0 + v * 16 < p.N) {
+              if (row_ok && col0 + c * 32 + v * 16 < p.N) {
+                auto f = [&r, v](int i) { return __uint_as_float(r[v * 16 + i]); };
                 Vec16 o;
-                const uint32_t* q = r + v * 16;
-                o.x = pack_e4m3x4(__uint_as_float(q[0]), __uint_as_float(q[1]),
-                                  __uint_as_float(q[2]), __uint_as_float(q[3]));
-                o.y = pack_e4m3x4(__uint_as_float(q[4]), __uint_as_float(q[5]),
-                                  __uint_as_float(q[6]), __uint_as_float(q[7]));
-                o.z = pack_e4m3x4(__uint_as_float(q[8]), __uint_as_float(q[9]),
-                                  __uint_as_float(q[10]), __uint_as_float(q[11]));
-                o.w = pack_e4m3x4(__uint_as_float(q[12]), __uint_as_float(q[13]),
-                                  __uint_as_float(q[14]), __uint_as_float(q[15]));
-                st_16(crow8 + c * 32 + v * 16, o);
+                o.x = pack_e4m3x4(f(0), f(1), f(2), f(3)); o.y = pack_e4m3x4(f(4), f(5), f(6), f(7));
+                o.z = pack_e4m3x4(f(8), f(9), f(10), f(11)); o.w = pack_e4m3x4(f(12), f(13), f(14), f(15));
+                st_16(crow + c * 32 + v * 16, o);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              if (row_ok && col0 + c * 32 + v * 8 < p.N) {
+                Vec16 o;
+                o.x = pack_bf16x2(__uint_as_float(r[v * 8 + 0]), __uint_as_float(r[v * 8 + 1]));
+                o.y = pack_bf16x2(__uint_as_float(r[v * 8 + 2]), __uint_as_float(r[v * 8 + 3]));
+                o.z = pack_bf16x2(__uint_as_float(r[v * 8 + 4]), __uint_as_float(r[v * 8 + 5]));
+                o.w = pack_bf16x2(__uint_as_float(r[v * 8 + 6]), __uint_as_float(r[v * 8 + 7]));
+                st_16(crow + (c * 32 + v * 8) * 2, o);
               }
             }
           }
-        } else if (valid && row < p.M) {
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            if (col0 + v * 8 < p.N) {
-              Vec16 o;
-              o.x = pack_bf16x2(__uint_as_float(r[v * 8 + 0]), __uint_as_float(r[v * 8 + 1]));
-              o.y = pack_bf16x2(__uint_as_float(r[v * 8 + 2]), __uint_as_float(r[v * 8 + 3]));
-              o.z = pack_bf16x2(__uint_as_float(r[v * 8 + 4]), __uint_as_float(r[v * 8 + 5]));
-              o.w = pack_bf16x2(__uint_as_float(r[v * 8 + 6]), __uint_as_float(r[v * 8 + 7]));
-              st_16(crow + c * 32 + v * 8, o);
-            }
-          }
         }
+        release_accumulator();
       }
-      }   // plain epilogue
-      tcgen05_fence_before_thread_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1;
     }
@@ -537,21 +575,88 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
   }
 }
 
-template <int BN, int STAGES, bool kFp8, bool kSwiGlu = false>
+template <int BN, int STAGES, bool kFp8, bool kSwiGlu = false, bool kResidual = false>
 int launch_pair_variant(const CUtensorMap& ta_shard, const CUtensorMap& ta_out, const CUtensorMap& tb,
-                        const CUtensorMap& tc, const AgMatmulParams& p, int grid, cudaStream_t stream) {
+                        const CUtensorMap& tc, const AgMatmulParams& p, int grid, bool overlap, cudaStream_t stream) {
   using L = PairSmem<BN, STAGES, pair_tma_store<BN, kFp8, kSwiGlu>()>;
   static_assert(L::kTotal <= 232448, "shared memory limit exceeded");
-  auto kern = ag_matmul_2cta_kernel<BN, STAGES, kFp8, kSwiGlu>;
+  auto kern = ag_matmul_2cta_kernel<BN, STAGES, kFp8, kSwiGlu, kResidual>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kTotal);
   if (e != cudaSuccess) return (int)e;
   // The pairs wait for one another (pieces of the gather, parts of the split-K tail): all of them must be resident.
   if (int rc = check_co_resident(kern, grid, kGemmThreads, L::kTotal, 2)) return rc;
-  kern<<<grid, kGemmThreads, L::kTotal, stream>>>(ta_shard, ta_out, tb, tc, p);
-  return (int)cudaGetLastError();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid, 1, 1);
+  cfg.blockDim = dim3(kGemmThreads, 1, 1);
+  cfg.dynamicSmemBytes = L::kTotal;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return (int)cudaLaunchKernelEx(&cfg, kern, ta_shard, ta_out, tb, tc, p);
 }
 
 }  // namespace
+
+namespace {
+
+// Parts a tile of the tail is cut into: `rem` tiles in the last wave of `pairs` pairs.
+int tail_parts(int rem, int pairs, int k_blocks, int most) {
+  if (rem <= 0 || rem * 2 > pairs) return 1;
+  int splits = pairs / rem;
+  if (splits > 8) splits = 8;
+  if (most > 0 && splits > most) splits = most;
+  while (splits > 1 && k_blocks < 2 * splits) --splits;
+  return splits;
+}
+
+}  // namespace
+
+// Tile width and tail of a GEMM by a model of its time, fitted to measurements of every width and split on 21 shapes
+// (M 17 to 6000): a wave of n of the P pairs takes, per K block of 128 bytes, t1 with few pairs at work (the
+// tensor core's own rate) up to t1 + t2 with all of them (shared L2 and power), so narrow tiles win where tiles
+// are few and 256 columns where waves are full; cutting the last wave along K costs a pass through L2.
+// Examples, before (always 256 columns, no cut below one wave) and after: 64 x 1280 x 8192 41 -> 13 us,
+// 129 x 7168 x 8192 45 -> 32 us, 509 x 1280 x 8192 42 -> 18 us, 300 x 2048 x 2048 15 -> 10 us.
+MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int block_n, int num_sms, int max_splits) {
+  struct Width { int bn; double t1, t2, merge; };                   // microseconds
+  constexpr Width kWidths[] = {{256, 0.285, 0.135, 6.4}, {192, 0.215, 0.115, 5.4}, {128, 0.14, 0.095, 4.2}};
+  const int pairs = num_sms / 2, rows = (M + 2 * kBM - 1) / (2 * kBM);
+  const int k_blocks = (K * elem_bytes + 127) / 128;
+  MatmulPlan best{block_n != 0 ? block_n : 256, 1, 0};
+  double best_cost = -1;
+  for (const Width& w : kWidths) {
+    // a width the caller (or the SwiGLU epilogue) asks for is taken with the figures of the nearest one
+    if (block_n != 0 || epilogue != 0) {
+      if (w.bn != (block_n == 128 || block_n == 192 ? block_n : 256)) continue;
+    }
+    const int bn = block_n != 0 ? block_n : w.bn;
+    const int tiles = rows * (epilogue != 0 ? (N / 2 + bn / 2 - 1) / (bn / 2) : (N + bn - 1) / bn);
+    // full waves of 256 columns lose more in fp8 (twice the MMA rate on the same operand bytes)
+    const double t2 = elem_bytes == 1 && w.bn == 256 ? 0.165 : w.t2;
+    auto wave_us = [&](int n, int parts) { return k_blocks * (w.t1 + t2 * n * parts / pairs) / parts; };
+    const int rem = tiles % pairs;
+    double cost = tiles / pairs * wave_us(pairs, 1);
+    int parts = 1;
+    if (rem > 0) {
+      double tail = wave_us(rem, 1);
+      for (int most = tail_parts(rem, pairs, k_blocks, max_splits); most >= 2; --most) {
+        const double cut = wave_us(rem, most) + w.merge;
+        if (cut < tail) { tail = cut; parts = most; }
+      }
+      cost += tail;
+    }
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best.block_n = bn;
+      best.tail_splits = parts;
+      best.tail_bytes = parts > 1 ? (size_t)rem * parts * 2 * kBM * bn * sizeof(float) : 0;
+    }
+  }
+  return best;
+}
 
 int launch_ag_matmul_2cta(const AgMatmulArgs& a, cudaStream_t stream) {
   if (a.elem_bytes != 0 && a.elem_bytes != 1 && a.elem_bytes != 2) return cudaErrorInvalidValue;
@@ -569,16 +674,22 @@ int launch_ag_matmul_2cta(const AgMatmulArgs& a, cudaStream_t stream) {
   }
   const int bn = a.block_n;
   if (bn != 128 && bn != 192 && bn != 224 && bn != 256) return cudaErrorInvalidValue;
-  const bool swiglu = a.epilogue == 1;
-  if (a.epilogue != 0 && a.epilogue != 1) return cudaErrorInvalidValue;
-  // gate / up interleaved in groups of 128 rows of B: whole groups only, bf16, 256-column tiles
-  if (swiglu && (fp8 || bn != 256 || a.N % 256 != 0)) return cudaErrorInvalidValue;
+  const bool swiglu = a.epilogue != 0;
+  if (a.epilogue < 0 || a.epilogue > 2) return cudaErrorInvalidValue;
+  // bf16, 256-column tiles; interleaved in groups of 128 rows of B: whole groups only
+  if (swiglu && (fp8 || bn != 256 || a.N % (a.epilogue == 1 ? 256 : 16) != 0)) return cudaErrorInvalidValue;
+  if (a.residual != nullptr && (swiglu || fp8 || comm || bn == 224 || (uintptr_t)a.residual % 16 != 0))
+    return cudaErrorInvalidValue;
 
   AgMatmulParams p{};
   p.c = static_cast<__nv_bfloat16*>(a.c);
   p.M = a.M; p.N = a.N; p.K = a.K;
   p.elem_bytes = es;
-  p.n_tiles_n = (a.N + bn - 1) / bn;
+  // with the SwiGLU epilogue a tile is 128 columns of C, whichever way its gate and up rows are stored
+  p.n_tiles_n = swiglu ? (a.N / 2 + bn / 2 - 1) / (bn / 2) : (a.N + bn - 1) / bn;
+  p.b_step = a.epilogue == 2 ? bn / 2 : bn;
+  p.b_pair = a.epilogue == 2 ? a.N / 2 : bn / 2;
+  p.residual = static_cast<const __nv_bfloat16*>(a.residual);
   p.panel_w = a.panel_w > 0 ? (a.panel_w < p.n_tiles_n ? a.panel_w : p.n_tiles_n)
                             : pick_panel_w(p.n_tiles_n, (size_t)bn * a.K * es);
   p.n_blocks_m = (a.M + kBM - 1) / kBM;
@@ -633,9 +744,28 @@ int launch_ag_matmul_2cta(const AgMatmulArgs& a, cudaStream_t stream) {
   if (make_tmap(&tc, a.c, (uint64_t)a.M, (uint64_t)c_cols, 32, es)) return cudaErrorInvalidValue;
 
   const int total_tiles = ((p.n_blocks_m + 1) / 2) * p.n_tiles_n;
-  int pairs = a.num_sms / 2;
-  if (pairs > total_tiles) pairs = total_tiles;
-  if (pairs < 1) return cudaErrorInvalidValue;
+  const int max_pairs = a.num_sms / 2;
+  if (max_pairs < 1) return cudaErrorInvalidValue;
+  const int k_blocks = (a.K * es + 127) / 128;                    // one K block = 128 bytes of a row
+  int pairs = max_pairs < total_tiles ? max_pairs : total_tiles;
+  // split-K tail: the tiles of a last wave that fills at most half of the pairs (all tiles, when there are so
+  // few), cut into as many parts as there are pairs for, each of at least two K blocks
+  p.tail_tiles = 0;
+  p.tail_splits = 1;
+  const int rem = total_tiles % max_pairs;
+  if (a.tail_scratch != nullptr && rem > 0 && rem * 2 <= max_pairs) {
+    int splits = tail_parts(rem, max_pairs, k_blocks, a.tail_splits);
+    while (splits > 1 && ((size_t)rem * splits * 2 * kBM * bn * sizeof(float) > a.tail_scratch_bytes ||
+                          (size_t)rem * 2 > a.tail_counter_slots))
+      --splits;
+    if (splits >= 2) {
+      p.tail_tiles = rem;
+      p.tail_splits = splits;
+      p.tail_scratch = static_cast<float*>(a.tail_scratch);
+      p.tail_counters = a.tail_counters;
+      if (total_tiles < max_pairs) pairs = rem * splits;
+    }
+  }
   const int grid = 2 * pairs;
   if (comm) {
     if (a.lead < 0) {
@@ -647,40 +777,27 @@ int launch_ag_matmul_2cta(const AgMatmulArgs& a, cudaStream_t stream) {
   }
   // the entry barrier of CTA i uses block slot (barrier_block_base + i): it must stay inside the block-slot region
   if (comm && ((size_t)a.barrier_block_base + grid) * a.world_size > kBlockSlots) return cudaErrorInvalidValue;
-  // split-K tail: only when the last wave fills less than half of the pairs
-  p.tail_tiles = 0;
-  p.tail_splits = 1;
-  const int rem = total_tiles % pairs;
-  const int k_blocks = (a.K * es + 127) / 128;                    // one K block = 128 bytes of a row
-  if (a.tail_scratch != nullptr && !swiglu && rem > 0 && rem * 2 <= pairs) {
-    int splits = pairs / rem;
-    splits = splits >= 8 ? 8 : (splits >= 4 ? 4 : 2);
-    // every part reduces BN / splits columns in vectors of 8
-    while (splits > 1 && bn % (8 * splits) != 0) splits >>= 1;
-    const size_t need = (size_t)rem * splits * 2 * kBM * bn * sizeof(float);
-    if (splits >= 2 && k_blocks >= 2 * splits && need <= a.tail_scratch_bytes && (size_t)rem * 2 <= a.tail_counter_slots) {
-      p.tail_tiles = rem;
-      p.tail_splits = splits;
-      p.tail_scratch = static_cast<float*>(a.tail_scratch);
-      p.tail_counters = a.tail_counters;
-      cudaError_t me = cudaMemsetAsync(a.tail_counters, 0, sizeof(uint32_t) * rem * 2, stream);
-      if (me != cudaSuccess) return (int)me;
-    }
-  }
-  if (swiglu) return launch_pair_variant<256, 6, false, true>(ta_shard, ta_out, tb, tc, p, grid, stream);
+  if (swiglu) return launch_pair_variant<256, 6, false, true>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
   if (fp8) {
     switch (bn) {
-      case 128: return launch_pair_variant<128, 8, true>(ta_shard, ta_out, tb, tc, p, grid, stream);
-      case 192: return launch_pair_variant<192, 7, true>(ta_shard, ta_out, tb, tc, p, grid, stream);
-      case 224: return launch_pair_variant<224, 7, true>(ta_shard, ta_out, tb, tc, p, grid, stream);
-      default:  return launch_pair_variant<256, 6, true>(ta_shard, ta_out, tb, tc, p, grid, stream);
+      case 128: return launch_pair_variant<128, 8, true>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
+      case 192: return launch_pair_variant<192, 7, true>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
+      case 224: return launch_pair_variant<224, 7, true>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
+      default:  return launch_pair_variant<256, 6, true>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
+    }
+  }
+  if (p.residual != nullptr) {
+    switch (bn) {
+      case 128: return launch_pair_variant<128, 8, false, false, true>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
+      case 192: return launch_pair_variant<192, 6, false, false, true>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
+      default:  return launch_pair_variant<256, 6, false, false, true>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
     }
   }
   switch (bn) {
-    case 128: return launch_pair_variant<128, 8, false>(ta_shard, ta_out, tb, tc, p, grid, stream);
-    case 192: return launch_pair_variant<192, 6, false>(ta_shard, ta_out, tb, tc, p, grid, stream);
-    case 224: return launch_pair_variant<224, 7, false>(ta_shard, ta_out, tb, tc, p, grid, stream);
-    default:  return launch_pair_variant<256, 6, false>(ta_shard, ta_out, tb, tc, p, grid, stream);
+    case 128: return launch_pair_variant<128, 8, false>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
+    case 192: return launch_pair_variant<192, 6, false>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
+    case 224: return launch_pair_variant<224, 7, false>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
+    default:  return launch_pair_variant<256, 6, false>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
   }
 }
 

@@ -63,9 +63,12 @@ struct AgMatmulParams {
   Status* status;
   // split-K tail (2-CTA kernel): the tiles of the last, partly filled wave are cut along K
   int tail_tiles;        // tiles handled that way (0 = none); they are the last ones of the schedule
-  int tail_splits;       // K parts per such tile (2, 4 or 8)
-  float* tail_scratch;   // [tail_tiles][tail_splits][2 CTAs][128 x BN] fp32 partial accumulators
-  uint32_t* tail_counters;   // [tail_tiles][2] arrivals, zeroed before the launch
+  int tail_splits;       // K parts per such tile (2 to 8)
+  float* tail_scratch;   // [tail_tiles][tail_splits][2 CTAs][BN / 4][128 rows] x 4 fp32: partial accumulators
+  uint32_t* tail_counters;   // [tail_tiles][2] arrivals, zero between launches (the last part to leave resets them)
+  // rows of B that tile ni takes: CTA c of the pair loads BN / 2 of them from ni * b_step + c * b_pair
+  int b_step, b_pair;
+  const __nv_bfloat16* residual;   // [M, N] added to the rounded product (plain bf16 epilogue), or nullptr
   // optional per-CTA %globaltimer record (2-CTA kernel), kTraceSlots words per CTA; see ag_trace::
   uint64_t* trace;
 };

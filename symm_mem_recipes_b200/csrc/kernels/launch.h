@@ -75,7 +75,10 @@ struct AgMatmulArgs {
   int elem_bytes;
   // 0: C[M, N] = A B^T.  1 (bf16, block_n 256, N % 256 == 0): B's rows are interleaved
   // in groups of 128 (gate rows, then the matching up rows) and C[M, N / 2] = SiLU(gate) * up.
+  // 2 (bf16, block_n 256, N % 16 == 0): the same with B = [gate rows; up rows].
   int epilogue;
+  const void* residual;  // epilogue 0, bf16, mode 0: C = bf16(bf16(A B^T) + residual), [M, N], or nullptr
+  bool overlap;          // mode 0: programmatic stream serialization
   int block_n;           // 128, 192, 224 or 256
   int num_sms;           // CTAs to launch at most
   // communication: mode 0 = none (GEMM over a_local only), 2 = push (a_out symmetric; the
@@ -92,11 +95,12 @@ struct AgMatmulArgs {
   uint32_t barrier_block_base;
   uint64_t timeout_ns;
   Status* status;
-  // optional scratch of the split-K tail (nullptr = never split)
+  // optional scratch of the split-K tail (nullptr = never split); the counters are zero between launches
   void* tail_scratch;
   size_t tail_scratch_bytes;
   uint32_t* tail_counters;
   size_t tail_counter_slots;
+  int tail_splits;       // K parts of a tile of the tail at most (0 = as many as the idle pairs allow, up to 8)
   // optional [num_sms][12] words of per-CTA timing (ag_trace:: in ag_matmul_common.cuh)
   uint64_t* trace;
   // push mode: own 128-row blocks multiplied before the first remote one (-1 = chosen by the launcher)
@@ -115,6 +119,13 @@ struct AgMatmulArgs {
   int panel_w;
 };
 int launch_ag_matmul_2cta(const AgMatmulArgs& args, cudaStream_t stream);
+// Tile width and split-K tail of a GEMM without a gather (mode 0).  `block_n` / `max_splits`: 0 = the plan's choice.
+struct MatmulPlan {
+  int block_n;
+  int tail_splits;        // K parts of a tail tile (1 = no split)
+  size_t tail_bytes;      // scratch for them
+};
+MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int block_n, int num_sms, int max_splits);
 
 // Host-side checks of the kernels' scheduling arithmetic (schedule_check.cu); 0 = invariants hold.
 int check_push_schedule(int world_size, int rank, int blocks_per_rank, int n_tiles_n, int n_units,

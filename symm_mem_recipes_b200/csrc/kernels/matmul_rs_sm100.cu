@@ -130,7 +130,7 @@ matmul_rs_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t stage = 0, phase = 0;
       for (int t = pair; t < total_tiles && !failed; t += n_pairs) {
         int pr, ni;
@@ -159,7 +159,7 @@ matmul_rs_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
-    if (leader && lane == 0) {
+    if (leader && elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16_f32(2 * kBM, kBN);
       uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
       for (int t = pair; t < total_tiles && !failed; t += n_pairs) {

@@ -70,7 +70,7 @@ def _tail_buffer(device: torch.device, config: "AgMatmulConfig"):
     idx = device.index if device.index is not None else torch.cuda.current_device()
     t = _tail_scratch.get(idx)
     if t is None:
-        t = torch.empty(_TAIL_SCRATCH_BYTES, dtype=torch.uint8, device=device)
+        t = torch.zeros(_TAIL_SCRATCH_BYTES, dtype=torch.uint8, device=device)    # the counters start at zero
         _tail_scratch[idx] = t
     return t
 
@@ -170,12 +170,22 @@ def _epilogue_code(epilogue, dtype: torch.dtype, N: int, config: "AgMatmulConfig
     return code
 
 
+def _matmul_local(a, b, c_out, config: "AgMatmulConfig", epilogue: Optional[str]) -> Optional[torch.Tensor]:
+    """The GEMM without a gather in one native call, or None when the operands are not for it."""
+    return C.matmul_local(a, b, c_out, _EPILOGUES.get(epilogue, -1), None, config.block_n, config.num_sms,
+                          config.split_k_tail, config.panel_w, config.timeout_ms * 1_000_000)
+
+
 @traced("smr.matmul")
 def matmul(a: torch.Tensor, b: torch.Tensor, c_out: Optional[torch.Tensor] = None,
            config: AgMatmulConfig = DEFAULT_CONFIG, epilogue: Optional[str] = None,
            trace: Optional[torch.Tensor] = None) -> torch.Tensor:
     """C[M, N] = A[M, K] @ B[N, K]^T on the tcgen05 kernel, no communication.
     `epilogue="swiglu"`: see `all_gather_matmul`."""
+    if a.is_cuda and trace is None:
+        c = _matmul_local(a, b, c_out, config, epilogue)
+        if c is not None:
+            return c
     _check_2d("a", a)
     _check_2d("b", b, a.dtype)
     M, K = a.shape
@@ -250,6 +260,14 @@ def all_gather_matmul(a_shard: torch.Tensor, b: torch.Tensor, a_out: Optional[to
     `trace`: an int64 CUDA tensor [num_sms, 12] that receives the per-CTA timing
     record of the CTA-pair kernel (`TRACE_FIELDS`; push gather or no gather).
     """
+    if a_shard.is_cuda and trace is None and not mm_only and \
+            (not dist.is_initialized() or dist.get_world_size(group) == 1):
+        # nothing to gather: the shard is the gathered A; copy only on request
+        c = _matmul_local(a_shard, b, c_out, config, epilogue)
+        if c is not None:
+            if a_out is not None:
+                a_out.copy_(a_shard)
+            return c
     _check_2d("a_shard", a_shard)
     _check_2d("b", b, a_shard.dtype)
     if mm_only:

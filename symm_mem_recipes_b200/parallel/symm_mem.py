@@ -502,6 +502,7 @@ def shutdown() -> None:
             pass
     _records.clear()
     _groups.clear()
+    C.release_tail_counters()
 
 
 def reset() -> None:

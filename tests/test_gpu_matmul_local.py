@@ -1,0 +1,78 @@
+"""The GEMM without a gather through its native call: tile widths, K splits of a short last wave, the three
+epilogues, ragged edges; and calls on several streams at once."""
+import pytest
+import torch
+
+
+def _operands(M, N, K, dtype=torch.bfloat16):
+    gen = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a = torch.randn(M, K, generator=gen, device="cuda") * 0.5
+    b = torch.randn(N, K, generator=gen, device="cuda") * 0.1
+    return a.to(dtype), b.to(dtype)
+
+
+def _run(a, b, out=None, epilogue=0, residual=None, block_n=0, splits=0, sms=0):
+    from symm_mem_recipes_b200._ext import C
+
+    return C.matmul_local(a, b, out, epilogue, residual, block_n, sms, True, 0, 2_000_000_000, splits)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (17, 520, 1024), (129, 1280, 2048), (300, 264, 4104), (2049, 272, 1000)])
+@pytest.mark.parametrize("block_n,sms", [(0, 0), (128, 64), (192, 0), (256, 24), (224, 0)])
+def test_tiles_splits_and_residual(M, N, K, block_n, sms):
+    from symm_mem_recipes_b200.parallel import symm_mem
+    from symm_mem_recipes_b200.utils.testing import guarded_empty
+
+    a, b = _operands(M, N, K)
+    ref = a.float() @ b.float().t()
+    res = (torch.randn(M, N, device="cuda")).to(torch.bfloat16)
+    for r in (None, res):
+        if r is not None and block_n == 224:
+            continue                                     # the launcher refuses it: no whole boxes of C
+        c, intact = guarded_empty((M, N), torch.bfloat16, "cuda")
+        for _ in range(2):                               # the second call finds the counters as the first left them
+            c.fill_(float("nan"))
+            assert _run(a, b, c, residual=r, block_n=block_n, sms=sms) is not None
+        symm_mem.check_status("cuda")
+        want = ref if r is None else ref + r.float()
+        assert bool(((c.float() - want).abs() <= want.abs() * 2.0 ** -6 + 2e-2).all())
+        assert intact(), "the kernel stored outside its output"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,F,K", [(1, 8, 64), (130, 1000, 2048), (700, 3584, 1024), (2048, 3584, 512)])
+def test_swiglu_of_separate_and_interleaved_halves(M, F, K):
+    from symm_mem_recipes_b200.ops import interleave_gate_up
+    from symm_mem_recipes_b200.parallel import symm_mem
+
+    a, b = _operands(M, 2 * F, K)
+    g, u = (a.float() @ b.float().t()).split(F, dim=1)
+    want = torch.nn.functional.silu(g) * u
+    outs = [_run(a, b, epilogue=2)]
+    if F % 128 == 0:
+        outs.append(_run(a, interleave_gate_up(b[:F], b[F:]), epilogue=1))
+    symm_mem.check_status("cuda")
+    for c in outs:
+        assert bool(((c.float() - want).abs() <= want.abs() * 2.0 ** -6 + 2e-2).all())
+
+
+@pytest.mark.gpu
+def test_split_calls_on_several_streams():
+    """Calls whose tiles are cut along K share neither scratch nor counters across streams."""
+    from symm_mem_recipes_b200.parallel import symm_mem
+
+    cases = [_operands(M, 1280, 4096) for M in (64, 200, 500)]
+    want = [a.float() @ b.float().t() for a, b in cases]
+    streams = [torch.cuda.Stream() for _ in cases]
+    torch.cuda.synchronize()
+    got = []
+    for _ in range(4):
+        for (a, b), st in zip(cases, streams):
+            with torch.cuda.stream(st):
+                got.append(_run(a, b, sms=48))           # three of them fit the GPU side by side
+    torch.cuda.synchronize()
+    symm_mem.check_status("cuda")
+    for i, c in enumerate(got):
+        ref = want[i % len(cases)]
+        assert bool(((c.float() - ref).abs() <= ref.abs() * 2.0 ** -6 + 2e-2).all())
