@@ -269,6 +269,60 @@ py::tuple host_all_reduce(const std::shared_ptr<HostSymmAllocation>& a, int64_t 
   return py::make_tuple(code, rank, 0, peer, (int)kWhereTwoShotExit, 0);
 }
 
+// The GEMM alone (no gather): checks, output, scratch and launch in one call.  Nothing when the operands are not what
+// the kernel takes: the caller's full path then says why.  epilogue: see AgMatmulArgs.
+c10::optional<torch::Tensor> matmul_local(const torch::Tensor& a, const torch::Tensor& b, const c10::optional<torch::Tensor>& out,
+                                        int epilogue, const c10::optional<torch::Tensor>& residual, int block_n, int num_sms,
+                                        bool split_k, int panel_w, uint64_t timeout_ns, int max_splits) {
+  const auto dtype = a.scalar_type();
+  const bool fp8 = dtype == at::kFloat8_e4m3fn;
+  if ((!fp8 && dtype != torch::kBFloat16) || !a.is_cuda()) return c10::nullopt;
+  const int dev = a.get_device();
+  auto ok = [dtype, dev](const torch::Tensor& t) {
+    return t.is_cuda() && t.get_device() == dev && t.dim() == 2 && t.is_contiguous() && t.scalar_type() == dtype &&
+           (uintptr_t)t.data_ptr() % 16 == 0;
+  };
+  if (!ok(a) || !ok(b) || a.size(1) != b.size(1)) return c10::nullopt;
+  const int64_t M = a.size(0), N = b.size(0), K = a.size(1), align = fp8 ? 16 : 8;
+  const bool swiglu = epilogue != 0;
+  if (M < 1 || N < 1 || K < 1 || N % align != 0 || K % align != 0 || epilogue < 0 || epilogue > 2) return c10::nullopt;
+  if (swiglu && (fp8 || N % (epilogue == 1 ? 256 : 16) != 0 || (block_n != 0 && block_n != 256))) return c10::nullopt;
+  const int64_t n_out = swiglu ? N / 2 : N;
+  if (out.has_value() && (!ok(*out) || out->size(0) != M || out->size(1) != n_out)) return c10::nullopt;
+  if (residual.has_value() && (fp8 || swiglu || !ok(*residual) || residual->size(0) != M || residual->size(1) != N))
+    return c10::nullopt;
+  c10::cuda::CUDAGuard guard(dev);
+  cudaStream_t stream = current_stream(dev);
+  torch::Tensor c = out.has_value() ? *out : at::empty({M, n_out}, a.options());
+  AgMatmulArgs args{};
+  args.a_local = a.data_ptr();
+  args.b = b.data_ptr();
+  args.c = c.data_ptr();
+  args.M = (int)M; args.N = (int)N; args.K = (int)K;
+  args.elem_bytes = fp8 ? 1 : 2;
+  args.epilogue = epilogue;
+  args.residual = residual ? residual->data_ptr() : nullptr;
+  args.num_sms = num_sms > 0 ? num_sms : at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  args.timeout_ns = timeout_ns;
+  args.status = status_for(dev);
+  args.panel_w = panel_w;
+  args.overlap = true;
+  const MatmulPlan plan = plan_matmul((int)M, (int)N, (int)K, args.elem_bytes, epilogue, block_n, args.num_sms,
+                                      split_k ? max_splits : 1);
+  args.block_n = plan.block_n;
+  torch::Tensor scratch, own_counters;
+  if (plan.tail_bytes > 0) {
+    scratch = at::empty({(int64_t)plan.tail_bytes}, a.options().dtype(torch::kUInt8));
+    args.tail_scratch = scratch.data_ptr();
+    args.tail_scratch_bytes = plan.tail_bytes;
+    args.tail_counters = tail_counters(dev, stream, own_counters);
+    args.tail_counter_slots = kTailCounterSlots;
+    args.tail_splits = plan.tail_splits;
+  }
+  rt_check(launch_ag_matmul_2cta(args, stream), "matmul");
+  return c;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -669,60 +723,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
      py::arg("push_ahead") = 0, py::arg("push_plain_stores") = false,
      py::arg("push_pieces") = 0, py::arg("panel_w") = 0);
 
-  // The GEMM alone (no gather): checks, output, scratch and launch in one call.  None when the operands are not
-  // what the kernel takes: the caller's full path then says why.  epilogue: see AgMatmulArgs.
-  m.def("matmul_local", [](const torch::Tensor& a, const torch::Tensor& b, const c10::optional<torch::Tensor>& out,
-                           int epilogue, const c10::optional<torch::Tensor>& residual, int block_n, int num_sms,
-                           bool split_k, int panel_w, uint64_t timeout_ns, int max_splits) -> c10::optional<torch::Tensor> {
-    const auto dtype = a.scalar_type();
-    const bool fp8 = dtype == at::kFloat8_e4m3fn;
-    if ((!fp8 && dtype != torch::kBFloat16) || !a.is_cuda()) return c10::nullopt;
-    const int dev = a.get_device();
-    auto ok = [dtype, dev](const torch::Tensor& t) {
-      return t.is_cuda() && t.get_device() == dev && t.dim() == 2 && t.is_contiguous() && t.scalar_type() == dtype &&
-             (uintptr_t)t.data_ptr() % 16 == 0;
-    };
-    if (!ok(a) || !ok(b) || a.size(1) != b.size(1)) return c10::nullopt;
-    const int64_t M = a.size(0), N = b.size(0), K = a.size(1), align = fp8 ? 16 : 8;
-    const bool swiglu = epilogue != 0;
-    if (M < 1 || N < 1 || K < 1 || N % align != 0 || K % align != 0 || epilogue < 0 || epilogue > 2) return c10::nullopt;
-    if (swiglu && (fp8 || N % (epilogue == 1 ? 256 : 16) != 0 || (block_n != 0 && block_n != 256))) return c10::nullopt;
-    const int64_t n_out = swiglu ? N / 2 : N;
-    if (out.has_value() && (!ok(*out) || out->size(0) != M || out->size(1) != n_out)) return c10::nullopt;
-    if (residual.has_value() && (fp8 || swiglu || !ok(*residual) || residual->size(0) != M || residual->size(1) != N))
-      return c10::nullopt;
-    c10::cuda::CUDAGuard guard(dev);
-    cudaStream_t stream = current_stream(dev);
-    torch::Tensor c = out.has_value() ? *out : at::empty({M, n_out}, a.options());
-    AgMatmulArgs args{};
-    args.a_local = a.data_ptr();
-    args.b = b.data_ptr();
-    args.c = c.data_ptr();
-    args.M = (int)M; args.N = (int)N; args.K = (int)K;
-    args.elem_bytes = fp8 ? 1 : 2;
-    args.epilogue = epilogue;
-    args.residual = residual ? residual->data_ptr() : nullptr;
-    args.num_sms = num_sms > 0 ? num_sms : at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-    args.timeout_ns = timeout_ns;
-    args.status = status_for(dev);
-    args.panel_w = panel_w;
-    args.overlap = true;
-    const MatmulPlan plan = plan_matmul((int)M, (int)N, (int)K, args.elem_bytes, epilogue, block_n, args.num_sms,
-                                        split_k ? max_splits : 1);
-    args.block_n = plan.block_n;
-    torch::Tensor scratch, own_counters;
-    if (plan.tail_bytes > 0) {
-      scratch = at::empty({(int64_t)plan.tail_bytes}, a.options().dtype(torch::kUInt8));
-      args.tail_scratch = scratch.data_ptr();
-      args.tail_scratch_bytes = plan.tail_bytes;
-      args.tail_counters = tail_counters(dev, stream, own_counters);
-      args.tail_counter_slots = kTailCounterSlots;
-      args.tail_splits = plan.tail_splits;
-    }
-    rt_check(launch_ag_matmul_2cta(args, stream), "matmul");
-    return c;
-  }, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("epilogue"), py::arg("residual"), py::arg("block_n"),
-     py::arg("num_sms"), py::arg("split_k"), py::arg("panel_w"), py::arg("timeout_ns"), py::arg("max_splits") = 0);
+  m.def("matmul_local", &matmul_local, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("epilogue"), py::arg("residual"),
+        py::arg("block_n"), py::arg("num_sms"), py::arg("split_k"), py::arg("panel_w"), py::arg("timeout_ns"),
+        py::arg("max_splits") = 0);
   m.def("release_tail_counters", &release_tail_counters);
 
   m.def("check_push_schedule", &check_push_schedule);
@@ -915,7 +918,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   }, py::arg("x"), py::arg("residual"), py::arg("w"), py::arg("sum_out"), py::arg("out"), py::arg("eps"));
   // `pos` (optional): int32 CUDA tensor of one element that holds the first position; read on the device
   m.def("rope_inplace", [](torch::Tensor qkv, int n_heads, int head_dim, int seq, int pos0, double theta,
-                           int num_sms, c10::optional<torch::Tensor> pos) {
+                           int /*num_sms*/, c10::optional<torch::Tensor> pos) {
     TORCH_CHECK(qkv.is_cuda() && qkv.is_contiguous() && qkv.dim() == 2 && qkv.scalar_type() == torch::kBFloat16,
                 "rope_inplace: qkv[tokens, row] contiguous bf16 on the GPU");
     int dev = qkv.get_device();
@@ -924,7 +927,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                 "rope_inplace: pos must be an int32 tensor of one element on qkv's GPU");
     c10::cuda::CUDAGuard guard(dev);
     rt_check(launch_rope_inplace(qkv.data_ptr(), qkv.size(0), (int)qkv.size(1), n_heads, head_dim, seq, pos0,
-                                 pos ? static_cast<const int*>(pos->data_ptr()) : nullptr, (float)theta, num_sms,
+                                 pos ? static_cast<const int*>(pos->data_ptr()) : nullptr, (float)theta,
                                  current_stream(dev)), "rope_inplace");
   }, py::arg("qkv"), py::arg("n_heads"), py::arg("head_dim"), py::arg("seq"), py::arg("pos0"), py::arg("theta"),
      py::arg("num_sms"), py::arg("pos") = py::none());
@@ -970,6 +973,62 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
              "decode_attention");
   }, py::arg("qkv"), py::arg("k_cache"), py::arg("v_cache"), py::arg("out"), py::arg("scratch"), py::arg("hq"),
      py::arg("hkv"), py::arg("pos0"), py::arg("pos") = py::none(), py::arg("rope_theta") = 0.0);
+
+  // Prefill of a layer whose projections have nobody to reduce with (a world of one): norm, QKV, rotation (which also
+  // fills the caches), attention, then three GEMMs whose epilogues carry the residual adds and the activation.
+  // One call, because on a short prompt the kernels take less time than Python needs to issue them.  None
+  // when the operands are not what these kernels take.
+  m.def("prefill_layer", [](const torch::Tensor& x, int64_t batch, int64_t seq, const c10::optional<torch::Tensor>& k_cache,
+                            const c10::optional<torch::Tensor>& v_cache, const torch::Tensor& w_qkv,
+                            const torch::Tensor& w_o, const torch::Tensor& w_gate_up, const torch::Tensor& w_down,
+                            const torch::Tensor& norm1, const torch::Tensor& norm2, int64_t hq, int64_t hkv, int64_t D,
+                            double eps, double rope_theta, uint64_t timeout_ns) -> c10::optional<torch::Tensor> {
+    const int dev = x.is_cuda() ? x.get_device() : -1;
+    auto ok = [dev](const torch::Tensor& t, int64_t dim) {
+      return t.is_cuda() && t.get_device() == dev && t.dim() == dim && t.is_contiguous() &&
+             t.scalar_type() == torch::kBFloat16 && (uintptr_t)t.data_ptr() % 16 == 0;
+    };
+    if (!ok(x, 2) || !ok(w_qkv, 2) || !ok(w_o, 2) || !ok(w_gate_up, 2) || !ok(w_down, 2) || !ok(norm1, 1) || !ok(norm2, 1))
+      return c10::nullopt;
+    const int64_t T = x.size(0), H = x.size(1), F = w_down.size(1), heads = hq + 2 * hkv;
+    if (T < 1 || batch < 1 || seq < 1 || T != batch * seq || H % 8 != 0 || F % 8 != 0 || D % 16 != 0 || D < 16 || hkv < 1 ||
+        hq % hkv != 0 || w_qkv.size(0) != heads * D || w_qkv.size(1) != H || w_o.size(0) != H || w_o.size(1) != hq * D ||
+        w_gate_up.size(0) != 2 * F || w_gate_up.size(1) != H || w_down.size(0) != H || norm1.size(0) != H ||
+        norm2.size(0) != H || rope_theta <= 1.0 || k_cache.has_value() != v_cache.has_value())
+      return c10::nullopt;
+    if (k_cache.has_value() &&
+        (!ok(*k_cache, 4) || !ok(*v_cache, 4) || k_cache->sizes() != v_cache->sizes() || k_cache->size(0) != batch ||
+         k_cache->size(1) < seq || k_cache->size(2) != hkv || k_cache->size(3) != D))
+      return c10::nullopt;
+    c10::cuda::CUDAGuard guard(dev);
+    cudaStream_t stream = current_stream(dev);
+    auto norm = [&](const torch::Tensor& in, const torch::Tensor& w) {
+      torch::Tensor out = at::empty_like(in);
+      rt_check(launch_rms_norm(in.data_ptr(), nullptr, w.data_ptr(), nullptr, out.data_ptr(), (int)T, (int)H, (float)eps,
+                               stream), "prefill_layer");
+      return out;
+    };
+    auto gemm = [&](const torch::Tensor& a, const torch::Tensor& b, int epilogue, const c10::optional<torch::Tensor>& residual) {
+      auto c = matmul_local(a, b, c10::nullopt, epilogue, residual, 0, 0, true, 0, timeout_ns, 0);
+      TORCH_CHECK(c.has_value(), "prefill_layer: operands refused by the GEMM");
+      return *c;
+    };
+    torch::Tensor qkv = gemm(norm(x, norm1), w_qkv, 0, c10::nullopt);
+    rt_check(launch_rope_inplace(qkv.data_ptr(), T, (int)(heads * D), (int)(hq + hkv), (int)D, (int)seq, 0, nullptr,
+                                 (float)rope_theta, stream, k_cache ? k_cache->data_ptr() : nullptr,
+                                 v_cache ? v_cache->data_ptr() : nullptr, k_cache ? (int)k_cache->size(1) : 0, (int)hkv),
+             "prefill_layer");
+    const torch::Tensor by_head = qkv.view({batch, seq, heads, D}).transpose(1, 2);
+    torch::Tensor o = at::scaled_dot_product_attention(by_head.narrow(1, 0, hq), by_head.narrow(1, hq, hkv),
+                                                       by_head.narrow(1, hq + hkv, hkv), c10::nullopt, 0.0, true,
+                                                       c10::nullopt, true);
+    o = o.transpose(1, 2).reshape({T, hq * D}).contiguous();
+    const torch::Tensor x1 = gemm(o, w_o, 0, x);
+    const torch::Tensor act = gemm(norm(x1, norm2), w_gate_up, 2, c10::nullopt);
+    return gemm(act, w_down, 0, x1);
+  }, py::arg("x"), py::arg("batch"), py::arg("seq"), py::arg("k_cache"), py::arg("v_cache"), py::arg("w_qkv"),
+     py::arg("w_o"), py::arg("w_gate_up"), py::arg("w_down"), py::arg("norm1"), py::arg("norm2"), py::arg("hq"),
+     py::arg("hkv"), py::arg("head_dim"), py::arg("eps"), py::arg("rope_theta"), py::arg("timeout_ns"));
 
   // One decode step of a layer whose projections have nobody to reduce with (a world of one): five launches,
   // each started under its predecessor.  `ss`: what this function returned beside the x it is given, or None

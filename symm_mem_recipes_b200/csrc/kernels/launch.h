@@ -197,8 +197,11 @@ int launch_row_sum_squares(const void* x, float* ss, int rows, int H, cudaStream
 // Rotary embedding in place on heads [0, n_heads) of every row (`row_stride` elements per row);
 // token t is at position pos0 + t % seq, with pos0 read from `pos_dev` on the device when that is
 // not null (graph-captured decode).  head_dim % 16 == 0.
+// With caches [tokens / seq, s_max, hkv, head_dim] (and positions from 0) the last hkv rotated heads and the hkv heads
+// after them are also written there.
 int launch_rope_inplace(void* qkv, long long tokens, int row_stride, int n_heads, int head_dim, int seq, int pos0,
-                        const int* pos_dev, float theta, int num_sms, cudaStream_t stream);
+                        const int* pos_dev, float theta, cudaStream_t stream, void* k_cache = nullptr,
+                        void* v_cache = nullptr, int s_max = 0, int hkv = 0);
 // out[rows, F] = SiLU(gate_up[:, :F]) * gate_up[:, F:].  F % 8 == 0.
 int launch_silu_mul(const void* gate_up, void* out, long long rows, int F, int num_sms, cudaStream_t stream);
 // Attention of one decode step: qkv [batch, (hq + 2 hkv) * head_dim] (new token, keys already rotated),

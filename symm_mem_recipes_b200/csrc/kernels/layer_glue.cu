@@ -17,14 +17,15 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
+#include "../device/pdl.cuh"
 #include "../device/vec.cuh"
 #include "launch.h"
 
 namespace smr {
 
 namespace {
-
-constexpr int kNormThreads = 256;
 
 __device__ __forceinline__ void unpack8(const Vec16& v, float (&f)[8]) {
   f[0] = bf16lo_to_f32(v.x); f[1] = bf16hi_to_f32(v.x);
@@ -42,69 +43,116 @@ __device__ __forceinline__ float round_bf16(float f) {
   return __bfloat162float(__float2bfloat16_rn(f));
 }
 
-// One CTA per row.  Pass 1: s = x (+ r), sum of squares (s stored when asked
-// for).  Pass 2 re-reads s (from L1 / L2) and writes the normalised row.
-// `sum_out` may be the buffer of `x` or of `residual` (running residual stream
+// A CTA takes rows blockIdx.x, blockIdx.x + gridDim.x, ...; a row lives in registers (VPT vectors of eight per thread):
+// x and the residual are read once, s and the result written once, and the next row is loaded before this one is
+// reduced, so that the reduction's latency is not a hole in the memory stream.  The weight stays in registers.
+// Bound by HBM for a prefill (32768 x 8192: 235 us with a second pass over the row; 1.07 GB are 164 us at
+// the measured copy rate), by latency for a handful of rows, which is why a row is spread over up to 1024
+// threads there.  `sum_out` may be the buffer of `x` or of `residual` (running residual stream
 // updated in place) and `out` may be the buffer of `x`; `out` must not be the
 // buffer of `sum_out` or of `residual`.
-__global__ void __launch_bounds__(kNormThreads)
+template <int THREADS, int VPT, bool kResidual>
+__global__ void __launch_bounds__(THREADS, THREADS > 256 ? 1 : (VPT <= 2 ? 4 : (VPT == 4 && !kResidual ? 3 : (VPT == 4 ? 2 : 1))))
 rms_norm_kernel(const __nv_bfloat16* x, const __nv_bfloat16* residual, const __nv_bfloat16* __restrict__ w,
-                __nv_bfloat16* sum_out, __nv_bfloat16* out, int H, float eps) {
+                __nv_bfloat16* sum_out, __nv_bfloat16* out, int rows, int H, float eps) {
+  pdl_launch_dependents();
+  const int n_vec = H / 8;
+  Vec16 g[VPT], s[VPT], r[kResidual ? VPT : 1];
+  pdl_wait();
+#pragma unroll
+  for (int j = 0; j < VPT; ++j)
+    g[j] = threadIdx.x + j * THREADS < n_vec ? ld_16(reinterpret_cast<const Vec16*>(w) + threadIdx.x + j * THREADS)
+                                             : Vec16{0u, 0u, 0u, 0u};
+  auto fetch = [&](int row) {
+    const Vec16* xr = reinterpret_cast<const Vec16*>(x + (size_t)row * H);
+    const Vec16* rr = reinterpret_cast<const Vec16*>(residual + (size_t)row * H);
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+      const int i = threadIdx.x + j * THREADS;
+      s[j] = i < n_vec ? ld_16_stream(xr + i) : Vec16{0u, 0u, 0u, 0u};
+      if constexpr (kResidual) r[j] = i < n_vec ? ld_16_stream(rr + i) : Vec16{0u, 0u, 0u, 0u};
+    }
+  };
+  __shared__ float warp_sums[2][THREADS / 32];
+  int parity = 0;
+  fetch(blockIdx.x);
+  for (int row = blockIdx.x; row < rows; row += gridDim.x, parity ^= 1) {
+    Vec16 v[VPT];
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+      v[j] = s[j];
+      if constexpr (kResidual) {
+        v[j] = add_bf16x8(v[j], r[j]);
+        const int i = threadIdx.x + j * THREADS;
+        if (i < n_vec && sum_out != nullptr) st_16(reinterpret_cast<Vec16*>(sum_out + (size_t)row * H) + i, v[j]);
+      }
+      float a[8];
+      unpack8(v[j], a);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) ss += a[q] * a[q];
+    }
+    if (row + (int)gridDim.x < rows) fetch(row + gridDim.x);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if ((threadIdx.x & 31) == 0) warp_sums[parity][threadIdx.x >> 5] = ss;
+    __syncthreads();
+    float t = (threadIdx.x & 31) < THREADS / 32 ? warp_sums[parity][threadIdx.x & 31] : 0.f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    const float scale = rsqrtf(t / (float)H + eps);
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+      const int i = threadIdx.x + j * THREADS;
+      float a[8], b[8];
+      unpack8(v[j], a);
+      unpack8(g[j], b);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) a[q] = round_bf16(a[q] * scale) * b[q];
+      if (i < n_vec) st_16(reinterpret_cast<Vec16*>(out + (size_t)row * H) + i, pack8(a));
+    }
+  }
+}
+
+// Rows too long for registers (H > 16384): one CTA per row, two passes.  Pass 2 re-reads s (from L1 / L2).
+__global__ void __launch_bounds__(256)
+rms_norm_long_kernel(const __nv_bfloat16* x, const __nv_bfloat16* residual, const __nv_bfloat16* __restrict__ w,
+                     __nv_bfloat16* sum_out, __nv_bfloat16* out, int H, float eps) {
   const size_t row = blockIdx.x;
   const Vec16* xr = reinterpret_cast<const Vec16*>(x + row * H);
   const Vec16* rr = residual ? reinterpret_cast<const Vec16*>(residual + row * H) : nullptr;
   Vec16* sr = sum_out ? reinterpret_cast<Vec16*>(sum_out + row * H) : nullptr;
   const int n_vec = H / 8;
   float ss = 0.f;
-  for (int i = threadIdx.x; i < n_vec; i += kNormThreads) {
+  for (int i = threadIdx.x; i < n_vec; i += 256) {
+    Vec16 v = ld_16(xr + i);
+    if (rr != nullptr) v = add_bf16x8(v, ld_16(rr + i));
+    if (sr != nullptr) st_16(sr + i, v);
     float a[8];
-    unpack8(ld_16(xr + i), a);
-    if (rr != nullptr) {
-      float b[8];
-      unpack8(ld_16(rr + i), b);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) a[q] = round_bf16(a[q] + b[q]);
-      if (sr != nullptr) st_16(sr + i, pack8(a));
-    }
+    unpack8(v, a);
 #pragma unroll
     for (int q = 0; q < 8; ++q) ss += a[q] * a[q];
   }
-  // block sum
-  __shared__ float warp_sums[kNormThreads / 32];
-  __shared__ float scale_s;
+  __shared__ float warp_sums[8];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
   if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = ss;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    float t = threadIdx.x < kNormThreads / 32 ? warp_sums[threadIdx.x] : 0.f;
+  float t = 0.f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (threadIdx.x == 0) scale_s = rsqrtf(t / (float)H + eps);
-  }
-  __syncthreads();
-  const float scale = scale_s;
-  const Vec16* wr = reinterpret_cast<const Vec16*>(w);
-  Vec16* orow = reinterpret_cast<Vec16*>(out + row * H);
-  for (int i = threadIdx.x; i < n_vec; i += kNormThreads) {
+  for (int i = 0; i < 8; ++i) t += warp_sums[i];
+  const float scale = rsqrtf(t / (float)H + eps);
+  for (int i = threadIdx.x; i < n_vec; i += 256) {
+    // this thread stored s[i] itself in pass 1; reading it back (instead of x and r again) also
+    // keeps the kernel correct when sum_out is the same buffer as x or as the residual
+    Vec16 v = ld_16(sr != nullptr ? sr + i : xr + i);
+    if (sr == nullptr && rr != nullptr) v = add_bf16x8(v, ld_16(rr + i));
     float a[8], g[8];
-    if (sr != nullptr) {
-      // this thread stored s[i] itself in pass 1; reading it back (instead of x and r again) also
-      // keeps the kernel correct when sum_out is the same buffer as x or as the residual
-      unpack8(ld_16(sr + i), a);
-    } else {
-      unpack8(ld_16(xr + i), a);
-      if (rr != nullptr) {
-        float b[8];
-        unpack8(ld_16(rr + i), b);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) a[q] = round_bf16(a[q] + b[q]);
-      }
-    }
-    unpack8(ld_16(wr + i), g);
+    unpack8(v, a);
+    unpack8(ld_16(reinterpret_cast<const Vec16*>(w) + i), g);
 #pragma unroll
     for (int q = 0; q < 8; ++q) a[q] = round_bf16(a[q] * scale) * g[q];
-    st_16(orow + i, pack8(a));
+    st_16(reinterpret_cast<Vec16*>(out + row * H) + i, pack8(a));
   }
 }
 
@@ -136,37 +184,81 @@ __global__ void __launch_bounds__(512) row_sum_squares_kernel(const __nv_bfloat1
 // In place on rows of `row_stride` elements: heads [0, n_heads) of D elements
 // each are rotated.  Token t sits at position pos0 + (t % seq); with `pos_dev`
 // the first position is read from device memory instead (a decode step
-// captured in a CUDA graph takes its position from a tensor).  One thread per
-// (token, head, 8 consecutive pair indices).
-__global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, long long n_items, int row_stride, int n_heads, int D,
-                            int seq, int pos0, const int* __restrict__ pos_dev, float log2_theta) {
+// captured in a CUDA graph takes its position from a tensor).
+// With caches ([tokens / seq, s_max, hkv, D] each) the last hkv of the rotated heads are also written to the key cache
+// and the hkv heads after them to the value cache, at the token's place in its sequence.
+// A warp takes a token: its angles are computed once into shared memory (a sine and cosine per pair instead of one per
+// pair and head), then a lane rotates eight pairs of a head at a time, two heads' loads in flight.  Bound by HBM: at
+// 32768 tokens of 9 heads x 128 the kernel with the angles per head took 47 us and the two cache copies 34.
+__global__ void __launch_bounds__(256)
+rope_kernel(__nv_bfloat16* __restrict__ qkv, long long tokens, int row_stride, int n_heads, int D, int seq, int pos0,
+            const int* __restrict__ pos_dev, float log2_theta, __nv_bfloat16* __restrict__ k_cache,
+            __nv_bfloat16* __restrict__ v_cache, int s_max, int hkv) {
+  extern __shared__ float2 angles[];                    // [warps][D / 2] (cos, sin)
+  pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, half = D / 2;
+  const long long t = (long long)blockIdx.x * (blockDim.x >> 5) + warp;
+  pdl_wait();
+  if (t >= tokens) return;
   if (pos_dev != nullptr) pos0 = *pos_dev;
-  const int vec_per_head = D / 16;                      // vectors of 8 pairs
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long item = (long long)blockIdx.x * blockDim.x + threadIdx.x; item < n_items; item += stride) {
-    const int v = (int)(item % vec_per_head);
-    const long long th = item / vec_per_head;
-    const int head = (int)(th % n_heads);
-    const long long t = th / n_heads;
-    const float pos = (float)(pos0 + (int)(t % seq));
-    __nv_bfloat16* base = qkv + t * row_stride + (long long)head * D + v * 8;
-    float x1[8], x2[8], y1[8], y2[8];
-    unpack8(ld_16(base), x1);
-    unpack8(ld_16(base + D / 2), x2);
+  const long long in_batch = t / seq;
+  const int in_seq = (int)(t - in_batch * seq);
+  float2* mine = angles + warp * half;
+  for (int i = lane; i < half; i += 32) {               // pair index in [0, D/2)
+    const float inv_freq = exp2f(-(2.0f * (float)i / (float)D) * log2_theta);
+    float ang = (float)(pos0 + in_seq) * inv_freq;
+    // bring the angle into [-pi, pi] before the fast sine / cosine
+    ang -= 6.283185307179586f * rintf(ang * 0.15915494309189535f);
+    float sn, cs;
+    __sincosf(ang, &sn, &cs);
+    mine[i] = make_float2(cs, sn);
+  }
+  __syncwarp();
+  const int vecs = D / 16;                              // items of eight pairs per head
+  const int n_items = (n_heads + (v_cache != nullptr ? hkv : 0)) * vecs;
+  __nv_bfloat16* row = qkv + t * row_stride;
+  const size_t cache_row = ((size_t)in_batch * s_max + in_seq) * hkv;   // the token's row of a cache, in heads
+  for (int item0 = lane; item0 < n_items; item0 += 64) {
+    Vec16 lo[2], hi[2];
+    int head[2], v[2];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int i = v * 8 + q;                          // pair index in [0, D/2)
-      const float inv_freq = exp2f(-(2.0f * (float)i / (float)D) * log2_theta);
-      float ang = pos * inv_freq;
-      // bring the angle into [-pi, pi] before the fast sine / cosine
-      ang -= 6.283185307179586f * rintf(ang * 0.15915494309189535f);
-      float sn, cs;
-      __sincosf(ang, &sn, &cs);
-      y1[q] = x1[q] * cs - x2[q] * sn;
-      y2[q] = x2[q] * cs + x1[q] * sn;
+    for (int u = 0; u < 2; ++u) {
+      const int item = item0 + 32 * u;
+      head[u] = item / vecs;
+      v[u] = (item - head[u] * vecs) * 8;
+      if (item < n_items) {
+        lo[u] = ld_16_stream(row + (size_t)head[u] * D + v[u]);
+        hi[u] = ld_16_stream(row + (size_t)head[u] * D + half + v[u]);
+      }
     }
-    st_16(base, pack8(y1));
-    st_16(base + D / 2, pack8(y2));
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (item0 + 32 * u >= n_items) continue;
+      if (head[u] >= n_heads) {                         // a value head: only copied
+        __nv_bfloat16* dst = v_cache + (cache_row + (head[u] - n_heads)) * D + v[u];
+        st_16(dst, lo[u]);
+        st_16(dst + half, hi[u]);
+        continue;
+      }
+      float x1[8], x2[8], y1[8], y2[8];
+      unpack8(lo[u], x1);
+      unpack8(hi[u], x2);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float2 c = mine[v[u] + q];
+        y1[q] = x1[q] * c.x - x2[q] * c.y;
+        y2[q] = x2[q] * c.x + x1[q] * c.y;
+      }
+      const Vec16 o1 = pack8(y1), o2 = pack8(y2);
+      __nv_bfloat16* src = row + (size_t)head[u] * D + v[u];
+      st_16(src, o1);
+      st_16(src + half, o2);
+      if (k_cache != nullptr && head[u] >= n_heads - hkv) {
+        __nv_bfloat16* dst = k_cache + (cache_row + (head[u] - (n_heads - hkv))) * D + v[u];
+        st_16(dst, o1);
+        st_16(dst + half, o2);
+      }
+    }
   }
 }
 
@@ -207,11 +299,37 @@ int launch_rms_norm(const void* x, const void* residual, const void* w, void* su
     return cudaErrorInvalidValue;
   if (sum_out != nullptr && residual == nullptr) return cudaErrorInvalidValue;
   if (rows == 0) return cudaSuccess;
-  rms_norm_kernel<<<rows, kNormThreads, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(residual),
-      static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(sum_out), static_cast<__nv_bfloat16*>(out),
-      H, eps);
-  return (int)cudaGetLastError();
+  const int n_vec = H / 8;
+  const auto xb = static_cast<const __nv_bfloat16*>(x), rb = static_cast<const __nv_bfloat16*>(residual);
+  const auto wb = static_cast<const __nv_bfloat16*>(w);
+  const auto sb = static_cast<__nv_bfloat16*>(sum_out), ob = static_cast<__nv_bfloat16*>(out);
+  if (n_vec > 2048) {
+    rms_norm_long_kernel<<<rows, 256, 0, stream>>>(xb, rb, wb, sb, ob, H, eps);
+    return (int)cudaGetLastError();
+  }
+  auto go = [&](auto kernel, int threads, int per_sm) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(rows < 148 * per_sm ? rows : 148 * per_sm));
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, xb, rb, wb, sb, ob, rows, H, eps);
+  };
+  // fewer rows than SMs: one vector per thread, the shortest chain; else 256 threads, as many CTAs as the
+  // registers of the widest rows allow per SM
+  auto pick = [&](auto res) {
+    constexpr bool R = decltype(res)::value;
+    if (rows < 148 && n_vec > 256 && n_vec <= 1024) return go(rms_norm_kernel<1024, 1, R>, 1024, 1);
+    if (n_vec <= 256) return go(rms_norm_kernel<256, 1, R>, 256, 4);
+    if (n_vec <= 512) return go(rms_norm_kernel<256, 2, R>, 256, 4);
+    if (n_vec <= 1024) return go(rms_norm_kernel<256, 4, R>, 256, R ? 2 : 3);
+    return go(rms_norm_kernel<256, 8, R>, 256, 1);
+  };
+  return residual != nullptr ? pick(std::true_type{}) : pick(std::false_type{});
 }
 
 int launch_row_sum_squares(const void* x, float* ss, int rows, int H, cudaStream_t stream) {
@@ -221,15 +339,34 @@ int launch_row_sum_squares(const void* x, float* ss, int rows, int H, cudaStream
 }
 
 int launch_rope_inplace(void* qkv, long long tokens, int row_stride, int n_heads, int head_dim, int seq, int pos0,
-                        const int* pos_dev, float theta, int num_sms, cudaStream_t stream) {
+                        const int* pos_dev, float theta, cudaStream_t stream, void* k_cache, void* v_cache, int s_max,
+                        int hkv) {
   if (tokens < 0 || n_heads < 1 || head_dim < 16 || head_dim % 16 != 0 || seq < 1 || row_stride % 8 != 0 ||
       (long long)n_heads * head_dim > row_stride || theta <= 1.0f || !aligned16(qkv))
     return cudaErrorInvalidValue;
+  if ((k_cache == nullptr) != (v_cache == nullptr)) return cudaErrorInvalidValue;
+  if (k_cache != nullptr &&
+      (hkv < 1 || hkv > n_heads || (long long)(n_heads + hkv) * head_dim > row_stride || s_max < seq || tokens % seq != 0 ||
+       pos_dev != nullptr || pos0 != 0 || !aligned16(k_cache) || !aligned16(v_cache)))
+    return cudaErrorInvalidValue;
   if (tokens == 0) return cudaSuccess;
-  const long long items = tokens * n_heads * (head_dim / 16);
-  rope_kernel<<<grid_for(items, 256, num_sms), 256, 0, stream>>>(static_cast<__nv_bfloat16*>(qkv), items, row_stride,
-                                                                n_heads, head_dim, seq, pos0, pos_dev, log2f(theta));
-  return (int)cudaGetLastError();
+  int warps = 8;                                        // fewer where the tables of eight heads would not fit
+  while (warps > 1 && (size_t)warps * (head_dim / 2) * sizeof(float2) > 48 * 1024) warps >>= 1;
+  const size_t smem = (size_t)warps * (head_dim / 2) * sizeof(float2);
+  if (smem > 48 * 1024) return cudaErrorInvalidValue;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)((tokens + warps - 1) / warps));
+  cfg.blockDim = dim3((unsigned)warps * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, rope_kernel, static_cast<__nv_bfloat16*>(qkv), tokens, row_stride, n_heads,
+                                 head_dim, seq, pos0, pos_dev, log2f(theta), static_cast<__nv_bfloat16*>(k_cache),
+                                 static_cast<__nv_bfloat16*>(v_cache), s_max, hkv);
 }
 
 int launch_silu_mul(const void* gate_up, void* out, long long rows, int F, int num_sms, cudaStream_t stream) {

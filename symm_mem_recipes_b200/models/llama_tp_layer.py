@@ -222,6 +222,18 @@ class LlamaTPDecoderLayer:
     def _mlp_act(self, gu: torch.Tensor) -> torch.Tensor:
         return ops.silu_mul(gu) if self.fused_glue else self._mlp_act_torch(gu, self.ffn_local)
 
+    def _prefill_local(self, x: torch.Tensor, batch: int, seq: int, kv_cache) -> Optional[torch.Tensor]:
+        """The prefill of a world of one in one native call (the residual adds and SiLU-mul ride in the
+        GEMMs' epilogues, the rotation fills the caches), or None where it has to be composed of
+        single ops: with peers, without the glue kernels, off the GPU, or for operands it does not take."""
+        if self.ws != 1 or not self.fused_glue or not x.is_cuda or os.environ.get("SMR_SDPA_CUDNN", "0") == "1":
+            return None
+        k_cache, v_cache = kv_cache if kv_cache is not None else (None, None)
+        cfg = self.cfg
+        return C.prefill_layer(x, batch, seq, k_cache, v_cache, self.w_qkv, self.w_o, self.w_gate_up, self.w_down,
+                               self.norm1, self.norm2, self.hq, self.hkv, cfg.head_dim, cfg.eps, cfg.rope_theta,
+                               _TIMEOUT_NS)
+
     # ------------------------------------------------------------------
     def forward(self, x_shard: torch.Tensor, batch: int, seq: int, barrier_between_phases: bool = False,
                 kv_cache=None) -> torch.Tensor:
@@ -230,6 +242,10 @@ class LlamaTPDecoderLayer:
         cfg = self.cfg
         rows = x_shard.shape[0]
         assert rows * self.ws == batch * seq
+        if not barrier_between_phases and self.phase_marks is None:
+            y = self._prefill_local(x_shard, batch, seq, kv_cache)
+            if y is not None:
+                return y
         h = self._symmetric("attn_in", rows)
         self._mark("start")
         if self.fused_glue:
@@ -277,6 +293,9 @@ class LlamaTPDecoderLayer:
         full [batch*seq, H] output, identical on every rank."""
         cfg = self.cfg
         assert x.shape[0] == batch * seq
+        y = self._prefill_local(x, batch, seq, kv_cache)
+        if y is not None:
+            return y
         h = ops.rms_norm(x, self.norm1, cfg.eps) if self.fused_glue else _rms_norm(x, self.norm1, cfg.eps)
         qkv = ops.matmul(h, self.w_qkv)
         attn = self._attention(qkv, batch, seq, glue=self.fused_glue, kv_cache=kv_cache)
