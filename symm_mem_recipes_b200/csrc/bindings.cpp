@@ -16,6 +16,7 @@
 #include <mutex>
 #include <thread>
 
+#include "kernels/decode_stack.h"
 #include "kernels/gemv_local.h"
 #include "kernels/launch.h"
 #include "oracle/cpu_reference.h"
@@ -1030,92 +1031,66 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
      py::arg("w_o"), py::arg("w_gate_up"), py::arg("w_down"), py::arg("norm1"), py::arg("norm2"), py::arg("hq"),
      py::arg("hkv"), py::arg("head_dim"), py::arg("eps"), py::arg("rope_theta"), py::arg("timeout_ns"));
 
-  // One decode step of a layer whose projections have nobody to reduce with (a world of one): five launches,
-  // each started under its predecessor.  `ss`: what this function returned beside the x it is given, or None
-  // (then the sums of squares of x are taken by a kernel of their own).  That first kernel, or the first of
-  // the chain that produced x, is an ordinary launch, so weights, caches and `pos` written before it are
-  // safe to read early.  Returns (y, ss of y), or None when the operands are not what these kernels take.
-  m.def("decode_layer", [](const torch::Tensor& x, const c10::optional<torch::Tensor>& ss, const torch::Tensor& k_cache,
-                           const torch::Tensor& v_cache, int64_t pos0, const c10::optional<torch::Tensor>& pos,
-                           const torch::Tensor& w_qkv, const torch::Tensor& w_o, const torch::Tensor& w_gate_up,
-                           const torch::Tensor& w_down, const torch::Tensor& norm1, const torch::Tensor& norm2, int hq,
-                           double eps, double rope_theta, const torch::Tensor& scratch,
-                           uint64_t timeout_ns) -> c10::optional<std::pair<torch::Tensor, torch::Tensor>> {
+  // One decode step through layers whose projections have nobody to reduce with (a world of one): a persistent kernel
+  // for up to eight layers at a time.  Per layer: w_qkv, w_o, w_gate_up, w_down, norm1, norm2, k_cache, v_cache.
+  // None when the operands are not what the kernel takes.
+  m.def("decode_stack", [](const torch::Tensor& x, const std::vector<torch::Tensor>& tensors, int64_t pos0,
+                           const c10::optional<torch::Tensor>& pos, int hq, double eps, double rope_theta,
+                           uint64_t timeout_ns) -> c10::optional<torch::Tensor> {
     const int dev = x.is_cuda() ? x.get_device() : -1;
     auto ok = [dev](const torch::Tensor& t, int64_t dim) {
       return t.is_cuda() && t.get_device() == dev && t.dim() == dim && t.is_contiguous() &&
              t.scalar_type() == torch::kBFloat16 && (uintptr_t)t.data_ptr() % 16 == 0;
     };
-    if (!ok(x, 2) || !ok(k_cache, 4) || !ok(v_cache, 4) || !ok(w_qkv, 2) || !ok(w_o, 2) || !ok(w_gate_up, 2) ||
-        !ok(w_down, 2) || !ok(norm1, 1) || !ok(norm2, 1))
-      return c10::nullopt;
-    const int64_t B = x.size(0), H = x.size(1), S = k_cache.size(1), hkv = k_cache.size(2), D = k_cache.size(3);
-    const int64_t F = w_down.size(1), qkv_n = (hq + 2 * hkv) * D;
-    if (B < 1 || B > 16 || H % 8 != 0 || F % 8 != 0 || (D != 64 && D != 128) || hkv < 1 || hq % hkv != 0 ||
-        hq / hkv > 8 || k_cache.size(0) != B || v_cache.sizes() != k_cache.sizes() || w_qkv.size(0) != qkv_n ||
-        w_qkv.size(1) != H || w_o.size(0) != H || w_o.size(1) != hq * D || w_gate_up.size(0) != 2 * F ||
-        w_gate_up.size(1) != H || w_down.size(0) != H || norm1.size(0) != H || norm2.size(0) != H ||
-        rope_theta <= 1.0 || (!pos.has_value() && (pos0 < 0 || pos0 >= S)))
+    constexpr size_t kPer = 8;
+    if (!ok(x, 2) || tensors.empty() || tensors.size() % kPer != 0) return c10::nullopt;
+    const torch::Tensor& kc0 = tensors[6];
+    if (!ok(kc0, 4) || !ok(tensors[3], 2)) return c10::nullopt;
+    const int64_t B = x.size(0), H = x.size(1), F = tensors[3].size(1), S = kc0.size(1), hkv = kc0.size(2), D = kc0.size(3);
+    if (B < 1 || B > 16 || hq < 1 || hkv < 1 || hq % hkv != 0 || kc0.size(0) != B || rope_theta <= 1.0 ||
+        (!pos.has_value() && (pos0 < 0 || pos0 >= S)))
       return c10::nullopt;
     if (pos.has_value() && !(pos->is_cuda() && pos->get_device() == dev && pos->numel() == 1 &&
                              pos->scalar_type() == torch::kInt32))
       return c10::nullopt;
-    c10::cuda::CUDAGuard guard(dev);
-    cudaStream_t stream = current_stream(dev);
-    const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-    GemvLocalArgs g{};
-    g.batch = (int)B;
-    g.weights_nk = g.overlap = g.static_w = true;
-    g.eps = (float)eps;
-    g.num_sms = sms;
-    g.timeout_ns = timeout_ns;
-    g.status = status_for(dev);
-    const auto f32 = x.options().dtype(torch::kFloat32);
-    auto slots = [&](int64_t n, int64_t k) {
-      const int ctas = gemv_local_ctas((int)n, (int)k, true, false, sms);
-      TORCH_CHECK(ctas > 0, "decode_layer: ", cudaGetErrorString((cudaError_t)-ctas));
-      return at::empty({ctas, 16}, f32);
-    };
-    auto project = [&](const torch::Tensor& in, const torch::Tensor& w, const torch::Tensor& out, const torch::Tensor* norm,
-                       const torch::Tensor* ss_in, bool silu, const torch::Tensor* residual, const torch::Tensor* ss_out) {
-      GemvLocalArgs a = g;
-      a.x = in.data_ptr(); a.w = w.data_ptr(); a.out = out.data_ptr();
-      a.K = (int)w.size(1); a.N = (int)w.size(0);
-      if (norm != nullptr) {
-        a.norm_w = norm->data_ptr();
-        a.ss_in = ss_in->data_ptr<float>();
-        a.n_ss = (int)ss_in->size(0);
-      }
-      a.silu = silu;
-      if (residual != nullptr) a.residual = residual->data_ptr();
-      if (ss_out != nullptr) a.ss_out = ss_out->data_ptr<float>();
-      rt_check(launch_gemv_local(a, stream), "decode_layer");
-    };
-    torch::Tensor ss_x;
-    if (ss.has_value()) {
-      ss_x = *ss;
-      TORCH_CHECK(ss_x.is_cuda() && ss_x.dim() == 2 && ss_x.size(1) == 16 && ss_x.is_contiguous() &&
-                  ss_x.scalar_type() == torch::kFloat32, "ss must be what an earlier call returned");
-    } else {
-      ss_x = at::empty({1, 16}, f32);
-      rt_check(launch_row_sum_squares(x.data_ptr(), ss_x.data_ptr<float>(), (int)B, (int)H, stream), "decode_layer");
+    std::vector<DecodeStackLayer> layers(tensors.size() / kPer);
+    for (size_t l = 0; l < layers.size(); ++l) {
+      const torch::Tensor* t = &tensors[l * kPer];
+      if (!ok(t[0], 2) || !ok(t[1], 2) || !ok(t[2], 2) || !ok(t[3], 2) || !ok(t[4], 1) || !ok(t[5], 1) || !ok(t[6], 4) ||
+          !ok(t[7], 4) || t[0].size(0) != (hq + 2 * hkv) * D || t[0].size(1) != H || t[1].size(0) != H ||
+          t[1].size(1) != hq * D || t[2].size(0) != 2 * F || t[2].size(1) != H || t[3].size(0) != H ||
+          t[3].size(1) != F || t[4].size(0) != H || t[5].size(0) != H || t[6].sizes() != kc0.sizes() ||
+          t[7].sizes() != kc0.sizes())
+        return c10::nullopt;
+      layers[l] = {t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), t[3].data_ptr(),
+                   t[4].data_ptr(), t[5].data_ptr(), t[6].data_ptr(), t[7].data_ptr()};
     }
-    torch::Tensor qkv = at::empty({B, qkv_n}, x.options()), attn = at::empty({B, hq * D}, x.options());
-    torch::Tensor x1 = at::empty({B, H}, x.options()), act = at::empty({B, F}, x.options());
-    torch::Tensor y = at::empty({B, H}, x.options());
-    torch::Tensor ss_x1 = slots(H, hq * D), ss_y = slots(H, F);
-    project(x, w_qkv, qkv, &norm1, &ss_x, false, nullptr, nullptr);
-    rt_check(launch_decode_attention(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), attn.data_ptr(),
-                                     scratch.data_ptr(), (size_t)scratch.nbytes(), (int)B, hq, (int)hkv, (int)D, (int)S,
-                                     (int)pos0, pos ? static_cast<const int*>(pos->data_ptr()) : nullptr,
-                                     (float)rope_theta, stream, true), "decode_layer");
-    project(attn, w_o, x1, nullptr, nullptr, false, &x, &ss_x1);
-    project(x1, w_gate_up, act, &norm2, &ss_x1, true, nullptr, nullptr);
-    project(act, w_down, y, nullptr, nullptr, false, &x1, &ss_y);
-    return std::make_pair(y, ss_y);
-  }, py::arg("x"), py::arg("ss"), py::arg("k_cache"), py::arg("v_cache"), py::arg("pos0"), py::arg("pos"),
-     py::arg("w_qkv"), py::arg("w_o"), py::arg("w_gate_up"), py::arg("w_down"), py::arg("norm1"), py::arg("norm2"),
-     py::arg("hq"), py::arg("eps"), py::arg("rope_theta"), py::arg("scratch"), py::arg("timeout_ns"));
+    c10::cuda::CUDAGuard guard(dev);
+    const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+    if (decode_stack_supported((int)B, (int)H, (int)F, hq, (int)hkv, (int)D, (int)S, sms) != 0) return c10::nullopt;
+    const size_t bytes = decode_stack_scratch_bytes((int)B, (int)H, (int)F, hq, (int)hkv, (int)D, (int)S, sms);
+    torch::Tensor scratch = at::empty({(int64_t)bytes}, x.options().dtype(torch::kUInt8));
+    torch::Tensor y = at::empty_like(x);
+    DecodeStackArgs args{};
+    args.layers = layers.data();
+    args.n_layers = (int)layers.size();
+    args.x = x.data_ptr();
+    args.y = y.data_ptr();
+    args.scratch = scratch.data_ptr();
+    args.scratch_bytes = bytes;
+    args.batch = (int)B; args.hidden = (int)H; args.ffn = (int)F; args.hq = hq; args.hkv = (int)hkv;
+    args.head_dim = (int)D; args.s_max = (int)S;
+    args.pos0 = (int)pos0;
+    args.pos_dev = pos ? static_cast<const int*>(pos->data_ptr()) : nullptr;
+    args.eps = (float)eps;
+    args.rope_theta = (float)rope_theta;
+    args.num_sms = sms;
+    args.timeout_ns = timeout_ns;
+    args.status = status_for(dev);
+    rt_check(launch_decode_stack(args, current_stream(dev)), "decode_stack");
+    return y;
+  }, py::arg("x"), py::arg("tensors"), py::arg("pos0"), py::arg("pos"), py::arg("hq"), py::arg("eps"),
+     py::arg("rope_theta"), py::arg("timeout_ns"));
 
   // ---- oracles (CPU tensors) ----
   m.def("oracle_rms_norm_bf16", [](torch::Tensor x, c10::optional<torch::Tensor> residual, torch::Tensor w,

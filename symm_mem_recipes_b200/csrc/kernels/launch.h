@@ -192,8 +192,6 @@ int launch_matmul_reduce_scatter(const MatmulRsArgs& args, cudaStream_t stream);
 // `out` must not be the buffer of `sum_out` or `residual`.  H % 8 == 0, 16-byte aligned pointers.
 int launch_rms_norm(const void* x, const void* residual, const void* w, void* sum_out, void* out, int rows, int H,
                     float eps, cudaStream_t stream);
-// ss[row] = sum of squares of x[row, 0..H)
-int launch_row_sum_squares(const void* x, float* ss, int rows, int H, cudaStream_t stream);
 // Rotary embedding in place on heads [0, n_heads) of every row (`row_stride` elements per row);
 // token t is at position pos0 + t % seq, with pos0 read from `pos_dev` on the device when that is
 // not null (graph-captured decode).  head_dim % 16 == 0.
@@ -211,10 +209,8 @@ int launch_silu_mul(const void* gate_up, void* out, long long rows, int F, int n
 // hq / hkv <= 8.
 size_t decode_attention_scratch_bytes(int batch, int hkv, int head_dim, int s_max, int* n_split_out);
 // `rope_theta` != 0: the new token's queries and key are taken unrotated and rotated in the kernel.
-// `overlap`: programmatic stream serialization; caches and `pos_dev` are then read before the predecessor in
-// the stream has finished, so they must have been written before the last ordinary launch.
 int launch_decode_attention(const void* qkv, void* k_cache, void* v_cache, void* out, void* scratch,
                             size_t scratch_bytes, int batch, int hq, int hkv, int head_dim, int s_max, int pos0,
-                            const int* pos_dev, float rope_theta, cudaStream_t stream, bool overlap = false);
+                            const int* pos_dev, float rope_theta, cudaStream_t stream);
 
 }  // namespace smr

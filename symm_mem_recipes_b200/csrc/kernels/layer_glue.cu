@@ -156,31 +156,6 @@ rms_norm_long_kernel(const __nv_bfloat16* x, const __nv_bfloat16* residual, cons
   }
 }
 
-// ss[row] = sum of squares of x[row, :], the input of the RMSNorm that gemv_local.cu folds into the first
-// projection of a decode step (later ones get theirs from the kernel before).  At most 16 rows: latency only.
-__global__ void __launch_bounds__(512) row_sum_squares_kernel(const __nv_bfloat16* __restrict__ x, float* ss, int H) {
-  const Vec16* xr = reinterpret_cast<const Vec16*>(x + (size_t)blockIdx.x * H);
-  float t = 0.f;
-#pragma unroll 4
-  for (int i = threadIdx.x; i < H / 8; i += 512) {
-    float a[8];
-    unpack8(ld_16_nc(xr + i), a);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) t += a[q] * a[q];
-  }
-  __shared__ float warp_sums[16];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = t;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    t = threadIdx.x < 16 ? warp_sums[threadIdx.x] : 0.f;
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (threadIdx.x == 0) ss[blockIdx.x] = t;
-  }
-}
-
 // In place on rows of `row_stride` elements: heads [0, n_heads) of D elements
 // each are rotated.  Token t sits at position pos0 + (t % seq); with `pos_dev`
 // the first position is read from device memory instead (a decode step
@@ -330,12 +305,6 @@ int launch_rms_norm(const void* x, const void* residual, const void* w, void* su
     return go(rms_norm_kernel<256, 8, R>, 256, 1);
   };
   return residual != nullptr ? pick(std::true_type{}) : pick(std::false_type{});
-}
-
-int launch_row_sum_squares(const void* x, float* ss, int rows, int H, cudaStream_t stream) {
-  if (rows < 1 || H < 8 || H % 8 != 0 || !aligned16(x)) return cudaErrorInvalidValue;
-  row_sum_squares_kernel<<<rows, 512, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), ss, H);
-  return (int)cudaGetLastError();
 }
 
 int launch_rope_inplace(void* qkv, long long tokens, int row_stride, int n_heads, int head_dim, int seq, int pos0,

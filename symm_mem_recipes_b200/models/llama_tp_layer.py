@@ -50,7 +50,6 @@ import torch.nn.functional as F
 
 from .. import ops
 from .._ext import C
-from ..ops.layer_glue import attention_scratch
 from ..parallel import symm_mem
 
 _TIMEOUT_NS = int(os.environ.get("SMR_TIMEOUT_MS", "10000")) * 1_000_000
@@ -390,9 +389,9 @@ class LlamaTPDecoderLayer:
         """One decode step.  x [B, H] replicated on all ranks; caches
         [B, S_max, hkv, D] hold this rank's KV heads and are updated at `pos`."""
         if fused:
-            out = self.decode_local(x, None, k_cache, v_cache, pos)
-            if out is not None:
-                return out[0]
+            y = decode_local([self], [(k_cache, v_cache)], x, pos)
+            if y is not None:
+                return y
         cfg = self.cfg
         B, D, hq, hkv = x.shape[0], cfg.head_dim, self.hq, self.hkv
         glue = fused and self.fused_glue
@@ -412,20 +411,6 @@ class LlamaTPDecoderLayer:
                                            v_cache[:, : pos + 1].transpose(1, 2), enable_gqa=True)
         o_proj = self._row_parallel_decode(o.transpose(1, 2).reshape(B, hq * D).contiguous(), "o", fused)
         return self._decode_mlp(x, o_proj, fused, glue)
-
-    def decode_local(self, x: torch.Tensor, ss: Optional[torch.Tensor], k_cache: torch.Tensor,
-                     v_cache: torch.Tensor, pos):
-        """A decode step of a world of one as five kernels that start under one another: the norms are
-        folded into the projections after them, SiLU-mul and the residual adds into those before.
-        `ss` is the second value this returned beside `x` (None for an x from elsewhere).  Returns
-        `(y, ss of y)`, or None where the step has to be composed of single ops: with peers, without
-        the glue kernels, off the GPU, or for shapes these kernels do not take."""
-        if self.ws != 1 or not self.fused_glue or not x.is_cuda or k_cache.dim() != 4:
-            return None
-        on_device = isinstance(pos, torch.Tensor)
-        return C.decode_layer(x, ss, k_cache, v_cache, 0 if on_device else pos, pos if on_device else None,
-                              self.w_qkv, self.w_o, self.w_gate_up, self.w_down, self.norm1, self.norm2, self.hq,
-                              self.cfg.eps, self.cfg.rope_theta, attention_scratch(k_cache), _TIMEOUT_NS)
 
     def chains_residual(self, fused: bool = True) -> bool:
         """Whether `decode_static` can take and hand on an unfinished residual add (glue kernels only)."""
@@ -451,9 +436,9 @@ class LlamaTPDecoderLayer:
         if (pending_residual is not None or defer_residual) and not glue:
             raise ValueError("chaining the residual add needs the glue kernels (see chains_residual)")
         if glue and pending_residual is None and not defer_residual:
-            out = self.decode_local(x, None, k_cache, v_cache, pos)
-            if out is not None:
-                return out[0]
+            y = decode_local([self], [(k_cache, v_cache)], x, pos)
+            if y is not None:
+                return y
         if pending_residual is not None:
             h1, x = ops.rms_norm(x, self.norm1, cfg.eps, residual=pending_residual)    # x = previous x1 + down
         else:
@@ -477,19 +462,29 @@ class LlamaTPDecoderLayer:
         return self._decode_mlp(x, o_proj, fused, glue)
 
 
+def decode_local(layers, caches, x: torch.Tensor, pos) -> Optional[torch.Tensor]:
+    """A decode step of a world of one through `layers` as one persistent kernel (per eight layers), or None
+    where the step has to be composed of single ops: with peers, without the glue kernels, off the GPU,
+    or for layers the kernel does not take.  `pos`: an int, or an int32 tensor of one element on the GPU."""
+    cfg = layers[0].cfg
+    if not x.is_cuda or any(lyr.ws != 1 or not lyr.fused_glue or lyr.cfg != cfg for lyr in layers):
+        return None
+    tensors = []
+    for lyr, (kc, vc) in zip(layers, caches):
+        tensors += (lyr.w_qkv, lyr.w_o, lyr.w_gate_up, lyr.w_down, lyr.norm1, lyr.norm2, kc, vc)
+    on_device = isinstance(pos, torch.Tensor)
+    return C.decode_stack(x, tensors, 0 if on_device else pos, pos if on_device else None, layers[0].hq, cfg.eps,
+                          cfg.rope_theta, _TIMEOUT_NS)
+
+
 def decode_static_through(layers, caches, x: torch.Tensor, pos: torch.Tensor, fused: bool = True) -> torch.Tensor:
     """One decode step through stacked layers; where two neighbours both run the glue kernels the
     residual add that closes the first rides in the RMSNorm kernel that opens the second."""
     layers = list(layers)
-    h, ss = x, None
     if fused:
-        for lyr, (kc, vc) in zip(layers, caches):
-            out = lyr.decode_local(h, ss, kc, vc, pos)
-            if out is None:
-                break
-            h, ss = out
-        else:
-            return h
+        y = decode_local(layers, caches, x, pos)
+        if y is not None:
+            return y
     h, pending = x, None
     for i, (lyr, (kc, vc)) in enumerate(zip(layers, caches)):
         defer = (i + 1 < len(layers) and lyr.chains_residual(fused) and layers[i + 1].chains_residual(fused))

@@ -29,31 +29,35 @@ def test_gemv_tile_edges(B, K, N, nk):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("B,hidden,heads,kv,D,ffn,s_max,pos", [
-    (1, 512, 4, 1, 64, 512, 32, 0), (3, 512, 8, 1, 128, 520, 40, 15), (16, 1024, 8, 2, 128, 1544, 300, 257),
-    (5, 264, 3, 1, 64, 264, 4096, 4095), (2, 8192, 8, 1, 128, 3584, 2048, 1000)])
-def test_decode_step_matches_the_composition(B, hidden, heads, kv, D, ffn, s_max, pos):
-    """Five fused launches against the layer composed of library GEMMs and PyTorch attention."""
-    from symm_mem_recipes_b200.models.llama_tp_layer import LlamaTPConfig, LlamaTPDecoderLayer
+@pytest.mark.parametrize("n_layers,B,hidden,heads,kv,D,ffn,s_max,pos", [
+    (1, 1, 512, 4, 1, 64, 512, 32, 0), (2, 3, 512, 8, 1, 128, 576, 40, 15), (1, 16, 1024, 8, 2, 128, 1536, 300, 257),
+    (3, 5, 256, 3, 1, 64, 320, 4096, 4095), (1, 16, 512, 64, 16, 64, 512, 64, 40), (9, 2, 512, 4, 1, 128, 512, 64, 33),
+    (2, 2, 8192, 8, 1, 128, 3584, 2048, 1000)])
+def test_decode_step_matches_the_composition(n_layers, B, hidden, heads, kv, D, ffn, s_max, pos):
+    """The persistent step against the layers composed of library GEMMs and PyTorch attention."""
+    from symm_mem_recipes_b200.models.llama_tp_layer import LlamaTPConfig, LlamaTPDecoderLayer, decode_local
     from symm_mem_recipes_b200.parallel import symm_mem
 
     dev = torch.device("cuda", 0)
     cfg = LlamaTPConfig(hidden=hidden, n_heads=heads, n_kv_heads=kv, head_dim=D, ffn=ffn)
-    layer = LlamaTPDecoderLayer(cfg, dev, seed=3)
+    layers = [LlamaTPDecoderLayer(cfg, dev, seed=3 + i) for i in range(n_layers)]
     gen = torch.Generator().manual_seed(B + hidden + pos)
     x = _normal(gen, B, hidden, std=0.5)
-    kc, vc = _normal(gen, B, s_max, kv, D), _normal(gen, B, s_max, kv, D)
-    ka, va, kb, vb = kc.clone(), vc.clone(), kc.clone(), vc.clone()
-    got = layer.decode_local(x, None, ka, va, pos)
-    assert got is not None, "these shapes are meant for the fused step"
-    again = layer.decode_local(x, None, ka, va, torch.tensor([pos], dtype=torch.int32, device=dev))
-    want = layer.decode(x, kb, vb, pos, fused=False)
+    caches = [(_normal(gen, B, s_max, kv, D), _normal(gen, B, s_max, kv, D)) for _ in layers]
+    mine, theirs = ([(k.clone(), v.clone()) for k, v in caches] for _ in range(2))
+    got = decode_local(layers, mine, x, pos)
     symm_mem.check_status(dev)
-    assert torch.equal(got[0], again[0]) and torch.equal(got[1].sum(0)[:B], again[1].sum(0)[:B])
-    assert (got[0].float() - want.float()).norm() < 1e-2 * want.float().norm()
-    assert torch.allclose(got[1].sum(0)[:B], got[0].float().pow(2).sum(1), rtol=1e-4)
-    assert torch.allclose(va.float(), vb.float(), rtol=2e-2, atol=2e-2)
-    assert torch.allclose(ka.float(), kb.float(), rtol=2e-2, atol=2e-2)
+    assert got is not None, "these shapes are meant for the persistent step"
+    again = decode_local(layers, mine, x, torch.tensor([pos], dtype=torch.int32, device=dev))
+    symm_mem.check_status(dev)
+    assert torch.equal(got, again)
+    want = x
+    for layer, (kc, vc) in zip(layers, theirs):
+        want = layer.decode(want, kc, vc, pos, fused=False)
+    assert (got.float() - want.float()).norm() < 1e-2 * want.float().norm()
     other = torch.ones(s_max, dtype=torch.bool, device=dev)
     other[pos] = False
-    assert torch.equal(ka[:, other], kc[:, other]) and torch.equal(va[:, other], vc[:, other]), "only the new position may change"
+    for (ka, va), (kb, vb), (kc, vc) in zip(mine, theirs, caches):
+        for a, b, c in ((ka, kb, kc), (va, vb, vc)):
+            assert (a.float() - b.float()).norm() < 1e-2 * b.float().norm()
+            assert torch.equal(a[:, other], c[:, other]), "only the new position may change"
