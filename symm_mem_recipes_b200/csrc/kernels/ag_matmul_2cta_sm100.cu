@@ -618,12 +618,17 @@ int tail_parts(int rem, int pairs, int k_blocks, int most) {
 // (M 17 to 6000): a wave of n of the P pairs takes, per K block of 128 bytes, t1 with few pairs at work (the
 // tensor core's own rate) up to t1 + t2 with all of them (shared L2 and power), so narrow tiles win where tiles
 // are few and 256 columns where waves are full; cutting the last wave along K costs a pass through L2.
+// Two more terms, fitted on 17 shapes (M 2048 to 16384).  Rows whose pitch is no multiple of 128 bytes make every
+// TMA row touch two L2 lines: `skew` more per K block (fp8 13201 x 880 x 7440: 83 us at 256 columns, 102 at
+// 128; with K = 7424 67 and 65).  And a tile cannot take less than its epilogue, `epi` in fp8, where K is short
+// (fp8 9000 x 7168 x 1024: 51 us at 256 columns, 74 at 192, 69 at 128).
 // Examples, before (always 256 columns, no cut below one wave) and after: 64 x 1280 x 8192 41 -> 13 us,
 // 129 x 7168 x 8192 45 -> 32 us, 509 x 1280 x 8192 42 -> 18 us, 300 x 2048 x 2048 15 -> 10 us.
 MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int block_n, int num_sms, int max_splits) {
-  struct Width { int bn; double t1, t2, merge; };                   // microseconds
-  constexpr Width kWidths[] = {{256, 0.285, 0.135, 6.4}, {192, 0.215, 0.115, 5.4}, {128, 0.14, 0.095, 4.2}};
-  const int pairs = num_sms / 2, rows = (M + 2 * kBM - 1) / (2 * kBM);
+  struct Width { int bn; double t1, t2, merge, skew, epi; };        // microseconds
+  constexpr Width kWidths[] = {{256, 0.285, 0.135, 6.4, 0.07, 3.5}, {192, 0.215, 0.115, 5.4, 0.08, 4.0},
+                               {128, 0.14, 0.095, 4.2, 0.115, 2.5}};
+  const int pairs = num_sms < 4 ? 1 : num_sms / 2, rows = (M + 2 * kBM - 1) / (2 * kBM);
   const int k_blocks = (K * elem_bytes + 127) / 128;
   MatmulPlan best{block_n != 0 ? block_n : 256, 1, 0};
   double best_cost = -1;
@@ -636,7 +641,11 @@ MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int bl
     const int tiles = rows * (epilogue != 0 ? (N / 2 + bn / 2 - 1) / (bn / 2) : (N + bn - 1) / bn);
     // full waves of 256 columns lose more in fp8 (twice the MMA rate on the same operand bytes)
     const double t2 = elem_bytes == 1 && w.bn == 256 ? 0.165 : w.t2;
-    auto wave_us = [&](int n, int parts) { return k_blocks * (w.t1 + t2 * n * parts / pairs) / parts; };
+    const double t1 = w.t1 + (K * elem_bytes % 128 != 0 ? w.skew : 0.0), least = elem_bytes == 1 ? w.epi : 0.0;
+    auto wave_us = [&](int n, int parts) {
+      const double us = k_blocks * (t1 + t2 * n * parts / pairs) / parts;
+      return us > least ? us : least;
+    };
     const int rem = tiles % pairs;
     double cost = tiles / pairs * wave_us(pairs, 1);
     int parts = 1;
