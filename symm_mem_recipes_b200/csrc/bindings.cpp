@@ -1019,17 +1019,36 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                                  (float)rope_theta, stream, k_cache ? k_cache->data_ptr() : nullptr,
                                  v_cache ? v_cache->data_ptr() : nullptr, k_cache ? (int)k_cache->size(1) : 0, (int)hkv),
              "prefill_layer");
-    const torch::Tensor by_head = qkv.view({batch, seq, heads, D}).transpose(1, 2);
-    torch::Tensor o = at::scaled_dot_product_attention(by_head.narrow(1, 0, hq), by_head.narrow(1, hq, hkv),
-                                                       by_head.narrow(1, hq + hkv, hkv), c10::nullopt, 0.0, true,
-                                                       c10::nullopt, true);
-    o = o.transpose(1, 2).reshape({T, hq * D}).contiguous();
+    torch::Tensor o;
+    if (prefill_attention_preferred((int)batch, (int)seq, (int)hq, (int)hkv, (int)D)) {
+      o = at::empty({T, hq * D}, x.options());
+      rt_check(launch_prefill_attention(qkv.data_ptr(), o.data_ptr(), (int)batch, (int)seq, (int)hq, (int)hkv, (int)D, stream),
+               "prefill_layer");
+    } else {
+      const torch::Tensor by_head = qkv.view({batch, seq, heads, D}).transpose(1, 2);
+      o = at::scaled_dot_product_attention(by_head.narrow(1, 0, hq), by_head.narrow(1, hq, hkv),
+                                           by_head.narrow(1, hq + hkv, hkv), c10::nullopt, 0.0, true, c10::nullopt, true);
+      o = o.transpose(1, 2).reshape({T, hq * D}).contiguous();
+    }
     const torch::Tensor x1 = gemm(o, w_o, 0, x);
     const torch::Tensor act = gemm(norm(x1, norm2), w_gate_up, 2, c10::nullopt);
     return gemm(act, w_down, 0, x1);
   }, py::arg("x"), py::arg("batch"), py::arg("seq"), py::arg("k_cache"), py::arg("v_cache"), py::arg("w_qkv"),
      py::arg("w_o"), py::arg("w_gate_up"), py::arg("w_down"), py::arg("norm1"), py::arg("norm2"), py::arg("hq"),
      py::arg("hkv"), py::arg("head_dim"), py::arg("eps"), py::arg("rope_theta"), py::arg("timeout_ns"));
+
+  // The attention of that call by itself: qkv [batch * seq, (hq + 2 hkv) * D], rotated -> [batch * seq, hq * D].
+  m.def("prefill_attention", [](const torch::Tensor& qkv, int batch, int seq, int hq, int hkv) {
+    TORCH_CHECK(qkv.is_cuda() && qkv.is_contiguous() && qkv.dim() == 2 && qkv.scalar_type() == torch::kBFloat16 && hkv > 0 &&
+                hq > 0 && batch > 0 && seq > 0 && qkv.size(0) == (int64_t)batch * seq && qkv.size(1) % (hq + 2 * hkv) == 0,
+                "prefill_attention: contiguous bf16 CUDA [batch * seq, (hq + 2 hkv) * head_dim]");
+    c10::cuda::CUDAGuard guard(qkv.get_device());
+    const int D = (int)(qkv.size(1) / (hq + 2 * hkv));
+    torch::Tensor out = at::empty({qkv.size(0), (int64_t)hq * D}, qkv.options());
+    rt_check(launch_prefill_attention(qkv.data_ptr(), out.data_ptr(), batch, seq, hq, hkv, D,
+                                      current_stream(qkv.get_device())), "prefill_attention");
+    return out;
+  }, py::arg("qkv"), py::arg("batch"), py::arg("seq"), py::arg("hq"), py::arg("hkv"));
 
   // One decode step through layers whose projections have nobody to reduce with (a world of one): a persistent kernel
   // for up to eight layers at a time.  Per layer: w_qkv, w_o, w_gate_up, w_down, norm1, norm2, k_cache, v_cache.

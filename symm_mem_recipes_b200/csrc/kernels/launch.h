@@ -212,5 +212,10 @@ size_t decode_attention_scratch_bytes(int batch, int hkv, int head_dim, int s_ma
 int launch_decode_attention(const void* qkv, void* k_cache, void* v_cache, void* out, void* scratch,
                             size_t scratch_bytes, int batch, int hq, int hkv, int head_dim, int s_max, int pos0,
                             const int* pos_dev, float rope_theta, cudaStream_t stream);
+// Causal attention over qkv [batch * seq, (hq + 2 hkv) * head_dim] (queries and keys rotated) -> out
+// [batch * seq, hq * head_dim]; head_dim 64 or 128.  `preferred`: whether it is the faster one for these sizes.
+bool prefill_attention_preferred(int batch, int seq, int hq, int hkv, int head_dim);
+int launch_prefill_attention(const void* qkv, void* out, int batch, int seq, int hq, int hkv, int head_dim,
+                             cudaStream_t stream);
 
 }  // namespace smr
