@@ -76,3 +76,30 @@ def test_split_calls_on_several_streams():
     for i, c in enumerate(got):
         ref = want[i % len(cases)]
         assert bool(((c.float() - ref).abs() <= ref.abs() * 2.0 ** -6 + 2e-2).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 64, 65, 128])
+@pytest.mark.parametrize("N,K", [(16, 8), (1280, 2048), (2816, 600), (4096, 72), (8192, 520)])
+def test_few_rows(M, N, K):
+    """Where the weights are streamed past a few rows: paddings of the batch, K splits, partial tiles, the three ends."""
+    from symm_mem_recipes_b200.ops import interleave_gate_up
+    from symm_mem_recipes_b200.parallel import symm_mem
+    from symm_mem_recipes_b200.utils.testing import guarded_empty
+
+    a, b = _operands(M, N, K)
+    ref = a.float() @ b.float().t()
+    res = torch.randn(M, N, device="cuda").to(torch.bfloat16)
+    g, u = ref.split(N // 2, dim=1)
+    swiglu = torch.nn.functional.silu(g) * u
+    runs = [(b, 0, None, ref), (b, 0, res, ref + res.float()), (b, 2, None, swiglu)]
+    if N % 256 == 0:
+        runs.append((interleave_gate_up(b[: N // 2], b[N // 2:]), 1, None, swiglu))
+    for w, epilogue, r, want in runs:
+        c, intact = guarded_empty(tuple(want.shape), torch.bfloat16, "cuda")
+        for _ in range(2):
+            c.fill_(float("nan"))
+            assert _run(a, w, c, epilogue=epilogue, residual=r) is not None
+        symm_mem.check_status("cuda")
+        assert bool(((c.float() - want).abs() <= want.abs() * 2.0 ** -6 + 2e-2).all())
+        assert intact(), "the kernel stored outside its output"
