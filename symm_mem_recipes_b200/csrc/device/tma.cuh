@@ -40,6 +40,23 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* m
         "r"(x), "r"(y), "r"(z), "r"(w)
       : "memory");
 }
+// The same load of data that nobody reads again: its lines are the first to leave L2.
+__device__ __forceinline__ void tma_load_4d_once(void* smem_dst, const CUtensorMap* map, uint64_t* bar,
+                                                 int32_t x, int32_t y, int32_t z, int32_t w) {
+  uint64_t policy;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint"
+      " [%0], [%1, {%3, %4, %5, %6}], [%2], %7;"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)),
+        "r"(x), "r"(y), "r"(z), "r"(w), "l"(policy)
+      : "memory");
+}
+// The same box into L2 only.
+__device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap* map, int32_t c0, int32_t c1, int32_t c2, int32_t c3) {
+  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];"
+               ::"l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
 
 // 2-D tile shared -> global, tracked by bulk async-groups.  Parts of the box outside the tensor
 // are not written.  The shared-memory writes that filled the tile must be followed by

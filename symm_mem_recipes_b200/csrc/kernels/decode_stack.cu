@@ -8,6 +8,7 @@
 //   * one CTA per SM stays for the whole step, and its producer warp streams the weights of all phases of all layers
 //     through one ring without ever waiting for activations: while the CTAs meet at a phase boundary, 150 KB per
 //     SM (about 3 us of HBM) keep arriving;
+//   * when they wait longer, DRAM goes on filling L2 with the weights that come next (see kAhead);
 //   * a phase is a GEMM with the weight rows as the MMA's M and the batch (padded to 16) as its N; its rows are dealt
 //     out evenly over the CTAs (tile i starts at floor(i N / tiles), so 8192 rows are 148 tiles of 55 or 56), K is
 //     only split where a phase has too few rows (QKV), and then the attention adds the fp32 parts up;
@@ -17,9 +18,9 @@
 //     thread, about 1.3 us); attention is dealt out over (sequence, KV head, split of the context), then the sums of
 //     the splits over (sequence, query head).
 // The CTAs wait for one another, so the launch is cooperative.  Every wait is bounded.
-// Two layers of that share, against the five kernels: batch 1 at position 3000 133 -> 118 us, batch 16 at 6500 172 -> 156 us.  Of the
-// 54 us a layer takes at batch 1, QKV / attention / o / gate-up / down have their MMAs running for 4 / 0 / 2 / 17 / 7 us
-// and 12 us are attention with its three meeting points, 12 us the other meeting points and first loads of x.
+// Two layers of that share, against the five kernels: batch 1 at position 3000 133 -> 105 us, batch 16 at 6500 172 -> 145 us.
+// Of the 48 us a layer takes at batch 1 about 14 are attention with its meeting points, 12 the other meeting points
+// and first loads of x, the rest is the weight stream.
 //
 // Arithmetic is that of the single ops: bf16 activations between phases, fp32 accumulation, the norm rounded before and
 // after its weight, a projection rounded before its residual add, every sum in a fixed order.
@@ -52,6 +53,14 @@ constexpr int kThreads = 256;
 constexpr int kComputeWarp0 = 2, kWarps = 6, kCompute = kWarps * 32;
 constexpr uint32_t kSlotBytes = 28672;                          // four k blocks of 56 rows, or two of 112
 constexpr int kSlots = 6;
+// The weight stream of an SM at a meeting point: a slot that has not become free for twice the time its bytes take at the
+// SM's share of HBM (25 bytes a cycle) means that the phase is waiting, and then the steps after the ring go into
+// L2 at that rate, up to six of them (25 MB over all SMs).  Two layers at batch 1 / batch 16: without 107.5 / 143, up
+// to 4 steps 101.8 / 138.4, 6 101.0 / 139.9, 12 100.8 / 143.7; all the time instead of only when idle, 4 steps 109 /
+// 147 and 16 steps 136 / 175 us.  Weights are loaded as the first to leave L2 (113 / 151 us before that): what stays
+// are the activations, the new keys and values and what was prefetched.
+constexpr int kAhead = 6;
+constexpr int kShareOfHbm = 25, kIdleCycles = 2 * (int)kSlotBytes / kShareOfHbm;
 constexpr int kGroupBlocks = 4;                                 // k blocks of x under one barrier
 constexpr int kXGroups = 4;
 constexpr uint32_t kXBlockBytes = kBatchN * kBK * 2;            // 2 KB
@@ -437,27 +446,57 @@ __global__ void __launch_bounds__(kThreads, 1) decode_stack_kernel(const __grid_
   if (warp == 0) {
     // ---------------- the weight stream of the whole step ----------------
     if (elect_one()) {
-      int slot = 0;
+      // Ring slot `i` of phase `step` (of layer step / 4): a cursor over all the loads of this CTA.
+      struct Cursor {
+        int step, i;
+        Share sh;
+      };
+      const int n_phases = 4 * p.n_layers;
+      auto settle = [&](Cursor& c) {                               // on a step that exists, or at the end
+        while (c.i >= c.sh.n_steps && ++c.step < n_phases) {
+          c.i = 0;
+          c.sh = share_of(p.plan[c.step & 3], cta);
+        }
+      };
+      Cursor at{0, 0, share_of(p.plan[0], cta)}, ahead = at;
+      settle(at);
+      int slot = 0, lead = 0;                                      // lead: steps from `at` to `ahead`, in L2 or on their way there
       uint32_t use = 0;                                            // times the ring has wrapped
-      for (int l = 0; l < p.n_layers && !failed; ++l) {
-        for (int ph = 0; ph < 4 && !failed; ++ph) {
-          const PhasePlan& pl = p.plan[ph];
-          const Share sh = share_of(pl, cta);
-          const CUtensorMap* map = &p.layer[l].w[ph];
-          const uint32_t block_tx = (uint32_t)(pl.box * pl.halves) * 128u;
-          for (int i = 0; i < sh.n_steps; ++i) {
-            if (use > 0 && !mbar_wait(&w_empty[slot], (use - 1) & 1u, p.timeout_ns)) {
-              report_status(p.status, kTimeoutMbarrier, 0, blockIdx.x, slot, kWhereGemmEmpty, l * 4 + ph);
+      while (at.step < n_phases) {
+        const PhasePlan& pl = p.plan[at.step & 3];
+        if (use > 0) {
+          Deadline d(p.timeout_ns);
+          const long long t0 = clock64();
+          long long due = kIdleCycles;
+          while (!mbar_test(&w_empty[slot], (use - 1) & 1u)) {
+            if (lead < kAhead && ahead.step < n_phases && clock64() - t0 >= due) {
+              const PhasePlan& next = p.plan[ahead.step & 3];
+              for (int j = 0; j < next.slot_blocks; ++j)
+                tma_prefetch_4d(&p.layer[ahead.step >> 2].w[ahead.step & 3], 0, ahead.sh.n0, 0,
+                                ahead.sh.kb0 + ahead.i * next.slot_blocks + j);
+              due += next.slot_blocks * next.box * next.halves * 128 / kShareOfHbm;
+              ++ahead.i;
+              settle(ahead);
+              ++lead;
+            }
+            if (!d.alive()) {
+              report_status(p.status, kTimeoutMbarrier, 0, blockIdx.x, slot, kWhereGemmEmpty, at.step);
               failed = true;
               break;
             }
-            mbar_arrive_expect_tx(&w_full[slot], block_tx * (uint32_t)pl.slot_blocks);
-            for (int j = 0; j < pl.slot_blocks; ++j)
-              tma_load_4d(smem + (size_t)slot * kSlotBytes + (size_t)j * pl.block_bytes, map, &w_full[slot], 0, sh.n0, 0,
-                          sh.kb0 + i * pl.slot_blocks + j);
-            if (++slot == kSlots) { slot = 0; ++use; }
           }
+          if (failed) break;
         }
+        mbar_arrive_expect_tx(&w_full[slot], (uint32_t)(pl.box * pl.halves) * 128u * (uint32_t)pl.slot_blocks);
+        for (int j = 0; j < pl.slot_blocks; ++j)
+          tma_load_4d_once(smem + (size_t)slot * kSlotBytes + (size_t)j * pl.block_bytes,
+                           &p.layer[at.step >> 2].w[at.step & 3], &w_full[slot], 0, at.sh.n0, 0,
+                           at.sh.kb0 + at.i * pl.slot_blocks + j);
+        if (++slot == kSlots) { slot = 0; ++use; }
+        ++at.i;
+        settle(at);
+        if (lead > 0) --lead;
+        else ahead = at;
       }
     }
   } else if (warp == 1) {
