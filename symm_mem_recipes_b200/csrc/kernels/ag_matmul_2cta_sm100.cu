@@ -62,8 +62,9 @@ constexpr bool pair_tma_store() { return pair_row_bytes<BN, kFp8, kSwiGlu>() % 1
 
 // kOut: the epilogue leaves through shared memory: each epilogue warp owns two 4 KB boxes (32 rows x 128
 // bytes, 128-byte swizzle) that it fills from its accumulator rows and hands to a TMA store while it
-// converts the next columns into the other box.
-template <int BN, int STAGES, bool kOut = false>
+// converts the next columns into the other box.  kBoxes > 2: a box for every 128 bytes of a tile's row, into which TMA
+// brings the residual before the accumulator is complete.
+template <int BN, int STAGES, bool kOut = false, int kBoxes = 2>
 struct PairSmem {
   static constexpr uint32_t kABytes = kBM * kBK * 2;
   static constexpr uint32_t kBBytes = (BN / 2) * kBK * 2;     // this CTA's half of the B tile
@@ -71,9 +72,9 @@ struct PairSmem {
   static constexpr uint32_t kRingBytes = kStageBytes * STAGES;
   static constexpr uint32_t kOutBoxBytes = 32 * 128;          // 32 rows x 64 bf16
   static constexpr uint32_t kOutOffset = kRingBytes;
-  static constexpr uint32_t kOutBytes = kOut ? 4 * 2 * kOutBoxBytes : 0;
+  static constexpr uint32_t kOutBytes = kOut ? 4 * kBoxes * kOutBoxBytes : 0;
   static constexpr uint32_t kBarOffset = kRingBytes + kOutBytes;
-  static constexpr uint32_t kNumBars = 2 * STAGES + 4;
+  static constexpr uint32_t kNumBars = 2 * STAGES + 4 + 4 * kBoxes;   // the last ones: residual, [warp][box]
   static constexpr uint32_t kMiscOffset = kBarOffset + 8 * kNumBars;
   static constexpr uint32_t kTotal = kMiscOffset + 16 + 1024;
   static_assert(kStageBytes % 1024 == 0, "stage bases must stay 1024-byte aligned");
@@ -92,13 +93,13 @@ struct PairSmem {
 // its own over C.
 template <int BN, int STAGES, bool kFp8, bool kSwiGlu = false, bool kResidual = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
-ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
+ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,   // kResidual: the residual instead
                       const __grid_constant__ CUtensorMap tmap_a_out,
                       const __grid_constant__ CUtensorMap tmap_b,
                       const __grid_constant__ CUtensorMap tmap_c, const AgMatmulParams p) {
   constexpr bool kTmaStore = pair_tma_store<BN, kFp8, kSwiGlu>();
   static_assert(!kResidual || (kTmaStore && !kFp8 && !kSwiGlu), "the residual belongs to the plain bf16 epilogue");
-  using L = PairSmem<BN, STAGES, kTmaStore>;
+  using L = PairSmem<BN, STAGES, kTmaStore, kResidual ? BN / 64 : 2>;
   extern __shared__ uint8_t smem_raw[];
   // same offset in both CTAs: the dynamic window starts at the same shared address
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -129,6 +130,8 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
       mbar_init(&tmem_full[b], 1);
       mbar_init(&tmem_empty[b], 8);   // 4 epilogue warps x 2 CTAs (used in the leader)
     }
+    if constexpr (kResidual)
+      for (int b = 0; b < 4 * (BN / 64); ++b) mbar_init(&bars[2 * STAGES + 4 + b], 1);
     mbar_fence_init();
     tma_prefetch_desc(&tmap_a_shard);
     tma_prefetch_desc(&tmap_a_out);
@@ -287,6 +290,10 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
     const int all_pieces = p.blocks_per_rank * p.pieces;
     pdl_wait();
     [[maybe_unused]] int out_box = 0;                  // which of this warp's two output boxes is filled next
+    // Residual: a tile's boxes are brought in while the tile is multiplied; res_phase has the parity of each box's barrier.
+    // (Loaded by the lanes themselves, 16 bytes of 32 rows at a time, it cost 16384 x 8192 x 3584 123 us on top of 624.)
+    [[maybe_unused]] uint64_t* res_full = bars + 2 * STAGES + 4 + quarter * (BN / 64);
+    [[maybe_unused]] uint32_t res_phase = 0;
     if (p.mode == 2 && !push_entry_barrier(p, (int)blockIdx.x, etid)) failed = true;
     const bool trt = tr && etid == 0;
     uint64_t t_push = 0, t_acc = 0, n_units = 0;
@@ -307,6 +314,16 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
                                  pieces_due(p, round, n_pairs, 2, all_pieces), etid);
         ++round;
         if (trt) t_push += globaltimer_ns() - t0;
+      }
+      if constexpr (kResidual) {
+        if (w.part < 0 && valid && mblk * kBM + quarter * 32 < p.M && lane == 0) {
+          bulk_wait_group_read<0>();                   // the stores of the tile before have read these boxes
+          for (int c = 0; c < BN / 64 && ni * BN + c * 64 < p.N; ++c) {
+            mbar_arrive_expect_tx(&res_full[c], L::kOutBoxBytes);
+            tma_load_2d(smem + L::kOutOffset + ((size_t)quarter * (BN / 64) + c) * L::kOutBoxBytes, &tmap_a_shard, &res_full[c],
+                        ni * BN + c * 64, mblk * kBM + quarter * 32);
+          }
+        }
       }
       {
         const uint64_t t0 = trt ? globaltimer_ns() : 0;
@@ -432,22 +449,14 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
         // conflict-free for the warp's stores) -> one TMA store.
         constexpr int kBoxes = pair_row_bytes<BN, kFp8, kSwiGlu>() / 128;
         constexpr int kBoxCols = kOutCols / kBoxes;                  // columns of C per box
-        const uint32_t box0 = smem_u32(smem + L::kOutOffset) + (uint32_t)quarter * 2u * L::kOutBoxBytes;
+        const uint32_t box0 = smem_u32(smem + L::kOutOffset) + (uint32_t)quarter * (kResidual ? kBoxes : 2) * L::kOutBoxBytes;
         const bool store_ok = valid && mblk * kBM + quarter * 32 < p.M;
-        Vec16 res[kResidual ? 8 : 1];
-        auto fetch_residual = [&](int c) {
-          if constexpr (kResidual) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              res[j] = row_ok && col0 + c * kBoxCols + j * 8 < n_out ? ld_16(rrow + c * kBoxCols + j * 8) : Vec16{0u, 0u, 0u, 0u};
-          }
-        };
-        fetch_residual(0);
 #pragma unroll 1
         for (int c = 0; c < kBoxes; ++c) {
           // 64 accumulator columns in flight: the whole box, or half of it where two go into one of C's bytes (fp8)
           // or columns (SwiGLU)
           constexpr int kPasses = kFp8 || kSwiGlu ? 2 : 1;
+          if constexpr (kResidual) out_box = c;
           const uint32_t box = box0 + (uint32_t)out_box * L::kOutBoxBytes;
           const uint32_t rowaddr = box + (uint32_t)lane * 128u;
           const uint32_t sw = (uint32_t)(lane & 7);
@@ -461,7 +470,15 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
               tmem_ld_32x32b_x32(taddr + (uint32_t)(c * kBoxCols + h * 64), v[0]);
               tmem_ld_32x32b_x32(taddr + (uint32_t)(c * kBoxCols + h * 64 + 32), v[1]);
             }
-            if (h == 0) {
+            if constexpr (kResidual) {
+              if (store_ok && col0 + c * kBoxCols < n_out) {
+                if (!mbar_wait(&res_full[c], (res_phase >> c) & 1u, p.timeout_ns)) {
+                  if (lane == 0) report_status(p.status, kTimeoutMbarrier, p.rank, blockIdx.x, c, kWhereGemmFull);
+                  failed = true;
+                }
+                res_phase ^= 1u << c;
+              }
+            } else if (h == 0) {
               if (lane == 0) bulk_wait_group_read<1>();      // the store that last read this box is done with it
               __syncwarp();
             }
@@ -486,22 +503,22 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
                 }
                 o.x = pack_bf16x2(y[0], y[1]); o.y = pack_bf16x2(y[2], y[3]);
                 o.z = pack_bf16x2(y[4], y[5]); o.w = pack_bf16x2(y[6], y[7]);
-                if constexpr (kResidual) o = add_bf16x8(o, res[j]);
               }
-              st_shared_16(rowaddr + (((uint32_t)(h * (8 / kPasses) + j) ^ sw) << 4), o.x, o.y, o.z, o.w);
+              const uint32_t chunk = rowaddr + (((uint32_t)(h * (8 / kPasses) + j) ^ sw) << 4);
+              if constexpr (kResidual) o = add_bf16x8(o, ld_shared_16(chunk));
+              st_shared_16(chunk, o.x, o.y, o.z, o.w);
             }
           }
-          if (c + 1 < kBoxes) fetch_residual(c + 1);
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
             if (store_ok && col0 + c * kBoxCols < n_out) {
-              uint8_t* src = smem + L::kOutOffset + ((size_t)quarter * 2 + out_box) * L::kOutBoxBytes;
+              uint8_t* src = smem + L::kOutOffset + ((size_t)quarter * (kResidual ? kBoxes : 2) + out_box) * L::kOutBoxBytes;
               tma_store_2d(&tmap_c, src, col0 + c * kBoxCols, mblk * kBM + quarter * 32);
             }
             bulk_commit_group();
           }
-          out_box ^= 1;
+          if constexpr (!kResidual) out_box ^= 1;
         }
       } else {
 #pragma unroll 1
@@ -578,7 +595,7 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,
 template <int BN, int STAGES, bool kFp8, bool kSwiGlu = false, bool kResidual = false>
 int launch_pair_variant(const CUtensorMap& ta_shard, const CUtensorMap& ta_out, const CUtensorMap& tb,
                         const CUtensorMap& tc, const AgMatmulParams& p, int grid, bool overlap, cudaStream_t stream) {
-  using L = PairSmem<BN, STAGES, pair_tma_store<BN, kFp8, kSwiGlu>()>;
+  using L = PairSmem<BN, STAGES, pair_tma_store<BN, kFp8, kSwiGlu>(), kResidual ? BN / 64 : 2>;
   static_assert(L::kTotal <= 232448, "shared memory limit exceeded");
   auto kern = ag_matmul_2cta_kernel<BN, STAGES, kFp8, kSwiGlu, kResidual>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kTotal);
@@ -744,7 +761,10 @@ int launch_ag_matmul_2cta(const AgMatmulArgs& a, cudaStream_t stream) {
 
   CUtensorMap ta_shard, ta_out, tb, tc;
   int rows_local = comm ? a.rows_per_rank : a.M;
-  if (make_tmap(&ta_shard, a.a_local, (uint64_t)rows_local, (uint64_t)a.K, kBM, es)) return cudaErrorInvalidValue;
+  // without a gather nobody reads the shard's map, and the residual (32 x 64 boxes, as C) takes its place
+  if (a.residual != nullptr ? make_tmap(&ta_shard, a.residual, (uint64_t)a.M, (uint64_t)a.N, 32, es)
+                            : make_tmap(&ta_shard, a.a_local, (uint64_t)rows_local, (uint64_t)a.K, kBM, es))
+    return cudaErrorInvalidValue;
   if (make_tmap(&ta_out, comm ? a.a_out : a.a_local, (uint64_t)a.M, (uint64_t)a.K, kBM, es))
     return cudaErrorInvalidValue;
   if (make_tmap(&tb, a.b, (uint64_t)a.N, (uint64_t)a.K, (uint32_t)(bn / 2), es)) return cudaErrorInvalidValue;
@@ -799,7 +819,7 @@ int launch_ag_matmul_2cta(const AgMatmulArgs& a, cudaStream_t stream) {
     switch (bn) {
       case 128: return launch_pair_variant<128, 8, false, false, true>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
       case 192: return launch_pair_variant<192, 6, false, false, true>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
-      default:  return launch_pair_variant<256, 6, false, false, true>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
+      default:  return launch_pair_variant<256, 5, false, false, true>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
     }
   }
   switch (bn) {
