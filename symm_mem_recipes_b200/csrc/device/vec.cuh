@@ -38,6 +38,10 @@ __device__ __forceinline__ void st_16(void* p, const Vec16& v) {
   asm volatile("st.global.v4.u32 [%0], {%1,%2,%3,%4};"
                ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
+// The same for data that will not be read back from L2: its lines are the first to leave it.
+__device__ __forceinline__ void st_16_stream(void* p, Vec16 v) {
+  asm volatile("st.global.cs.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
 
 __device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
   uint32_t c;
