@@ -425,8 +425,9 @@ struct GemvPlan {
   int rows = kMaxRows, ksplit = 1, tiles = 1;
 };
 
-// Row tile and K split: the pair whose busiest CTA has the least to do, counted as cycles per k block x k blocks x
-// waves.  A k block costs the SM's share of HBM for its weight rows (25 bytes a cycle), its share of L2 for the
+// Row tile and K split: the pair whose busiest CTA has the least to do, counted as cycles per k block x k blocks plus
+// 5000 (set-up, the first loads' latency, the reduction) for each wave: without these 5176 columns stored [1584, N]
+// went in three waves of eight K splits, 14.7 us, now 6.6 in one of two.  A k block costs the SM's share of HBM for its weight rows (25 bytes a cycle), its share of L2 for the
 // weight rows and x (45), and the issuing thread 155 cycles or, at 64 rows of x and more, two for each of them.
 // Rows are cut to a multiple of 8 (the swizzle atom) so that one wave covers N evenly: at batch 16, 8192 columns become
 // 147 tiles of 56 rows on 148 SMs.  With gate and up a tile has half the columns, and where they alternate in groups
@@ -435,7 +436,7 @@ struct GemvPlan {
 GemvPlan plan_gemv(const DeviceFit& fit, int batch, int padded, int N, int K, bool nk, int halves, bool interleaved, int num_sms) {
   GemvPlan best;
   const int kb_total = (K + kBK - 1) / kBK, n_out = N / halves;
-  double best_cost = 0;
+  double best_cost = 0, best_work = 0;
   for (int i = 0; i < 4; ++i) {
     const int ks = 1 << i;
     if (ks > 1 && kb_total < kStageBlocks * ks) break;
@@ -449,9 +450,10 @@ GemvPlan plan_gemv(const DeviceFit& fit, int batch, int padded, int N, int K, bo
     const double l2 = (rows + batch) * 128 / 45.0, issue = padded < 64 ? 155.0 : 30.0 + 2.0 * padded;
     if (l2 > per) per = l2;
     if (issue > per) per = issue;
-    const double cost = per * k_blocks_per_cta(kb_total, ks) * waves;
-    if (i == 0 || cost < 0.95 * best_cost) {
+    const double work = per * k_blocks_per_cta(kb_total, ks) * waves, cost = work + 5000.0 * waves;
+    if (i == 0 || cost < best_cost - 0.05 * best_work) {
       best_cost = cost;
+      best_work = work;
       best.rows = rows;
       best.ksplit = ks;
       best.tiles = tiles;
