@@ -427,15 +427,19 @@ struct GemvPlan {
 
 // Row tile and K split: the pair whose busiest CTA has the least to do, counted as cycles per k block x k blocks plus
 // 5000 (set-up, the first loads' latency, the reduction) for each wave: without these 5176 columns stored [1584, N]
-// went in three waves of eight K splits, 14.7 us, now 6.6 in one of two.  A k block costs the SM's share of HBM for its weight rows (25 bytes a cycle), its share of L2 for the
-// weight rows and x (45), and the issuing thread 155 cycles or, at 64 rows of x and more, two for each of them.
+// went in three waves of eight K splits, 14.7 us, now 6.4 in one of two.
+// A k block costs the SM's share of HBM for its weight rows (25 bytes a cycle), its share of L2 for the weight rows and x
+// (45), and the issuing thread 155 cycles or, at 64 rows of x and more, two for each of them.  Rows of W that do not
+// start on 128-byte lines come in box by box, and tiles below 96 rows then cost as much as 96 where K is long: 6912 x
+// 7048 24.4 -> 20.4 us, 3000 x 5000 11.3 -> 9.6 (below the line 960 x 1248 would lose, 4.3 -> 4.7).
 // Rows are cut to a multiple of 8 (the swizzle atom) so that one wave covers N evenly: at batch 16, 8192 columns become
 // 147 tiles of 56 rows on 148 SMs.  With gate and up a tile has half the columns, and where they alternate in groups
-// of 128 it must not straddle one.  A larger cluster has to win by 5 % to be worth its wider barrier.  W stored
-// [K, N] comes in whole 128-column tiles.
+// of 128 it must not straddle one.  A larger cluster has to win by 5 % to be worth its wider barrier.  W stored [K, N]
+// comes in whole 128-column tiles.
 GemvPlan plan_gemv(const DeviceFit& fit, int batch, int padded, int N, int K, bool nk, int halves, bool interleaved, int num_sms) {
   GemvPlan best;
   const int kb_total = (K + kBK - 1) / kBK, n_out = N / halves;
+  const bool narrow_costs = nk && K % kBK != 0 && K >= 1536;
   double best_cost = 0, best_work = 0;
   for (int i = 0; i < 4; ++i) {
     const int ks = 1 << i;
@@ -446,7 +450,7 @@ GemvPlan plan_gemv(const DeviceFit& fit, int batch, int padded, int N, int K, bo
     if (cols > kMaxRows / halves) cols = kMaxRows / halves;
     if (interleaved) cols = cols <= 16 ? 16 : (cols <= 32 ? 32 : 64);
     const int rows = cols * halves, tiles = (n_out + cols - 1) / cols, waves = (tiles + clusters - 1) / clusters;
-    double per = rows * 128 / 25.0;
+    double per = (narrow_costs && rows < 96 ? 96 : rows) * 128 / 25.0;
     const double l2 = (rows + batch) * 128 / 45.0, issue = padded < 64 ? 155.0 : 30.0 + 2.0 * padded;
     if (l2 > per) per = l2;
     if (issue > per) per = issue;
