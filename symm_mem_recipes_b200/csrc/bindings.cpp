@@ -3,6 +3,7 @@
 // pointers and a stream.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
@@ -79,11 +80,19 @@ cudaStream_t current_stream(int device) { return c10::cuda::getCurrentCUDAStream
 // 4 KiB per (device, stream), zero between launches (the kernel resets them), so that calls on different
 // streams never share one.  At most kMaxCounterBuffers of them; a call beyond that, or one that is being
 // captured (its graph may be replayed beside anything), takes its counters from the framework's allocator
-// and clears them in the stream.
+// and clears them in the stream.  A new buffer is cleared in the stream that will use it: a clear on the legacy stream is
+// ordered neither after what waits there nor before a kernel on a non-blocking stream.
 constexpr size_t kTailCounterSlots = 1024;
 constexpr size_t kMaxCounterBuffers = 64;
 std::mutex g_counters_mu;
-std::map<std::pair<int, cudaStream_t>, uint32_t*> g_counters;
+// never destroyed: the framework that owns the tensors may be gone when static objects are (release_tail_counters empties it)
+auto& g_counters = *new std::map<std::pair<int, cudaStream_t>, torch::Tensor>;
+
+torch::Tensor zeroed_counters(int device, cudaStream_t stream) {
+  torch::Tensor t = new_tensor({(int64_t)kTailCounterSlots}, torch::kInt32, device);
+  rt_check(cudaMemsetAsync(t.data_ptr(), 0, t.nbytes(), stream), "cudaMemsetAsync(counters)");
+  return t;
+}
 
 uint32_t* tail_counters(int device, cudaStream_t stream, torch::Tensor& own) {
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
@@ -91,32 +100,27 @@ uint32_t* tail_counters(int device, cudaStream_t stream, torch::Tensor& own) {
   if (capturing == cudaStreamCaptureStatusNone) {
     std::lock_guard<std::mutex> lock(g_counters_mu);
     auto it = g_counters.find({device, stream});
-    if (it != g_counters.end()) return it->second;
-    if (g_counters.size() < kMaxCounterBuffers) {
-      uint32_t* c = nullptr;
-      rt_check(cudaMalloc(reinterpret_cast<void**>(&c), kTailCounterSlots * 4), "cudaMalloc(counters)");
-      rt_check(cudaMemset(c, 0, kTailCounterSlots * 4), "cudaMemset(counters)");
-      return g_counters[{device, stream}] = c;
+    if (it == g_counters.end() && g_counters.size() < kMaxCounterBuffers) {
+      // the allocation must not break a capture that another thread has running on another stream
+      c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+      it = g_counters.emplace(std::make_pair(device, stream), zeroed_counters(device, stream)).first;
     }
+    if (it != g_counters.end()) return static_cast<uint32_t*>(it->second.data_ptr());
   }
-  own = at::empty({(int64_t)kTailCounterSlots}, torch::TensorOptions().dtype(torch::kInt32).device(torch::kCUDA, device));
-  rt_check(cudaMemsetAsync(own.data_ptr(), 0, kTailCounterSlots * 4, stream), "cudaMemsetAsync(counters)");
-  return reinterpret_cast<uint32_t*>(own.data_ptr());
+  own = zeroed_counters(device, stream);
+  return static_cast<uint32_t*>(own.data_ptr());
 }
 
 // After a kernel gave up on a wait its counters hold whatever they held: back to zero (the device is idle).
 void clear_tail_counters(int device) {
   std::lock_guard<std::mutex> lock(g_counters_mu);
   for (auto& kv : g_counters)
-    if (kv.first.first == device) rt_check(cudaMemset(kv.second, 0, kTailCounterSlots * 4), "cudaMemset(counters)");
+    if (kv.first.first == device) rt_check(cudaMemsetAsync(kv.second.data_ptr(), 0, kv.second.nbytes(), nullptr), "cudaMemsetAsync(counters)");
+  rt_check(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize");
 }
 
 void release_tail_counters() {
   std::lock_guard<std::mutex> lock(g_counters_mu);
-  for (auto& kv : g_counters) {
-    c10::cuda::CUDAGuard guard(kv.first.first);
-    cudaFree(kv.second);
-  }
   g_counters.clear();
 }
 

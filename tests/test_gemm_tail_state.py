@@ -1,0 +1,96 @@
+"""What a GEMM whose tiles are cut along K keeps between calls: where it comes from, and the state in which a call finds it."""
+import pathlib
+import re
+import threading
+
+import pytest
+import torch
+
+CSRC = pathlib.Path(__file__).resolve().parent.parent / "symm_mem_recipes_b200" / "csrc"
+M, N, K = 200, 1280, 4096                          # 10 tiles of 128 columns on 74 pairs: every tile is cut
+
+
+def test_counters_are_not_cleared_on_the_legacy_stream():
+    """cudaMemset runs on the legacy stream: it is not ordered before a kernel on a non-blocking stream, and it waits
+    behind whatever the default stream has queued."""
+    source = (CSRC / "bindings.cpp").read_text()
+    assert not re.findall(r"cudaMemset\([^;]*counters", source)
+    assert not re.findall(r"cudaMalloc\([^;]*counters", source)
+
+
+def _operands():
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    a = (torch.randn(M, K, generator=gen, device="cuda") * 0.5).to(torch.bfloat16)
+    b = (torch.randn(N, K, generator=gen, device="cuda") * 0.1).to(torch.bfloat16)
+    return a, b, a.float() @ b.float().t()
+
+
+def _cut_gemm(a, b):
+    from symm_mem_recipes_b200._ext import C
+
+    return C.matmul_local(a, b, None, 0, None, 0, 0, True, 0, 2_000_000_000, 0)
+
+
+def _matches(c, want):
+    return bool(((c.float() - want).abs() <= want.abs() * 2.0 ** -6 + 2e-2).all())
+
+
+@pytest.mark.gpu
+def test_first_cut_call_on_a_stream_while_the_default_stream_is_busy():
+    from symm_mem_recipes_b200._ext import C
+    from symm_mem_recipes_b200.parallel import symm_mem
+
+    a, b, want = _operands()
+    C.release_tail_counters()
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):                # what the allocator hands out next on this stream is not zero
+        poison = [torch.full((1024,), 0x01010101, dtype=torch.int32, device="cuda") for _ in range(32)]
+        del poison
+    torch.cuda.synchronize()
+    torch.cuda._sleep(100_000_000)                 # about 50 ms on the default stream
+    with torch.cuda.stream(stream):
+        got = [_cut_gemm(a, b) for _ in range(3)]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):                # and nothing that was queued late has touched the counters
+        got.append(_cut_gemm(a, b))
+    torch.cuda.synchronize()
+    symm_mem.check_status("cuda")
+    assert all(_matches(c, want) for c in got)
+
+
+@pytest.mark.gpu
+def test_first_cut_call_while_another_thread_captures():
+    """The buffers that a first call makes do not break a capture in progress elsewhere in the process."""
+    from symm_mem_recipes_b200._ext import C
+
+    a, b, want = _operands()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):                # kernels loaded, output and scratch in the allocator's cache
+        _cut_gemm(a, b)                            # (without torch.cuda.graph below, which would empty it)
+    torch.cuda.synchronize()
+    C.release_tail_counters()
+    x = torch.ones(16, device="cuda")
+    out, errors = [], []
+
+    def call():
+        try:
+            with torch.cuda.stream(stream):
+                out.append(_cut_gemm(a, b))
+        except Exception as e:  # noqa: BLE001 - reported by the assertion below
+            errors.append(e)
+
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        graph.capture_begin(capture_error_mode="global")
+        y = x + 1
+        t = threading.Thread(target=call)
+        t.start()
+        t.join()
+        y = y * 2
+        graph.capture_end()
+    assert not errors, errors
+    graph.replay()
+    torch.cuda.synchronize()
+    assert bool((y == 4).all()) and _matches(out[0], want)
