@@ -57,8 +57,6 @@ Status* status_for(int device) {
   return s;
 }
 
-void clear_tail_counters(int device);
-
 // Synchronises the device, returns (code, rank, block, peer, where, aux) and
 // clears the record.
 py::tuple read_status(int device) {
@@ -67,61 +65,70 @@ py::tuple read_status(int device) {
   Status h{};
   rt_check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
   rt_check(cudaMemcpy(&h, s, sizeof(Status), cudaMemcpyDeviceToHost), "cudaMemcpy(status)");
-  if (h.code != 0) {
-    rt_check(cudaMemset(s, 0, sizeof(Status)), "cudaMemset(status)");
-    clear_tail_counters(device);
-  }
+  if (h.code != 0) rt_check(cudaMemset(s, 0, sizeof(Status)), "cudaMemset(status)");
   return py::make_tuple(h.code, h.rank, h.block, h.peer, h.where, h.aux);
 }
 
 cudaStream_t current_stream(int device) { return c10::cuda::getCurrentCUDAStream(device).stream(); }
 
-// ---- arrival counters of the GEMM's split-K tail -----------------------------
-// 4 KiB per (device, stream), zero between launches (the kernel resets them), so that calls on different
-// streams never share one.  At most kMaxCounterBuffers of them; a call beyond that, or one that is being
-// captured (its graph may be replayed beside anything), takes its counters from the framework's allocator
-// and clears them in the stream.  A new buffer is cleared in the stream that will use it: a clear on the legacy stream is
-// ordered neither after what waits there nor before a kernel on a non-blocking stream.
-constexpr size_t kTailCounterSlots = 1024;
-constexpr size_t kMaxCounterBuffers = 64;
-std::mutex g_counters_mu;
-// never destroyed: the framework that owns the tensors may be gone when static objects are (release_tail_counters empties it)
-auto& g_counters = *new std::map<std::pair<int, cudaStream_t>, torch::Tensor>;
+// ---- marks of the GEMM's split-K tail ------------------------------------------
+// 4 KiB per (device, stream), so that calls on different streams never share one, and the number of calls that
+// have used it.  A call marks with its own number, so it does not matter what the calls before it left, not even
+// one whose waits ran out.  At most kMaxMarkBuffers of them; a call beyond that, or one that is being captured (its
+// graph may be replayed beside anything, and with the same number each time), takes marks from the framework's
+// allocator and clears them in the stream.  A new buffer is cleared in the stream that will use it: a clear on the
+// legacy stream is ordered neither after what waits there nor before a kernel on a non-blocking stream.
+constexpr size_t kTailMarkSlots = 1024;
+constexpr size_t kMaxMarkBuffers = 64;
+struct TailMarks {
+  torch::Tensor words;
+  uint32_t calls;
+};
+std::mutex g_marks_mu;
+// never destroyed: the framework that owns the tensors may be gone when static objects are (release_tail_marks empties it)
+auto& g_marks = *new std::map<std::pair<int, cudaStream_t>, TailMarks>;
 
-torch::Tensor zeroed_counters(int device, cudaStream_t stream) {
-  torch::Tensor t = new_tensor({(int64_t)kTailCounterSlots}, torch::kInt32, device);
-  rt_check(cudaMemsetAsync(t.data_ptr(), 0, t.nbytes(), stream), "cudaMemsetAsync(counters)");
+torch::Tensor zeroed_marks(int device, cudaStream_t stream) {
+  torch::Tensor t = new_tensor({(int64_t)kTailMarkSlots}, torch::kInt32, device);
+  rt_check(cudaMemsetAsync(t.data_ptr(), 0, t.nbytes(), stream), "cudaMemsetAsync(marks)");
   return t;
 }
 
-uint32_t* tail_counters(int device, cudaStream_t stream, torch::Tensor& own) {
+// Marks and call number of a launch on `stream`; `own` keeps the marks of a call that shares none until it is launched.
+void set_tail_marks(AgMatmulArgs& args, int device, cudaStream_t stream, torch::Tensor& own) {
+  args.tail_mark_slots = kTailMarkSlots;
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   rt_check(cudaStreamIsCapturing(stream, &capturing), "cudaStreamIsCapturing");
   if (capturing == cudaStreamCaptureStatusNone) {
-    std::lock_guard<std::mutex> lock(g_counters_mu);
-    auto it = g_counters.find({device, stream});
-    if (it == g_counters.end() && g_counters.size() < kMaxCounterBuffers) {
+    std::lock_guard<std::mutex> lock(g_marks_mu);
+    auto it = g_marks.find({device, stream});
+    if (it == g_marks.end() && g_marks.size() < kMaxMarkBuffers) {
       // the allocation must not break a capture that another thread has running on another stream
       c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
-      it = g_counters.emplace(std::make_pair(device, stream), zeroed_counters(device, stream)).first;
+      it = g_marks.emplace(std::make_pair(device, stream), TailMarks{zeroed_marks(device, stream), 0u}).first;
     }
-    if (it != g_counters.end()) return static_cast<uint32_t*>(it->second.data_ptr());
+    if (it != g_marks.end()) {
+      if (++it->second.calls == 0u) it->second.calls = 1u;
+      args.tail_call = it->second.calls;
+      args.tail_marks = static_cast<uint32_t*>(it->second.words.data_ptr());
+      return;
+    }
   }
-  own = zeroed_counters(device, stream);
-  return static_cast<uint32_t*>(own.data_ptr());
+  own = zeroed_marks(device, stream);
+  args.tail_call = 1u;
+  args.tail_marks = static_cast<uint32_t*>(own.data_ptr());
 }
 
-// After a kernel gave up on a wait its counters hold whatever they held: back to zero (the device is idle).
-void clear_tail_counters(int device) {
-  std::lock_guard<std::mutex> lock(g_counters_mu);
-  for (auto& kv : g_counters)
-    if (kv.first.first == device) rt_check(cudaMemsetAsync(kv.second.data_ptr(), 0, kv.second.nbytes(), nullptr), "cudaMemsetAsync(counters)");
-  rt_check(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize");
+std::vector<torch::Tensor> tail_marks_in_use() {
+  std::lock_guard<std::mutex> lock(g_marks_mu);
+  std::vector<torch::Tensor> all;
+  for (auto& kv : g_marks) all.push_back(kv.second.words);
+  return all;
 }
 
-void release_tail_counters() {
-  std::lock_guard<std::mutex> lock(g_counters_mu);
-  g_counters.clear();
+void release_tail_marks() {
+  std::lock_guard<std::mutex> lock(g_marks_mu);
+  g_marks.clear();
 }
 
 // ---- which symmetric allocation an address belongs to ----------------------
@@ -343,13 +350,12 @@ c10::optional<torch::Tensor> matmul_local(const torch::Tensor& a, const torch::T
   const MatmulPlan plan = plan_matmul((int)M, (int)N, (int)K, args.elem_bytes, epilogue, block_n, args.num_sms,
                                       split_k ? max_splits : 1);
   args.block_n = plan.block_n;
-  torch::Tensor scratch, own_counters;
+  torch::Tensor scratch, own_marks;
   if (plan.tail_bytes > 0) {
     scratch = new_tensor({(int64_t)plan.tail_bytes}, torch::kUInt8, dev);
     args.tail_scratch = scratch.data_ptr();
     args.tail_scratch_bytes = plan.tail_bytes;
-    args.tail_counters = tail_counters(dev, stream, own_counters);
-    args.tail_counter_slots = kTailCounterSlots;
+    set_tail_marks(args, dev, stream, own_marks);
     args.tail_splits = plan.tail_splits;
   }
   rt_check(launch_ag_matmul_2cta(args, stream), "matmul");
@@ -727,15 +733,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     }
     TORCH_CHECK(c.size(0) == args.M && c.size(1) == (epilogue == 1 ? args.N / 2 : args.N),
                 "c must be [M, N] ([M, N / 2] with the SwiGLU epilogue)");
+    torch::Tensor own_marks;
     if (tail_scratch.has_value()) {
-      // first 4 KiB: arrival counters; the rest: fp32 partial accumulators
-      TORCH_CHECK(tail_scratch->is_cuda() && tail_scratch->is_contiguous() && tail_scratch->nbytes() > 8192,
-                  "tail_scratch must be a contiguous CUDA tensor");
-      char* base = static_cast<char*>(tail_scratch->data_ptr());
-      args.tail_counters = reinterpret_cast<uint32_t*>(base);
-      args.tail_counter_slots = 1024;
-      args.tail_scratch = base + 4096;
-      args.tail_scratch_bytes = tail_scratch->nbytes() - 4096;
+      // fp32 partial accumulators
+      TORCH_CHECK(tail_scratch->is_cuda() && tail_scratch->get_device() == dev && tail_scratch->is_contiguous() &&
+                  (uintptr_t)tail_scratch->data_ptr() % 16 == 0, "tail_scratch must be a contiguous CUDA tensor on a's GPU");
+      args.tail_scratch = tail_scratch->data_ptr();
+      args.tail_scratch_bytes = tail_scratch->nbytes();
+      set_tail_marks(args, dev, stream, own_marks);
     }
     args.lead = lead;
     args.push_ahead = push_ahead;
@@ -759,7 +764,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("matmul_local", &matmul_local, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("epilogue"), py::arg("residual"),
         py::arg("block_n"), py::arg("num_sms"), py::arg("split_k"), py::arg("panel_w"), py::arg("timeout_ns"),
         py::arg("max_splits") = 0);
-  m.def("release_tail_counters", &release_tail_counters);
+  m.def("tail_marks_in_use", &tail_marks_in_use);
+  m.def("release_tail_marks", &release_tail_marks);
 
   m.def("check_push_schedule", &check_push_schedule);
   m.def("check_pair_work", &check_pair_work);

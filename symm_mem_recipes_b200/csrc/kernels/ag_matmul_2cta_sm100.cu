@@ -23,10 +23,11 @@
 // pairs to begin with), each of its tiles is cut along K into 2 to 8 parts that run
 // on as many pairs at once.  Every part stores its fp32
 // partial accumulator to scratch memory (four columns x 128 rows contiguous, so
-// that a warp's accesses are whole lines), bumps the tile's arrival counter,
-// waits (bounded) for the other parts and then reduces ITS share of the tile's
-// columns in part order, so the result does not depend on timing.  The last part
-// to leave puts the counter back to zero: no memset in front of the kernel.
+// that a warp's accesses are whole lines), marks them with the number of the call,
+// waits (bounded) for the other parts' marks and then reduces ITS share of the tile's
+// columns in part order, so the result does not depend on timing.  Nothing is put back
+// and no memset stands in front of the kernel: what an earlier call left, also one that
+// gave up half-way, carries another number.
 // The two 128-row blocks of a pair are two consecutive positions of the M
 // schedule, not necessarily neighbours in memory: each CTA loads, waits for and
 // stores its own block.
@@ -372,15 +373,14 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,   // kRe
         __threadfence();
         if (etid == 0) tail_ok = 1;
         epilogue_group_sync();
-        uint32_t* counter = p.tail_counters + w.tail_idx * 2 + cta_rank;
-        if (etid == 0) {
-          red_add_release_gpu(counter, 1u);
-          if (!wait_ge_acquire_gpu(counter, (uint32_t)p.tail_splits, p.timeout_ns)) {
-            report_status(p.status, kTimeoutFlag, p.rank, blockIdx.x, w.tail_idx, kWhereGemmTmemFull, w.part);
+        uint32_t* marks = p.tail_marks + (w.tail_idx * 2 + cta_rank) * kMaxTailParts;
+        if (etid < 32) {                                             // one warp, a lane per part
+          if (lane == 0) st_release_gpu(marks + w.part, p.tail_call);
+          const int missing = await_marks(marks, p.tail_splits, p.tail_call, lane, p.timeout_ns);
+          if (missing >= 0 && lane == 0) {
+            report_status(p.status, kTimeoutFlag, p.rank, blockIdx.x, w.tail_idx, kWhereGemmTmemFull, missing);
             tail_ok = 0;
           }
-          // every part counts twice; the one that brings the counter to 2 x parts is the last to have seen it
-          if (atomicAdd(counter, 1u) == 2u * (uint32_t)p.tail_splits - 1u) *counter = 0u;
         }
         epilogue_group_sync();
         if (!tail_ok) { failed = true; break; }
@@ -623,7 +623,7 @@ namespace {
 int tail_parts(int rem, int pairs, int k_blocks, int most) {
   if (rem <= 0 || rem * 2 > pairs) return 1;
   int splits = pairs / rem;
-  if (splits > 8) splits = 8;
+  if (splits > kMaxTailParts) splits = kMaxTailParts;
   if (most > 0 && splits > most) splits = most;
   while (splits > 1 && k_blocks < 2 * splits) --splits;
   return splits;
@@ -785,13 +785,14 @@ int launch_ag_matmul_2cta(const AgMatmulArgs& a, cudaStream_t stream) {
   if (a.tail_scratch != nullptr && rem > 0 && rem * 2 <= max_pairs) {
     int splits = tail_parts(rem, max_pairs, k_blocks, a.tail_splits);
     while (splits > 1 && ((size_t)rem * splits * 2 * kBM * bn * sizeof(float) > a.tail_scratch_bytes ||
-                          (size_t)rem * 2 > a.tail_counter_slots))
+                          (size_t)rem * 2 * kMaxTailParts > a.tail_mark_slots))
       --splits;
     if (splits >= 2) {
       p.tail_tiles = rem;
       p.tail_splits = splits;
       p.tail_scratch = static_cast<float*>(a.tail_scratch);
-      p.tail_counters = a.tail_counters;
+      p.tail_marks = a.tail_marks;
+      p.tail_call = a.tail_call;
       if (total_tiles < max_pairs) pairs = rem * splits;
     }
   }

@@ -59,20 +59,15 @@ class AgMatmulConfig:
 
 DEFAULT_CONFIG = AgMatmulConfig()
 _sm_count: dict[int, int] = {}
-_tail_scratch: dict[int, torch.Tensor] = {}
-_TAIL_SCRATCH_BYTES = 4096 + 37 * 8 * 2 * 128 * 256 * 4     # counters + the largest tail (37 tiles x 8 parts)
 
 
 def _tail_buffer(device: torch.device, config: "AgMatmulConfig"):
-    """Scratch of the split-K tail (fp32 partial accumulators), one per device."""
+    """Scratch of one call's split-K tail: fp32 partial accumulators of at most one 128 x 256 block per CTA.
+    From the caching allocator each time, so that calls on two streams never share it."""
     if not config.split_k_tail:
         return None
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    t = _tail_scratch.get(idx)
-    if t is None:
-        t = torch.zeros(_TAIL_SCRATCH_BYTES, dtype=torch.uint8, device=device)    # the counters start at zero
-        _tail_scratch[idx] = t
-    return t
+    ctas = config.num_sms or _num_sms(device)
+    return torch.empty(max(ctas, 2) * 128 * 256 * 4, dtype=torch.uint8, device=device)
 
 
 def _push_plain_stores(config: "AgMatmulConfig", world_size: int) -> bool:

@@ -502,7 +502,7 @@ def shutdown() -> None:
             pass
     _records.clear()
     _groups.clear()
-    C.release_tail_counters()
+    C.release_tail_marks()
 
 
 def reset() -> None:

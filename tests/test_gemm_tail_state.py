@@ -10,12 +10,25 @@ CSRC = pathlib.Path(__file__).resolve().parent.parent / "symm_mem_recipes_b200" 
 M, N, K = 200, 1280, 4096                          # 10 tiles of 128 columns on 74 pairs: every tile is cut
 
 
-def test_counters_are_not_cleared_on_the_legacy_stream():
+def test_marks_are_not_cleared_on_the_legacy_stream():
     """cudaMemset runs on the legacy stream: it is not ordered before a kernel on a non-blocking stream, and it waits
     behind whatever the default stream has queued."""
     source = (CSRC / "bindings.cpp").read_text()
-    assert not re.findall(r"cudaMemset\([^;]*counters", source)
-    assert not re.findall(r"cudaMalloc\([^;]*counters", source)
+    assert not re.findall(r"cudaMemset\([^;]*(counters|marks)", source)
+    assert not re.findall(r"cudaMalloc\([^;]*(counters|marks)", source)
+
+
+def test_calls_that_are_alive_at_once_share_no_scratch():
+    import importlib
+
+    ag = importlib.import_module("symm_mem_recipes_b200.ops.ag_matmul")
+    config = ag.AgMatmulConfig(num_sms=148, split_k_tail=True)
+    first, second = (ag._tail_buffer(torch.device("cpu"), config) for _ in range(2))
+    assert first.data_ptr() != second.data_ptr()
+    assert first.nbytes == 74 * 2 * 128 * 256 * 4      # a 256 x 256 fp32 partial on every one of 74 pairs
+    kept = [k for k, v in vars(ag).items() if isinstance(v, dict) and "scratch" in k]
+    assert not kept, "state that symm_mem.reset() does not know of"
+    assert ag._tail_buffer(torch.device("cpu"), ag.AgMatmulConfig(num_sms=148, split_k_tail=False)) is None
 
 
 def _operands():
@@ -41,7 +54,7 @@ def test_first_cut_call_on_a_stream_while_the_default_stream_is_busy():
     from symm_mem_recipes_b200.parallel import symm_mem
 
     a, b, want = _operands()
-    C.release_tail_counters()
+    C.release_tail_marks()
     stream = torch.cuda.Stream()
     torch.cuda.synchronize()
     with torch.cuda.stream(stream):                # what the allocator hands out next on this stream is not zero
@@ -52,7 +65,7 @@ def test_first_cut_call_on_a_stream_while_the_default_stream_is_busy():
     with torch.cuda.stream(stream):
         got = [_cut_gemm(a, b) for _ in range(3)]
     torch.cuda.synchronize()
-    with torch.cuda.stream(stream):                # and nothing that was queued late has touched the counters
+    with torch.cuda.stream(stream):                # and nothing that was queued late has touched the marks
         got.append(_cut_gemm(a, b))
     torch.cuda.synchronize()
     symm_mem.check_status("cuda")
@@ -69,7 +82,7 @@ def test_first_cut_call_while_another_thread_captures():
     with torch.cuda.stream(stream):                # kernels loaded, output and scratch in the allocator's cache
         _cut_gemm(a, b)                            # (without torch.cuda.graph below, which would empty it)
     torch.cuda.synchronize()
-    C.release_tail_counters()
+    C.release_tail_marks()
     x = torch.ones(16, device="cuda")
     out, errors = [], []
 
@@ -94,3 +107,42 @@ def test_first_cut_call_while_another_thread_captures():
     graph.replay()
     torch.cuda.synchronize()
     assert bool((y == 4).all()) and _matches(out[0], want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("traced", [False, True])
+def test_call_after_one_that_gave_up(traced):
+    """Whatever part of its marks a call that gave up has left, the next one waits for its own parts."""
+    import symm_mem_recipes_b200 as smr
+    from symm_mem_recipes_b200._ext import C
+    from symm_mem_recipes_b200.parallel import symm_mem
+
+    a, b, want = _operands()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    trace = torch.zeros(sms, 12, dtype=torch.int64, device="cuda") if traced else None   # a record takes the other binding
+    C.release_tail_marks()
+    for left in (lambda w: w.zero_(), lambda w: w.fill_(int(w.max())), lambda w: w[::2].zero_(), lambda w: w[1::3].sub_(1)):
+        assert _matches(smr.matmul(a, b, trace=trace), want)
+        (words,) = C.tail_marks_in_use()
+        assert int(words.max()) > 0, "the call was not cut"
+        left(words)
+        assert _matches(smr.matmul(a, b, trace=trace), want)
+    symm_mem.check_status("cuda")
+    symm_mem.reset()
+    assert C.tail_marks_in_use() == []
+
+
+@pytest.mark.gpu
+def test_captured_cut_call_replays():
+    from symm_mem_recipes_b200.parallel import symm_mem
+
+    a, b, want = _operands()
+    _cut_gemm(a, b)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        c = _cut_gemm(a, b)
+    for _ in range(3):
+        c.zero_()
+        graph.replay()
+        assert _matches(c, want) and _matches(_cut_gemm(a, b), want)
+    symm_mem.check_status("cuda")
