@@ -3,7 +3,6 @@
 // pointers and a stream.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
-#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
@@ -70,66 +69,6 @@ py::tuple read_status(int device) {
 }
 
 cudaStream_t current_stream(int device) { return c10::cuda::getCurrentCUDAStream(device).stream(); }
-
-// ---- marks of the GEMM's split-K tail ------------------------------------------
-// 4 KiB per (device, stream), so that calls on different streams never share one, and the number of calls that
-// have used it.  A call marks with its own number, so it does not matter what the calls before it left, not even
-// one whose waits ran out.  At most kMaxMarkBuffers of them; a call beyond that, or one that is being captured (its
-// graph may be replayed beside anything, and with the same number each time), takes marks from the framework's
-// allocator and clears them in the stream.  A new buffer is cleared in the stream that will use it: a clear on the
-// legacy stream is ordered neither after what waits there nor before a kernel on a non-blocking stream.
-constexpr size_t kTailMarkSlots = 1024;
-constexpr size_t kMaxMarkBuffers = 64;
-struct TailMarks {
-  torch::Tensor words;
-  uint32_t calls;
-};
-std::mutex g_marks_mu;
-// never destroyed: the framework that owns the tensors may be gone when static objects are (release_tail_marks empties it)
-auto& g_marks = *new std::map<std::pair<int, cudaStream_t>, TailMarks>;
-
-torch::Tensor zeroed_marks(int device, cudaStream_t stream) {
-  torch::Tensor t = new_tensor({(int64_t)kTailMarkSlots}, torch::kInt32, device);
-  rt_check(cudaMemsetAsync(t.data_ptr(), 0, t.nbytes(), stream), "cudaMemsetAsync(marks)");
-  return t;
-}
-
-// Marks and call number of a launch on `stream`; `own` keeps the marks of a call that shares none until it is launched.
-void set_tail_marks(AgMatmulArgs& args, int device, cudaStream_t stream, torch::Tensor& own) {
-  args.tail_mark_slots = kTailMarkSlots;
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  rt_check(cudaStreamIsCapturing(stream, &capturing), "cudaStreamIsCapturing");
-  if (capturing == cudaStreamCaptureStatusNone) {
-    std::lock_guard<std::mutex> lock(g_marks_mu);
-    auto it = g_marks.find({device, stream});
-    if (it == g_marks.end() && g_marks.size() < kMaxMarkBuffers) {
-      // the allocation must not break a capture that another thread has running on another stream
-      c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
-      it = g_marks.emplace(std::make_pair(device, stream), TailMarks{zeroed_marks(device, stream), 0u}).first;
-    }
-    if (it != g_marks.end()) {
-      if (++it->second.calls == 0u) it->second.calls = 1u;
-      args.tail_call = it->second.calls;
-      args.tail_marks = static_cast<uint32_t*>(it->second.words.data_ptr());
-      return;
-    }
-  }
-  own = zeroed_marks(device, stream);
-  args.tail_call = 1u;
-  args.tail_marks = static_cast<uint32_t*>(own.data_ptr());
-}
-
-std::vector<torch::Tensor> tail_marks_in_use() {
-  std::lock_guard<std::mutex> lock(g_marks_mu);
-  std::vector<torch::Tensor> all;
-  for (auto& kv : g_marks) all.push_back(kv.second.words);
-  return all;
-}
-
-void release_tail_marks() {
-  std::lock_guard<std::mutex> lock(g_marks_mu);
-  g_marks.clear();
-}
 
 // ---- which symmetric allocation an address belongs to ----------------------
 // Looked up on every all-reduce, so it lives here and not in a Python dictionary: an ordered map from payload
@@ -350,12 +289,11 @@ c10::optional<torch::Tensor> matmul_local(const torch::Tensor& a, const torch::T
   const MatmulPlan plan = plan_matmul((int)M, (int)N, (int)K, args.elem_bytes, epilogue, block_n, args.num_sms,
                                       split_k ? max_splits : 1);
   args.block_n = plan.block_n;
-  torch::Tensor scratch, own_marks;
+  torch::Tensor scratch;
   if (plan.tail_bytes > 0) {
     scratch = new_tensor({(int64_t)plan.tail_bytes}, torch::kUInt8, dev);
     args.tail_scratch = scratch.data_ptr();
     args.tail_scratch_bytes = plan.tail_bytes;
-    set_tail_marks(args, dev, stream, own_marks);
     args.tail_splits = plan.tail_splits;
   }
   rt_check(launch_ag_matmul_2cta(args, stream), "matmul");
@@ -733,14 +671,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     }
     TORCH_CHECK(c.size(0) == args.M && c.size(1) == (epilogue == 1 ? args.N / 2 : args.N),
                 "c must be [M, N] ([M, N / 2] with the SwiGLU epilogue)");
-    torch::Tensor own_marks;
     if (tail_scratch.has_value()) {
       // fp32 partial accumulators
       TORCH_CHECK(tail_scratch->is_cuda() && tail_scratch->get_device() == dev && tail_scratch->is_contiguous() &&
                   (uintptr_t)tail_scratch->data_ptr() % 16 == 0, "tail_scratch must be a contiguous CUDA tensor on a's GPU");
       args.tail_scratch = tail_scratch->data_ptr();
       args.tail_scratch_bytes = tail_scratch->nbytes();
-      set_tail_marks(args, dev, stream, own_marks);
     }
     args.lead = lead;
     args.push_ahead = push_ahead;
@@ -764,8 +700,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("matmul_local", &matmul_local, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("epilogue"), py::arg("residual"),
         py::arg("block_n"), py::arg("num_sms"), py::arg("split_k"), py::arg("panel_w"), py::arg("timeout_ns"),
         py::arg("max_splits") = 0);
-  m.def("tail_marks_in_use", &tail_marks_in_use);
-  m.def("release_tail_marks", &release_tail_marks);
 
   m.def("check_push_schedule", &check_push_schedule);
   m.def("check_pair_work", &check_pair_work);

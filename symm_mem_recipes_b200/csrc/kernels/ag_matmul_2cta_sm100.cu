@@ -23,11 +23,9 @@
 // pairs to begin with), each of its tiles is cut along K into 2 to 8 parts that run
 // on as many pairs at once.  Every part stores its fp32
 // partial accumulator to scratch memory (four columns x 128 rows contiguous, so
-// that a warp's accesses are whole lines), marks them with the number of the call,
-// waits (bounded) for the other parts' marks and then reduces ITS share of the tile's
-// columns in part order, so the result does not depend on timing.  Nothing is put back
-// and no memset stands in front of the kernel: what an earlier call left, also one that
-// gave up half-way, carries another number.
+// that a warp's accesses are whole lines); a second kernel adds the parts up in their
+// order, so the result does not depend on timing (merge_tail_kernel).  No CTA of a GEMM
+// without a gather waits for another pair.
 // The two 128-row blocks of a pair are two consecutive positions of the M
 // schedule, not necessarily neighbours in memory: each CTA loads, waits for and
 // stores its own block.
@@ -299,7 +297,6 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,   // kRe
     const bool trt = tr && etid == 0;
     uint64_t t_push = 0, t_acc = 0, n_units = 0;
     if (trt) trc[ag_trace::kEntered] = globaltimer_ns();
-    __shared__ int tail_ok;
     PairWork w;
     for (int wi = 0; !failed && pair_work(p, pair, n_pairs, total_tiles, k_blocks, wi, w); ++wi) {
       const int t = w.tile;
@@ -349,9 +346,8 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,   // kRe
       const int n_out = kSwiGlu ? p.N >> 1 : p.N;                    // columns of C
       const int col0 = ni * kOutCols;
       uint8_t* crow = reinterpret_cast<uint8_t*>(p.c) + ((size_t)row * n_out + col0) * (kFp8 ? 1 : 2);
-      [[maybe_unused]] const __nv_bfloat16* rrow = kResidual ? p.residual + (size_t)row * n_out + col0 : nullptr;
       if (w.part >= 0) {
-        // ---- split-K tail: park the fp32 partial, meet the other parts, reduce my columns ----
+        // ---- split-K tail: park the fp32 partial for merge_tail_kernel ----
         const size_t blk = (size_t)kBM * BN;                         // floats per CTA block
         const int r = quarter * 32 + lane;
         float* mine = p.tail_scratch + (((size_t)w.tail_idx * p.tail_splits + w.part) * 2 + cta_rank) * blk + r * 4;
@@ -370,79 +366,6 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,   // kRe
             st_16(mine + (size_t)(c * 8 + q) * (kBM * 4), Vec16{v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]});
         }
         release_accumulator();
-        __threadfence();
-        if (etid == 0) tail_ok = 1;
-        epilogue_group_sync();
-        uint32_t* marks = p.tail_marks + (w.tail_idx * 2 + cta_rank) * kMaxTailParts;
-        if (etid < 32) {                                             // one warp, a lane per part
-          if (lane == 0) st_release_gpu(marks + w.part, p.tail_call);
-          const int missing = await_marks(marks, p.tail_splits, p.tail_call, lane, p.timeout_ns);
-          if (missing >= 0 && lane == 0) {
-            report_status(p.status, kTimeoutFlag, p.rank, blockIdx.x, w.tail_idx, kWhereGemmTmemFull, missing);
-            tail_ok = 0;
-          }
-        }
-        epilogue_group_sync();
-        if (!tail_ok) { failed = true; break; }
-        // My share of the tile's columns of C, in groups of eight.  Four groups of accumulator columns (with
-        // SwiGLU two of gate and the matching two of up) times two parts are in flight at once, because one
-        // group at a time would pay the L2's latency for each.
-        constexpr int kGroups = kOutCols / 8, kBatch = kSwiGlu ? 2 : 4;
-        const int g0 = w.part * kGroups / p.tail_splits, g1 = (w.part + 1) * kGroups / p.tail_splits;
-        const float* base = p.tail_scratch + ((size_t)w.tail_idx * p.tail_splits * 2 + cta_rank) * blk + r * 4;
-#pragma unroll 1
-        for (int g = g0; g < g1; g += kBatch) {
-          float s[4][8];
-          const float* src[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int col = kSwiGlu ? (i >> 1) * (BN / 2) + (g + (i & 1)) * 8 : (g + i) * 8;
-            src[i] = base + (size_t)(col / 4) * (kBM * 4);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) s[i][q] = 0.f;
-          }
-#pragma unroll 1
-          for (int sp = 0; sp < p.tail_splits; sp += 2) {             // parts in order: deterministic
-            Vec16 v[2][4][2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u)
-#pragma unroll
-              for (int i = 0; i < 4; ++i)
-                if (sp + u < p.tail_splits && g + (kSwiGlu ? i & 1 : i) < g1) {
-                  v[u][i][0] = ld_16_stream(src[i] + (size_t)(sp + u) * 2 * blk);
-                  v[u][i][1] = ld_16_stream(src[i] + (size_t)(sp + u) * 2 * blk + kBM * 4);
-                }
-#pragma unroll
-            for (int u = 0; u < 2; ++u)
-#pragma unroll
-              for (int i = 0; i < 4; ++i)
-                if (sp + u < p.tail_splits && g + (kSwiGlu ? i & 1 : i) < g1) {
-                  s[i][0] += __uint_as_float(v[u][i][0].x); s[i][1] += __uint_as_float(v[u][i][0].y);
-                  s[i][2] += __uint_as_float(v[u][i][0].z); s[i][3] += __uint_as_float(v[u][i][0].w);
-                  s[i][4] += __uint_as_float(v[u][i][1].x); s[i][5] += __uint_as_float(v[u][i][1].y);
-                  s[i][6] += __uint_as_float(v[u][i][1].z); s[i][7] += __uint_as_float(v[u][i][1].w);
-                }
-          }
-#pragma unroll
-          for (int i = 0; i < kBatch; ++i) {
-            if constexpr (kSwiGlu) {
-#pragma unroll
-              for (int q = 0; q < 8; ++q) s[i][q] = s[i][q] / (1.0f + __expf(-s[i][q])) * s[i + 2][q];
-            }
-            const int col = (g + i) * 8;
-            if (row_ok && g + i < g1 && col0 + col < n_out) {
-              if constexpr (kFp8) {
-                st_8(crow + col, pack_e4m3x4(s[i][0], s[i][1], s[i][2], s[i][3]), pack_e4m3x4(s[i][4], s[i][5], s[i][6], s[i][7]));
-              } else {
-                Vec16 o;
-                o.x = pack_bf16x2(s[i][0], s[i][1]); o.y = pack_bf16x2(s[i][2], s[i][3]);
-                o.z = pack_bf16x2(s[i][4], s[i][5]); o.w = pack_bf16x2(s[i][6], s[i][7]);
-                if constexpr (kResidual) o = add_bf16x8(o, ld_16(rrow + col));
-                st_16(crow + col * 2, o);
-              }
-            }
-          }
-        }
       } else if constexpr (kTmaStore) {
         // One box (128 bytes of every row) at a time: accumulator columns -> packed words -> this warp's free
         // box (16-byte chunk j of row r sits at chunk j ^ (r & 7): the 128-byte swizzle of the tensor map,
@@ -592,6 +515,78 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,   // kRe
   }
 }
 
+// The parts of the tail's tiles added up in their order, with the GEMM's three ends.  A warp takes eight rows of four
+// groups of eight columns: its loads are whole lines of the scratch layout, its stores 64 bytes of a row.  Bound by the
+// pass through L2; launched under the GEMM (its CTAs fit beside the GEMM's), it begins when the last part is stored.
+// A kernel of its own, because parts that wait for one another inside the GEMM need all of its CTAs resident at once:
+// against waits without that guarantee 1024 x 1280 x 8192 27.0 -> 25.0 us, 200 x 512 x 8192 11.8 -> 10.6, 200 x 1280 x
+// 4096 11.3 -> 11.6; a cooperative launch, which gives the guarantee, took fp8 4096 x 3584 x 8192 from 103.2 to 106.2.
+constexpr int kMergeThreads = 256;
+template <int BN, bool kFp8, bool kSwiGlu, bool kResidual>
+__global__ void __launch_bounds__(kMergeThreads) merge_tail_kernel(const AgMatmulParams p) {
+  pdl_launch_dependents();
+  constexpr int kOutCols = kSwiGlu ? BN / 2 : BN, kGroupBlocks = kOutCols / 32, kBlk = kBM * BN;
+  const int lane = threadIdx.x & 31;
+  int u = (int)(blockIdx.x * (kMergeThreads / 32) + (threadIdx.x >> 5));
+  const int g = u % kGroupBlocks * 4 + (lane >> 3);                  // columns 8 g .. 8 g + 7 of the tile's C
+  u /= kGroupBlocks;
+  const int r = u % (kBM / 8) * 8 + (lane & 7);                      // row of the CTA's block
+  u /= kBM / 8;
+  const int cta = u & 1, tail_idx = u >> 1;
+  if (tail_idx >= p.tail_tiles) return;
+  const int n_pair_rows = (p.n_blocks_m + 1) >> 1;
+  int prow, ni;
+  tile_coords(p, n_pair_rows, n_pair_rows * p.n_tiles_n - p.tail_tiles + tail_idx, prow, ni);
+  const int mi = prow * 2 + cta, n_out = kSwiGlu ? p.N >> 1 : p.N, col = ni * kOutCols + g * 8;
+  if (mi >= p.n_blocks_m || col >= n_out) return;
+  bool local_unused;
+  const int row = scheduled_block(p, mi, local_unused) * kBM + r;
+  if (row >= p.M) return;
+  const float* src = p.tail_scratch + ((size_t)tail_idx * p.tail_splits * 2 + cta) * kBlk + (size_t)g * (2 * kBM * 4) + r * 4;
+  const size_t up = (size_t)(BN / 8) * (kBM * 4);                    // from a gate column to the matching up column
+  pdl_wait();
+  constexpr int kHalves = kSwiGlu ? 2 : 1, kInFlight = 4;            // parts whose loads are in flight at once
+  float s[kHalves][8] = {};
+  for (int i0 = 0; i0 < p.tail_splits; i0 += kInFlight) {
+    Vec16 v[kInFlight][kHalves][2];
+#pragma unroll
+    for (int i = 0; i < kInFlight; ++i)
+#pragma unroll
+      for (int h = 0; h < kHalves; ++h)
+        if (i0 + i < p.tail_splits) {
+          const float* q = src + (size_t)(i0 + i) * 2 * kBlk + h * up;
+          v[i][h][0] = ld_16_stream(q);
+          v[i][h][1] = ld_16_stream(q + kBM * 4);
+        }
+#pragma unroll
+    for (int i = 0; i < kInFlight; ++i)                              // in part order
+#pragma unroll
+      for (int h = 0; h < kHalves; ++h)
+        if (i0 + i < p.tail_splits) {
+          const Vec16 &a = v[i][h][0], &b = v[i][h][1];
+          s[h][0] += __uint_as_float(a.x); s[h][1] += __uint_as_float(a.y);
+          s[h][2] += __uint_as_float(a.z); s[h][3] += __uint_as_float(a.w);
+          s[h][4] += __uint_as_float(b.x); s[h][5] += __uint_as_float(b.y);
+          s[h][6] += __uint_as_float(b.z); s[h][7] += __uint_as_float(b.w);
+        }
+  }
+  if constexpr (kSwiGlu) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s[0][q] = s[0][q] / (1.0f + __expf(-s[0][q])) * s[1][q];
+  }
+  const size_t at = (size_t)row * n_out + col;
+  if constexpr (kFp8) {
+    st_8(reinterpret_cast<uint8_t*>(p.c) + at, pack_e4m3x4(s[0][0], s[0][1], s[0][2], s[0][3]),
+         pack_e4m3x4(s[0][4], s[0][5], s[0][6], s[0][7]));
+  } else {
+    Vec16 o;
+    o.x = pack_bf16x2(s[0][0], s[0][1]); o.y = pack_bf16x2(s[0][2], s[0][3]);
+    o.z = pack_bf16x2(s[0][4], s[0][5]); o.w = pack_bf16x2(s[0][6], s[0][7]);
+    if constexpr (kResidual) o = add_bf16x8(o, ld_16(p.residual + at));
+    st_16(p.c + at, o);
+  }
+}
+
 template <int BN, int STAGES, bool kFp8, bool kSwiGlu = false, bool kResidual = false>
 int launch_pair_variant(const CUtensorMap& ta_shard, const CUtensorMap& ta_out, const CUtensorMap& tb,
                         const CUtensorMap& tc, const AgMatmulParams& p, int grid, bool overlap, cudaStream_t stream) {
@@ -600,8 +595,9 @@ int launch_pair_variant(const CUtensorMap& ta_shard, const CUtensorMap& ta_out, 
   auto kern = ag_matmul_2cta_kernel<BN, STAGES, kFp8, kSwiGlu, kResidual>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kTotal);
   if (e != cudaSuccess) return (int)e;
-  // The pairs wait for one another (pieces of the gather, parts of the split-K tail): all of them must be resident.
-  if (int rc = check_co_resident(kern, grid, kGemmThreads, L::kTotal, 2)) return rc;
+  // The pairs of a gather wait for one another's pieces: all of them must be resident.
+  if (p.mode != 0)
+    if (int rc = check_co_resident(kern, grid, kGemmThreads, L::kTotal, 2)) return rc;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)grid, 1, 1);
   cfg.blockDim = dim3(kGemmThreads, 1, 1);
@@ -612,7 +608,15 @@ int launch_pair_variant(const CUtensorMap& ta_shard, const CUtensorMap& ta_out, 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = overlap ? 1 : 0;
-  return (int)cudaLaunchKernelEx(&cfg, kern, ta_shard, ta_out, tb, tc, p);
+  e = cudaLaunchKernelEx(&cfg, kern, ta_shard, ta_out, tb, tc, p);
+  if (e != cudaSuccess || p.tail_tiles == 0) return (int)e;
+  constexpr int kWarpsPerBlock = kBM / 8 * (kSwiGlu ? BN / 2 : BN) / 32;
+  const int warps = p.tail_tiles * 2 * kWarpsPerBlock;
+  cfg.gridDim = dim3((unsigned)((warps + kMergeThreads / 32 - 1) / (kMergeThreads / 32)), 1, 1);
+  cfg.blockDim = dim3(kMergeThreads, 1, 1);
+  cfg.dynamicSmemBytes = 0;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, merge_tail_kernel<BN, kFp8, kSwiGlu, kResidual>, p);
 }
 
 }  // namespace
@@ -784,15 +788,11 @@ int launch_ag_matmul_2cta(const AgMatmulArgs& a, cudaStream_t stream) {
   const int rem = total_tiles % max_pairs;
   if (a.tail_scratch != nullptr && rem > 0 && rem * 2 <= max_pairs) {
     int splits = tail_parts(rem, max_pairs, k_blocks, a.tail_splits);
-    while (splits > 1 && ((size_t)rem * splits * 2 * kBM * bn * sizeof(float) > a.tail_scratch_bytes ||
-                          (size_t)rem * 2 * kMaxTailParts > a.tail_mark_slots))
-      --splits;
+    while (splits > 1 && (size_t)rem * splits * 2 * kBM * bn * sizeof(float) > a.tail_scratch_bytes) --splits;
     if (splits >= 2) {
       p.tail_tiles = rem;
       p.tail_splits = splits;
       p.tail_scratch = static_cast<float*>(a.tail_scratch);
-      p.tail_marks = a.tail_marks;
-      p.tail_call = a.tail_call;
       if (total_tiles < max_pairs) pairs = rem * splits;
     }
   }

@@ -31,7 +31,7 @@ constexpr int kUmmaK = 16;
 constexpr int kGemmThreads = 192; // 6 warps
 constexpr int kEpiWarp0 = 2;
 constexpr uint32_t kTmemCols = 512;
-constexpr int kMaxTailParts = 8;  // K parts of a tile of the split-K tail: their marks fill one 32-byte sector
+constexpr int kMaxTailParts = 8;  // K parts of a tile of the split-K tail
 // Push mode: a block's arrival counter grows by kArrivalUnits per call whatever the number of pieces
 // (each piece adds kArrivalUnits / pieces), so calls with different piece counts can share an allocation.
 constexpr uint32_t kArrivalUnits = 256;  // pieces: a power of two up to this
@@ -66,8 +66,6 @@ struct AgMatmulParams {
   int tail_tiles;        // tiles handled that way (0 = none); they are the last ones of the schedule
   int tail_splits;       // K parts per such tile (2 to kMaxTailParts)
   float* tail_scratch;   // [tail_tiles][tail_splits][2 CTAs][BN / 4][128 rows] x 4 fp32: partial accumulators
-  uint32_t* tail_marks;  // [tail_tiles][2 CTAs][kMaxTailParts]: the last call in which part i has stored its partial
-  uint32_t tail_call;    // number of this call, one that no earlier call on these marks had
   // rows of B that tile ni takes: CTA c of the pair loads BN / 2 of them from ni * b_step + c * b_pair
   int b_step, b_pair;
   const __nv_bfloat16* residual;   // [M, N] added to the rounded product (plain bf16 epilogue), or nullptr
@@ -103,21 +101,6 @@ constexpr int kTraceSlots = 12;
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void epilogue_group_sync() {
   asm volatile("bar.sync 1, 128;" ::: "memory");
-}
-
-// A warp waits until all `n` marks carry `call`; what their writers stored before is visible then.  Returns -1, or the
-// first part that is missing when the time is up.  The lanes leave together and the polls are relaxed, with one fence
-// at the end: lanes that leave one by one, or an acquire per poll, cost 1.5 us for eight parts.
-__device__ inline int await_marks(const uint32_t* marks, int n, uint32_t call, int lane, uint64_t timeout_ns) {
-  Deadline d(timeout_ns);
-  for (;;) {
-    const bool there = lane >= n || ld_relaxed_gpu(marks + lane) == call;
-    const unsigned missing = __ballot_sync(0xffffffffu, !there);
-    if (missing == 0u) break;
-    if (__any_sync(0xffffffffu, !d.alive())) return __ffs((int)missing) - 1;
-  }
-  fence_acq_rel_gpu();
-  return -1;
 }
 
 // Entry barrier of the push mode, among the CTAs with this index on every rank.

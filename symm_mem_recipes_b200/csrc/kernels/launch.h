@@ -95,13 +95,9 @@ struct AgMatmulArgs {
   uint32_t barrier_block_base;
   uint64_t timeout_ns;
   Status* status;
-  // optional scratch of the split-K tail (nullptr = never split), the words in which its parts say that they have stored
-  // theirs, and the number they say it with (not 0, and not one of an earlier launch on these words)
+  // optional scratch of the split-K tail (nullptr = never split)
   void* tail_scratch;
   size_t tail_scratch_bytes;
-  uint32_t* tail_marks;
-  size_t tail_mark_slots;
-  uint32_t tail_call;
   int tail_splits;       // K parts of a tile of the tail at most (0 = as many as the idle pairs allow, up to 8)
   // optional [num_sms][12] words of per-CTA timing (ag_trace:: in ag_matmul_common.cuh)
   uint64_t* trace;

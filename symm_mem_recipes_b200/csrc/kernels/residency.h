@@ -1,8 +1,8 @@
 // Launch-time check that every CTA of a grid can be resident at once.
 //
-// The CTAs of the fused kernels wait for one another (arrival counters of a
-// split-K tail, flags written by the CTAs of a peer rank that run the same grid,
-// the K splits of a GEMV tile).  A grid that does not fit on the GPU in one wave
+// The CTAs of the fused kernels wait for one another (flags written by the CTAs
+// of a peer rank that run the same grid, the K splits of a GEMV tile, the phases
+// of a decode step).  A grid that does not fit on the GPU in one wave
 // would leave the first wave waiting for CTAs that cannot start; the bounded
 // waits would turn that into a timeout seconds later.  The launchers call this
 // first and refuse such a grid with cudaErrorCooperativeLaunchTooLarge instead.

@@ -502,7 +502,6 @@ def shutdown() -> None:
             pass
     _records.clear()
     _groups.clear()
-    C.release_tail_marks()
 
 
 def reset() -> None:

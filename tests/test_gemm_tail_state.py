@@ -10,12 +10,13 @@ CSRC = pathlib.Path(__file__).resolve().parent.parent / "symm_mem_recipes_b200" 
 M, N, K = 200, 1280, 4096                          # 10 tiles of 128 columns on 74 pairs: every tile is cut
 
 
-def test_marks_are_not_cleared_on_the_legacy_stream():
-    """cudaMemset runs on the legacy stream: it is not ordered before a kernel on a non-blocking stream, and it waits
-    behind whatever the default stream has queued."""
-    source = (CSRC / "bindings.cpp").read_text()
-    assert not re.findall(r"cudaMemset\([^;]*(counters|marks)", source)
-    assert not re.findall(r"cudaMalloc\([^;]*(counters|marks)", source)
+def test_tail_needs_no_state_and_no_waits():
+    """The parts of a cut tile do not wait for one another, so nothing has to be cleared, kept between calls or resident at
+    the same time: the GEMM without a gather holds no wait on global memory."""
+    source = (CSRC / "kernels" / "ag_matmul_2cta_sm100.cu").read_text()
+    waits = re.findall(r"\b(wait_\w+|ld_acquire_\w+|await_\w+)\(", source)
+    assert waits == ["wait_reached_acquire_sys"]       # a gathered block of a peer
+    assert not re.search(r"counters|marks", (CSRC / "bindings.cpp").read_text())
 
 
 def test_calls_that_are_alive_at_once_share_no_scratch():
@@ -50,39 +51,30 @@ def _matches(c, want):
 
 @pytest.mark.gpu
 def test_first_cut_call_on_a_stream_while_the_default_stream_is_busy():
-    from symm_mem_recipes_b200._ext import C
     from symm_mem_recipes_b200.parallel import symm_mem
 
     a, b, want = _operands()
-    C.release_tail_marks()
     stream = torch.cuda.Stream()
     torch.cuda.synchronize()
     with torch.cuda.stream(stream):                # what the allocator hands out next on this stream is not zero
-        poison = [torch.full((1024,), 0x01010101, dtype=torch.int32, device="cuda") for _ in range(32)]
+        poison = [torch.full((n,), 0x01010101, dtype=torch.int32, device="cuda") for n in (1024, 1 << 20, 4 << 20) for _ in range(4)]
         del poison
     torch.cuda.synchronize()
     torch.cuda._sleep(100_000_000)                 # about 50 ms on the default stream
     with torch.cuda.stream(stream):
         got = [_cut_gemm(a, b) for _ in range(3)]
     torch.cuda.synchronize()
-    with torch.cuda.stream(stream):                # and nothing that was queued late has touched the marks
-        got.append(_cut_gemm(a, b))
-    torch.cuda.synchronize()
     symm_mem.check_status("cuda")
     assert all(_matches(c, want) for c in got)
 
 
 @pytest.mark.gpu
-def test_first_cut_call_while_another_thread_captures():
-    """The buffers that a first call makes do not break a capture in progress elsewhere in the process."""
-    from symm_mem_recipes_b200._ext import C
-
+def test_cut_call_while_another_thread_captures():
     a, b, want = _operands()
     stream = torch.cuda.Stream()
     with torch.cuda.stream(stream):                # kernels loaded, output and scratch in the allocator's cache
         _cut_gemm(a, b)                            # (without torch.cuda.graph below, which would empty it)
     torch.cuda.synchronize()
-    C.release_tail_marks()
     x = torch.ones(16, device="cuda")
     out, errors = [], []
 
@@ -111,38 +103,73 @@ def test_first_cut_call_while_another_thread_captures():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("traced", [False, True])
-def test_call_after_one_that_gave_up(traced):
-    """Whatever part of its marks a call that gave up has left, the next one waits for its own parts."""
+def test_calls_in_a_row_and_replayed(traced):
+    """Both bindings, again and again on one scratch, eagerly and from a graph."""
     import symm_mem_recipes_b200 as smr
-    from symm_mem_recipes_b200._ext import C
     from symm_mem_recipes_b200.parallel import symm_mem
 
     a, b, want = _operands()
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     trace = torch.zeros(sms, 12, dtype=torch.int64, device="cuda") if traced else None   # a record takes the other binding
-    C.release_tail_marks()
-    for left in (lambda w: w.zero_(), lambda w: w.fill_(int(w.max())), lambda w: w[::2].zero_(), lambda w: w[1::3].sub_(1)):
-        assert _matches(smr.matmul(a, b, trace=trace), want)
-        (words,) = C.tail_marks_in_use()
-        assert int(words.max()) > 0, "the call was not cut"
-        left(words)
-        assert _matches(smr.matmul(a, b, trace=trace), want)
-    symm_mem.check_status("cuda")
-    symm_mem.reset()
-    assert C.tail_marks_in_use() == []
-
-
-@pytest.mark.gpu
-def test_captured_cut_call_replays():
-    from symm_mem_recipes_b200.parallel import symm_mem
-
-    a, b, want = _operands()
-    _cut_gemm(a, b)
     graph = torch.cuda.CUDAGraph()
+    smr.matmul(a, b, trace=trace)
     with torch.cuda.graph(graph):
-        c = _cut_gemm(a, b)
+        c = smr.matmul(a, b, trace=trace)
     for _ in range(3):
         c.zero_()
         graph.replay()
-        assert _matches(c, want) and _matches(_cut_gemm(a, b), want)
+        assert _matches(c, want) and _matches(smr.matmul(a, b, trace=trace), want)
     symm_mem.check_status("cuda")
+
+
+@pytest.mark.gpu
+def test_cut_calls_of_two_priorities_at_once():
+    """Cut GEMMs as wide as the GPU on streams of two priorities, started while another kernel holds some of the SMs."""
+    from symm_mem_recipes_b200.parallel import symm_mem
+
+    a, b, want = _operands()
+    low, high = torch.cuda.Stream(priority=0), torch.cuda.Stream(priority=-1)
+    filler = torch.randn(2048, 2048, device="cuda")
+    torch.cuda.synchronize()
+    got = []
+    for _ in range(20):
+        filler = (filler @ filler).clamp_(-1, 1)   # on the default stream: its end frees SMs one after the other
+        for stream in (low, high, low, high):
+            with torch.cuda.stream(stream):
+                got.append(_cut_gemm(a, b))
+    torch.cuda.synchronize()
+    symm_mem.check_status("cuda")
+    assert all(_matches(c, want) for c in got)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k,block_n,sms,epilogue,dtype", [
+    (129, 136, 1024, 128, 0, 0, torch.bfloat16), (300, 1000, 2048, 192, 24, 0, torch.bfloat16),
+    (257, 520, 4096, 256, 0, 0, torch.bfloat16), (130, 464, 1160, 224, 0, 0, torch.bfloat16),
+    (300, 2000, 1024, 0, 0, 2, torch.bfloat16), (300, 768, 1024, 0, 0, 1, torch.bfloat16),
+    (129, 144, 4096, 128, 0, 0, torch.float8_e4m3fn), (300, 976, 2064, 192, 24, 0, torch.float8_e4m3fn),
+    (600, 464, 4096, 224, 0, 0, torch.float8_e4m3fn)])
+@pytest.mark.parametrize("splits", [2, 3, 8])
+def test_cut_tiles_equal_uncut_ones(m, n, k, block_n, sms, epilogue, dtype, splits):
+    """Every width, end and type of the cut path at ragged edges.  The same products in another order of fp32 sums: a
+    result may round to the neighbouring bf16 (2^-8 of it) or e4m3 (2^-3) number, and beside that differ by what
+    cancels, k * 2^-24 of a sum of k terms of 0.05."""
+    from symm_mem_recipes_b200._ext import C
+    from symm_mem_recipes_b200.parallel import symm_mem
+    from symm_mem_recipes_b200.utils.testing import guarded_empty
+
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = (torch.randn(m, k, generator=gen, device="cuda") * 0.5).to(dtype)
+    b = (torch.randn(n, k, generator=gen, device="cuda") * 0.1).to(dtype)
+    n_out = n // 2 if epilogue else n
+    if dtype == torch.bfloat16:
+        c, intact = guarded_empty((m, n_out), dtype, "cuda")
+    else:
+        c, intact = torch.empty(m, n_out, dtype=dtype, device="cuda"), lambda: True
+    whole = C.matmul_local(a, b, None, epilogue, None, block_n, sms, False, 0, 2_000_000_000, 1)
+    assert C.matmul_local(a, b, c, epilogue, None, block_n, sms, True, 0, 2_000_000_000, splits) is not None
+    symm_mem.check_status("cuda")
+    ulp = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -3
+    x, y = c.float(), whole.float()
+    assert bool(((x - y).abs() <= torch.maximum(x.abs(), y.abs()) * ulp + 0.05 * k * 2.0 ** -22).all())
+    assert intact(), "the kernel stored outside its output"
