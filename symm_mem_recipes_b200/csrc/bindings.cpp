@@ -3,6 +3,7 @@
 // pointers and a stream.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
@@ -44,14 +45,22 @@ torch::Tensor new_tensor(at::IntArrayRef sizes, torch::ScalarType dtype, int dev
 std::mutex g_status_mu;
 std::map<int, Status*> g_status;
 
+// The record of a device, made at its first call, which may be on any stream and beside or under a capture: cleared on
+// a stream of its own that the host waits for.  (A cudaMemset returns before the legacy stream has run it, and a
+// kernel on a non-blocking stream does not wait for that stream: it could lose what the kernel reports.)
 Status* status_for(int device) {
   std::lock_guard<std::mutex> lock(g_status_mu);
   auto it = g_status.find(device);
   if (it != g_status.end()) return it->second;
   c10::cuda::CUDAGuard guard(device);
+  c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
   Status* s = nullptr;
+  cudaStream_t own = nullptr;
   rt_check(cudaMalloc(reinterpret_cast<void**>(&s), sizeof(Status)), "cudaMalloc(status)");
-  rt_check(cudaMemset(s, 0, sizeof(Status)), "cudaMemset(status)");
+  rt_check(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking), "cudaStreamCreate(status)");
+  rt_check(cudaMemsetAsync(s, 0, sizeof(Status), own), "cudaMemsetAsync(status)");
+  rt_check(cudaStreamSynchronize(own), "cudaStreamSynchronize(status)");
+  rt_check(cudaStreamDestroy(own), "cudaStreamDestroy(status)");
   g_status[device] = s;
   return s;
 }
@@ -64,7 +73,10 @@ py::tuple read_status(int device) {
   Status h{};
   rt_check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
   rt_check(cudaMemcpy(&h, s, sizeof(Status), cudaMemcpyDeviceToHost), "cudaMemcpy(status)");
-  if (h.code != 0) rt_check(cudaMemset(s, 0, sizeof(Status)), "cudaMemset(status)");
+  if (h.code != 0) {
+    rt_check(cudaMemset(s, 0, sizeof(Status)), "cudaMemset(status)");
+    rt_check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");      // before the next kernel on a non-blocking stream
+  }
   return py::make_tuple(h.code, h.rank, h.block, h.peer, h.where, h.aux);
 }
 

@@ -105,8 +105,9 @@ extern "C" int smr_gemv_bf16_noalloc_status(void* stream_ptr, unsigned int recor
     record[3] = st.peer; record[4] = st.where; record[5] = st.aux;
   }
   if (st.code == kOk) return 0;
-  e = cudaMemset(base + kNoallocStatusOffset, 0, sizeof(Status));    // reported once
-  if (e != cudaSuccess) return noalloc_fail(3, err, err_len, "cudaMemset(status): ", cudaGetErrorString(e));
+  e = cudaMemsetAsync(base + kNoallocStatusOffset, 0, sizeof(Status), stream);    // reported once
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);                        // before a call on any other stream
+  if (e != cudaSuccess) return noalloc_fail(3, err, err_len, "clear of the status: ", cudaGetErrorString(e));
   return noalloc_fail(4, err, err_len, "a wait inside an earlier call ran out after 2 s (the CTAs of the kernel were "
                                        "not all resident at once?); that call left `out` unwritten");
 }

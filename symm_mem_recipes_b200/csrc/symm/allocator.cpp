@@ -235,6 +235,9 @@ void CudaSymmAllocation::finish_rendezvous() {
   rt_check(cudaMalloc(reinterpret_cast<void**>(&pads_dev_), sizeof(void*) * kMaxWorldSize), "cudaMalloc");
   rt_check(cudaMemcpy(buffers_dev_, bufs.data(), sizeof(void*) * world_size_, cudaMemcpyHostToDevice), "cudaMemcpy");
   rt_check(cudaMemcpy(pads_dev_, pads.data(), sizeof(void*) * world_size_, cudaMemcpyHostToDevice), "cudaMemcpy");
+  // a copy from pageable memory may return before its last part is on the device; kernels on non-blocking streams
+  // do not wait for it
+  rt_check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
   rendezvoused_ = true;
 }
 
