@@ -20,6 +20,7 @@
 #include "../device/multimem.cuh"
 #include "../device/vec.cuh"
 #include "launch.h"
+#include "residency.h"
 
 namespace smr {
 
@@ -160,7 +161,7 @@ one_shot_all_reduce_kernel(PeerPtrs ptrs, int rank, size_t offset_bytes, Vec16* 
 // itself).  Four 16-byte loads in flight per thread (eight: 14 MiB 6.7 us instead of 6.2) and up to 64 CTAs per SM in
 // turns.  kStream: from 32 MiB on input and output do not fit into one die's half of L2, and stores that leave it
 // first are faster (64 MiB: 22.9 us against 23.9); below, the output stays for its reader.
-constexpr int kLocalThreads = 256, kLocalUnroll = 4, kLocalMaxCtas = 148 * 64;
+constexpr int kLocalThreads = 256, kLocalUnroll = 4, kLocalCtasPerSm = 64;
 constexpr size_t kLocalStreamVecs = ((size_t)32 << 20) / 16;
 template <bool kStream>
 __global__ void __launch_bounds__(kLocalThreads)
@@ -408,7 +409,8 @@ int launch_one_shot_all_reduce(const PeerView& pv, const PeerPtrs& ptrs, size_t 
   if (pv.world_size == 1) {
     if (n_vec == 0) return cudaSuccess;
     const size_t chunks = (n_vec + (size_t)kLocalThreads * kLocalUnroll - 1) / ((size_t)kLocalThreads * kLocalUnroll);
-    const int blocks = (int)(chunks < kLocalMaxCtas ? chunks : kLocalMaxCtas);
+    const size_t most = (size_t)device_sms() * kLocalCtasPerSm;
+    const int blocks = (int)(chunks < most ? chunks : most);
     auto kernel = n_vec >= kLocalStreamVecs ? local_one_shot_kernel<true> : local_one_shot_kernel<false>;
     kernel<<<blocks, kLocalThreads, 0, stream>>>(
         reinterpret_cast<Vec16*>(static_cast<char*>(ptrs.buffers[0]) + offset_bytes), static_cast<Vec16*>(out), n_vec,

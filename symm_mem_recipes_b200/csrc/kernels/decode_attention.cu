@@ -18,6 +18,7 @@
 #include "../device/vec.cuh"
 #include "decode_attention.cuh"
 #include "launch.h"
+#include "residency.h"
 
 namespace smr {
 
@@ -173,7 +174,7 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 // would double the time.  A CTA's eight warps take 16 positions each, so more splits than s_max / 128 would
 // leave CTAs without a tile even at the end of the context; few enough for one CTA to combine them.
 int splits_for(int rows, int s_max) {
-  int n = 296 / (rows > 0 ? rows : 1);
+  int n = 2 * device_sms() / (rows > 0 ? rows : 1);
   const int by_length = (s_max + kTile * kWarps - 1) / (kTile * kWarps);
   if (n > by_length) n = by_length;
   return n < 1 ? 1 : (n > kMaxSplit ? kMaxSplit : n);

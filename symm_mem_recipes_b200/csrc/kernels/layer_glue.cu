@@ -22,6 +22,7 @@
 #include "../device/pdl.cuh"
 #include "../device/vec.cuh"
 #include "launch.h"
+#include "residency.h"
 
 namespace smr {
 
@@ -282,9 +283,10 @@ int launch_rms_norm(const void* x, const void* residual, const void* w, void* su
     rms_norm_long_kernel<<<rows, 256, 0, stream>>>(xb, rb, wb, sb, ob, H, eps);
     return (int)cudaGetLastError();
   }
+  const int sms = device_sms();
   auto go = [&](auto kernel, int threads, int per_sm) {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(rows < 148 * per_sm ? rows : 148 * per_sm));
+    cfg.gridDim = dim3((unsigned)(rows < sms * per_sm ? rows : sms * per_sm));
     cfg.blockDim = dim3((unsigned)threads);
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -298,7 +300,7 @@ int launch_rms_norm(const void* x, const void* residual, const void* w, void* su
   // registers of the widest rows allow per SM
   auto pick = [&](auto res) {
     constexpr bool R = decltype(res)::value;
-    if (rows < 148 && n_vec > 256 && n_vec <= 1024) return go(rms_norm_kernel<1024, 1, R>, 1024, 1);
+    if (rows < sms && n_vec > 256 && n_vec <= 1024) return go(rms_norm_kernel<1024, 1, R>, 1024, 1);
     if (n_vec <= 256) return go(rms_norm_kernel<256, 1, R>, 256, 4);
     if (n_vec <= 512) return go(rms_norm_kernel<256, 2, R>, 256, 4);
     if (n_vec <= 1024) return go(rms_norm_kernel<256, 4, R>, 256, R ? 2 : 3);

@@ -20,6 +20,7 @@
 #include "../device/vec.cuh"
 #include "decode_attention.cuh"
 #include "launch.h"
+#include "residency.h"
 
 namespace smr {
 
@@ -201,7 +202,7 @@ prefill_attention_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* _
 bool prefill_attention_preferred(int batch, int seq, int hq, int hkv, int head_dim) {
   if ((head_dim != 64 && head_dim != 128) || hkv < 1 || hq % hkv != 0) return false;
   const double ctas = (double)batch * hq * ((seq + kRows - 1) / kRows), read = (double)batch * hq * seq * seq / 8.0 * head_dim;
-  return ctas <= 592.0 && read <= 48.0e6;
+  return ctas <= 4.0 * device_sms() && read <= 48.0e6;
 }
 
 int launch_prefill_attention(const void* qkv, void* out, int batch, int seq, int hq, int hkv, int head_dim, cudaStream_t stream) {

@@ -13,10 +13,26 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <mutex>
 #include <unordered_map>
 
 namespace smr {
+
+// SMs of the current device, asked once per device.  Without one (sizes computed on a host) those of a B200.
+inline int device_sms() {
+  constexpr int kKnown = 64, kB200 = 148;
+  static std::atomic<int> known[kKnown];
+  int dev = -1, sms = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kKnown && (sms = known[dev].load(std::memory_order_relaxed)) > 0)
+    return sms;
+  if (dev < 0 || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) {
+    (void)cudaGetLastError();
+    return kB200;
+  }
+  if (dev < kKnown) known[dev].store(sms, std::memory_order_relaxed);
+  return sms;
+}
 
 // 0 when `grid` CTAs of `threads` threads and `smem` bytes of dynamic shared memory (in clusters of
 // `cluster` CTAs) fit on the current device at once, else a cudaError_t.  Answers are cached per

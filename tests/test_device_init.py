@@ -48,3 +48,13 @@ def test_first_call_of_a_process_may_be_captured():
     out = subprocess.run([sys.executable, "-c", _FIRST_CALL_IN_A_CAPTURE], cwd=CSRC.parent.parent, capture_output=True,
                          text=True, timeout=200)
     assert out.returncode == 0 and "first call ok" in out.stdout, out.stderr[-2000:]
+
+
+def test_launchers_ask_the_device_for_its_sms():
+    """148, or a multiple of it, in a launcher would size the grids of one chip."""
+    bad = []
+    for path in sorted((CSRC / "kernels").rglob("*.cu")):
+        for n, ln in enumerate(path.read_text().splitlines(), 1):
+            if re.search(r"\b(148|296|592|9472)\b", ln.split("//")[0]):
+                bad.append(f"{path.name}:{n}: {ln.strip()}")
+    assert not bad, bad
