@@ -224,20 +224,18 @@ void CudaSymmAllocation::multicast_teardown() {
 
 void CudaSymmAllocation::finish_rendezvous() {
   rt_check(cudaSetDevice(device_), "cudaSetDevice");
-  std::vector<void*> bufs(world_size_);
-  std::vector<uint32_t*> pads(world_size_);
+  void* tables[2 * kMaxWorldSize] = {};                            // payload bases, then signal pads
   for (int r = 0; r < world_size_; ++r) {
     if (peer_va_[r] == 0) throw std::runtime_error("rendezvous: rank " + std::to_string(r) + " was never mapped");
-    bufs[r] = reinterpret_cast<void*>(peer_va_[r]);
-    pads[r] = reinterpret_cast<uint32_t*>(peer_va_[r] + pad_offset_);
+    tables[r] = reinterpret_cast<void*>(peer_va_[r]);
+    tables[kMaxWorldSize + r] = reinterpret_cast<void*>(peer_va_[r] + pad_offset_);
   }
-  rt_check(cudaMalloc(reinterpret_cast<void**>(&buffers_dev_), sizeof(void*) * kMaxWorldSize), "cudaMalloc");
-  rt_check(cudaMalloc(reinterpret_cast<void**>(&pads_dev_), sizeof(void*) * kMaxWorldSize), "cudaMalloc");
-  rt_check(cudaMemcpy(buffers_dev_, bufs.data(), sizeof(void*) * world_size_, cudaMemcpyHostToDevice), "cudaMemcpy");
-  rt_check(cudaMemcpy(pads_dev_, pads.data(), sizeof(void*) * world_size_, cudaMemcpyHostToDevice), "cudaMemcpy");
+  rt_check(cudaMalloc(reinterpret_cast<void**>(&buffers_dev_), sizeof(tables)), "cudaMalloc");
+  pads_dev_ = reinterpret_cast<uint32_t**>(buffers_dev_ + kMaxWorldSize);
+  rt_check(cudaMemcpy(buffers_dev_, tables, sizeof(tables), cudaMemcpyHostToDevice), "cudaMemcpy");
   // a copy from pageable memory may return before its last part is on the device; kernels on non-blocking streams
   // do not wait for it
-  rt_check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
+  rt_check(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize");
   rendezvoused_ = true;
 }
 
@@ -256,7 +254,6 @@ void CudaSymmAllocation::release() {
     peer_va_[r] = 0;
   }
   if (buffers_dev_ != nullptr) cudaFree(buffers_dev_);
-  if (pads_dev_ != nullptr) cudaFree(pads_dev_);
   buffers_dev_ = nullptr;
   pads_dev_ = nullptr;
   if (va_ != 0) {
