@@ -409,7 +409,8 @@ int launch_one_shot_all_reduce(const PeerView& pv, const PeerPtrs& ptrs, size_t 
   if (pv.world_size == 1) {
     if (n_vec == 0) return cudaSuccess;
     const size_t chunks = (n_vec + (size_t)kLocalThreads * kLocalUnroll - 1) / ((size_t)kLocalThreads * kLocalUnroll);
-    const size_t most = (size_t)device_sms() * kLocalCtasPerSm;
+    // one SM's share needs no look at the device: 0.1 us of a 4.3 us call
+    const size_t most = chunks <= kLocalCtasPerSm ? chunks : (size_t)device_sms() * kLocalCtasPerSm;
     const int blocks = (int)(chunks < most ? chunks : most);
     auto kernel = n_vec >= kLocalStreamVecs ? local_one_shot_kernel<true> : local_one_shot_kernel<false>;
     kernel<<<blocks, kLocalThreads, 0, stream>>>(
