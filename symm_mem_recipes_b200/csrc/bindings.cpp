@@ -903,7 +903,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   }, py::arg("x"), py::arg("residual"), py::arg("w"), py::arg("sum_out"), py::arg("out"), py::arg("eps"));
   // `pos` (optional): int32 CUDA tensor of one element that holds the first position; read on the device
   m.def("rope_inplace", [](torch::Tensor qkv, int n_heads, int head_dim, int seq, int pos0, double theta,
-                           int /*num_sms*/, c10::optional<torch::Tensor> pos) {
+                           int /*num_sms: the grid follows from the tokens*/, c10::optional<torch::Tensor> pos) {
     TORCH_CHECK(qkv.is_cuda() && qkv.is_contiguous() && qkv.dim() == 2 && qkv.scalar_type() == torch::kBFloat16,
                 "rope_inplace: qkv[tokens, row] contiguous bf16 on the GPU");
     int dev = qkv.get_device();

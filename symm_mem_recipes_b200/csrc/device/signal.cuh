@@ -30,11 +30,6 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ uint32_t ld_relaxed_sys(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.relaxed.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ uint32_t ld_relaxed_gpu(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -45,9 +40,6 @@ __device__ __forceinline__ void st_release_sys(uint32_t* p, uint32_t v) {
 }
 __device__ __forceinline__ void st_release_gpu(uint32_t* p, uint32_t v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ void st_relaxed_sys(uint32_t* p, uint32_t v) {
-  asm volatile("st.relaxed.sys.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 __device__ __forceinline__ void red_add_release_sys(uint32_t* p, uint32_t v) {
   asm volatile("red.release.sys.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
@@ -66,12 +58,6 @@ __device__ __forceinline__ uint32_t cas_acquire_sys(uint32_t* p, uint32_t cmp, u
   asm volatile("atom.global.acquire.sys.cas.b32 %0, [%1], %2, %3;"
                : "=r"(old) : "l"(p), "r"(cmp), "r"(val) : "memory");
   return old;
-}
-__device__ __forceinline__ void fence_acq_rel_sys() {
-  asm volatile("fence.acq_rel.sys;" ::: "memory");
-}
-__device__ __forceinline__ void fence_acq_rel_gpu() {
-  asm volatile("fence.acq_rel.gpu;" ::: "memory");
 }
 // Orders generic-proxy accesses against async-proxy (TMA) accesses.
 __device__ __forceinline__ void fence_proxy_async() {
@@ -136,14 +122,6 @@ __device__ __forceinline__ bool wait_ge_acquire_gpu(const uint32_t* p, uint32_t 
                                                     uint64_t timeout_ns) {
   Deadline d(timeout_ns);
   while (ld_acquire_gpu(p) < target) {
-    if (!d.alive()) return false;
-  }
-  return true;
-}
-__device__ __forceinline__ bool wait_eq_acquire_sys(const uint32_t* p, uint32_t target,
-                                                    uint64_t timeout_ns) {
-  Deadline d(timeout_ns);
-  while (ld_acquire_sys(p) != target) {
     if (!d.alive()) return false;
   }
   return true;
