@@ -42,7 +42,7 @@ def main() -> int:
     args = ap.parse_args()
 
     import symm_mem_recipes_b200 as smr
-    from symm_mem_recipes_b200.ops.ag_matmul import AgMatmulConfig, choose_block_n
+    from symm_mem_recipes_b200.ops.ag_matmul import AgMatmulConfig
     from symm_mem_recipes_b200.parallel import symm_mem
     from symm_mem_recipes_b200.utils.benchmark import (ClockSampler, benchmark_with_event,
                                                        benchmark_with_graph)
@@ -64,7 +64,7 @@ def main() -> int:
             cfg = AgMatmulConfig(block_n=args.block_n)
             us = benchmark_with_event(lambda: smr.matmul(a, b, c, cfg, epilogue), **bench)
             out.update(smr_us=round(us, 1), smr_tflops=round(flops / us / 1e6, 1))
-            out.update(M=M, N=N, K=K, variant=args.variant, block_n=args.block_n or choose_block_n(M, N, 148))
+            out.update(M=M, N=N, K=K, variant=args.variant, block_n=args.block_n or "planned")
             if not args.no_cublas and args.variant == "bf16":
                 bt = b.t()
                 us2 = benchmark_with_event(lambda: torch.matmul(a, bt, out=c), **bench)

@@ -713,6 +713,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("block_n"), py::arg("num_sms"), py::arg("split_k"), py::arg("panel_w"), py::arg("timeout_ns"),
         py::arg("max_splits") = 0);
 
+  m.def("gemm_kernels", &gemm_kernels, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("elem_bytes"), py::arg("num_sms"),
+        py::arg("gather"));
+
   m.def("check_push_schedule", &check_push_schedule);
   m.def("check_pair_work", &check_pair_work);
   m.def("check_rs_pair_schedule", &check_rs_pair_schedule);

@@ -688,6 +688,12 @@ MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int bl
   return best;
 }
 
+int gemm_kernels(int M, int N, int K, int elem_bytes, int num_sms, bool gather) {
+  if (!gather) return plan_matmul(M, N, K, elem_bytes, 0, 0, num_sms, 0).tail_splits > 1 ? 2 : 1;
+  const int tiles = (M + 2 * kBM - 1) / (2 * kBM) * ((N + 255) / 256), pairs = num_sms < 4 ? 1 : num_sms / 2;
+  return tail_parts(tiles % pairs, pairs, (K * elem_bytes + 127) / 128, 0) > 1 ? 2 : 1;
+}
+
 int launch_ag_matmul_2cta(const AgMatmulArgs& a, cudaStream_t stream) {
   if (a.elem_bytes != 0 && a.elem_bytes != 1 && a.elem_bytes != 2) return cudaErrorInvalidValue;
   const bool fp8 = a.elem_bytes == 1;

@@ -124,6 +124,9 @@ struct MatmulPlan {
   size_t tail_bytes;      // scratch for them
 };
 MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int block_n, int num_sms, int max_splits);
+// Kernels that such a GEMM launches (bf16 or fp8, planned width; with `gather` the width and cut of the fused kernel): 1, or
+// 2 where tiles are cut and their parts added up.
+int gemm_kernels(int M, int N, int K, int elem_bytes, int num_sms, bool gather);
 
 // Host-side checks of the kernels' scheduling arithmetic (schedule_check.cu); 0 = invariants hold.
 int check_push_schedule(int world_size, int rank, int blocks_per_rank, int n_tiles_n, int n_units,

@@ -19,6 +19,15 @@ def test_tail_needs_no_state_and_no_waits():
     assert not re.search(r"counters|marks", (CSRC / "bindings.cpp").read_text())
 
 
+def test_launches_of_a_cut_gemm_are_counted():
+    """What bench.py reports as its launches: 896 tiles on 74 pairs leave 8, which are cut; 74 x 12 tiles leave none."""
+    from symm_mem_recipes_b200._ext import C
+
+    assert all(C.gemm_kernels(16384, 3584, 8192, 2, 148, gather) == 2 for gather in (False, True))
+    assert all(C.gemm_kernels(74 * 256, 12 * 256, 8192, 2, 148, gather) == 1 for gather in (False, True))
+    assert C.gemm_kernels(256, 64, 128, 2, 148, False) == 1      # too short a K to cut
+
+
 def test_calls_that_are_alive_at_once_share_no_scratch():
     import importlib
 
