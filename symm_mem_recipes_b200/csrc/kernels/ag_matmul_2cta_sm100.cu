@@ -638,13 +638,14 @@ int tail_parts(int rem, int pairs, int k_blocks, int most) {
 // Tile width and tail of a GEMM by a model of its time, fitted to measurements of every width and split on 21 shapes
 // (M 17 to 6000): a wave of n of the P pairs takes, per K block of 128 bytes, t1 with few pairs at work (the
 // tensor core's own rate) up to t1 + t2 with all of them (shared L2 and power), so narrow tiles win where tiles
-// are few and 256 columns where waves are full; cutting the last wave along K costs a pass through L2.
+// are few and 256 columns where waves are full; cutting the last wave along K costs a pass through L2 (`merge`, fitted
+// when the parts were still added up inside the GEMM: merge_tail_kernel takes the same within 1 us).
 // Two more terms, fitted on 17 shapes (M 2048 to 16384).  Rows whose pitch is no multiple of 128 bytes make every
 // TMA row touch two L2 lines: `skew` more per K block (fp8 13201 x 880 x 7440: 83 us at 256 columns, 102 at
 // 128; with K = 7424 67 and 65).  And a tile cannot take less than its epilogue, `epi` in fp8, where K is short
 // (fp8 9000 x 7168 x 1024: 51 us at 256 columns, 74 at 192, 69 at 128).
 // Examples, before (always 256 columns, no cut below one wave) and after: 64 x 1280 x 8192 41 -> 13 us,
-// 129 x 7168 x 8192 45 -> 32 us, 509 x 1280 x 8192 42 -> 18 us, 300 x 2048 x 2048 15 -> 10 us.
+// 129 x 7168 x 8192 45 -> 32 us, 509 x 1280 x 8192 42 -> 16 us, 300 x 2048 x 2048 15 -> 10 us.
 MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int block_n, int num_sms, int max_splits) {
   struct Width { int bn; double t1, t2, merge, skew, epi; };        // microseconds
   constexpr Width kWidths[] = {{256, 0.285, 0.135, 6.4, 0.07, 3.5}, {192, 0.215, 0.115, 5.4, 0.08, 4.0},

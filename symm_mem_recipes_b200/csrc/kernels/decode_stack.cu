@@ -16,14 +16,17 @@
 //     happen on the way out, so that x comes in by TMA as it is;
 //   * between phases the CTAs meet at a counter in global memory (release add by one thread, acquire poll by one
 //     thread, about 1.3 us); attention is dealt out over (sequence, KV head, split of the context), then the sums of
-//     the splits over (sequence, query head).
+//     the splits over (sequence, query head).  A layer has eight such round trips over the whole grid: six counters,
+//     and twice, before a norm, the exchange of the sums of squares.
 // The CTAs wait for one another, so the launch is cooperative.  Every wait is bounded.
-// Two layers of that share, against the five kernels: batch 1 at position 3000 133 -> 105 us, batch 16 at 6500 172 -> 145 us.
+// Two layers of that share, against the five kernels: batch 1 at position 3000 133 -> 105 us, batch 16 at 6500 172 -> 145
+// us.  Their weights and caches at the measured copy rate take 67 and 83.
 // Of the 48 us a layer takes at batch 1 about 14 are attention with its meeting points, 12 the other meeting points
 // and first loads of x, the rest is the weight stream.
 //
-// Arithmetic is that of the single ops: bf16 activations between phases, fp32 accumulation, the norm rounded before and
-// after its weight, a projection rounded before its residual add, every sum in a fixed order.
+// Arithmetic is that of the single ops but for one rounding: gate and up reach SiLU as fp32 accumulators, where separate ops
+// round them to bf16 first.  Else bf16 activations between phases, fp32 accumulation, the norm rounded before and after
+// its weight, a projection rounded before its residual add, every sum in a fixed order.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -55,9 +58,9 @@ constexpr uint32_t kSlotBytes = 28672;                          // four k blocks
 constexpr int kSlots = 6;
 // The weight stream of an SM at a meeting point: a slot that has not become free for twice the time its bytes take at the
 // SM's share of HBM (25 bytes a cycle) means that the phase is waiting, and then the steps after the ring go into
-// L2 at that rate, up to six of them (25 MB over all SMs).  Two layers at batch 1 / batch 16: without 107.5 / 143, up
-// to 4 steps 101.8 / 138.4, 6 101.0 / 139.9, 12 100.8 / 143.7; all the time instead of only when idle, 4 steps 109 /
-// 147 and 16 steps 136 / 175 us.  Weights are loaded as the first to leave L2 (113 / 151 us before that): what stays
+// L2 at that rate, up to six of them (25 MB over all SMs).  Two layers at batch 1 / batch 16: without 112.5 / 148.6, up
+// to 4 steps 106.1 / 144.8, 6 104.7 / 145.0, 12 106.3 / 148.5 us; all the time instead of only when idle costs 7 us with
+// 4 steps and 33 with 16.  Weights are loaded as the first to leave L2 (5 to 8 us slower before that): what stays
 // are the activations, the new keys and values and what was prefetched.
 constexpr int kAhead = 6;
 constexpr int kShareOfHbm = 25, kIdleCycles = 2 * (int)kSlotBytes / kShareOfHbm;
@@ -82,7 +85,8 @@ constexpr uint32_t kTmemCols = 32;
 static_assert(kCompute == 192 && 16 * 128 * 4 <= kWorkBytes && 4 * 8 * 132 * 4 <= kWorkBytes, "work area");
 static_assert(kSmemTotal <= 232448, "shared memory limit exceeded");
 
-// Meeting points of a layer: what is complete there
+// Counters at which a layer's CTAs meet: what is complete there.  Before kNormedX1 and kNormedY they have met once more,
+// at the sums of squares (`ss`).
 enum Meet { kQkvDone = 0, kSplitsDone, kAttnDone, kNormedX1, kActDone, kNormedY, kMeets };
 enum Phase { kQkv = 0, kO = 1, kGateUp = 2, kDown = 3 };
 
