@@ -163,10 +163,13 @@ rms_norm_long_kernel(const __nv_bfloat16* x, const __nv_bfloat16* residual, cons
 // captured in a CUDA graph takes its position from a tensor).
 // With caches ([tokens / seq, s_max, hkv, D] each) the last hkv of the rotated heads are also written to the key cache
 // and the hkv heads after them to the value cache, at the token's place in its sequence.
-// A warp takes a token: its angles are computed once into shared memory (a sine and cosine per pair instead of one per
-// pair and head), then a lane rotates eight pairs of a head at a time, two heads' loads in flight.  Bound by HBM: at
-// 32768 tokens of 9 heads x 128 the kernel with the angles per head took 47 us and the two cache copies 34.
-__global__ void __launch_bounds__(256)
+// A warp takes a token: its first loads go out, then its angles are computed once into shared memory (a sine and cosine
+// per pair instead of one per pair and head), then a lane rotates eight pairs of a head at a time.  The table is stored
+// by [pair of the eight][eight], because the lanes of a head read the same pair of neighbouring eights: in the order of
+// the pairs that was a 4-way bank conflict, as much time as the memory.  Four CTAs per SM need 64 registers.  Cold, 9 heads x
+// 128: 16384 tokens 24.7 us with the conflicts, 22.5 at three CTAs, 20.5 now; 4096 tokens 12.3, 11.1, 10.3; one angle per
+// pair and head 20.6 and 10.3, but 120 against 100 us for 72 heads of 16384 tokens, and two passes more for the caches.
+__global__ void __launch_bounds__(256, 4)
 rope_kernel(__nv_bfloat16* __restrict__ qkv, long long tokens, int row_stride, int n_heads, int D, int seq, int pos0,
             const int* __restrict__ pos_dev, float log2_theta, __nv_bfloat16* __restrict__ k_cache,
             __nv_bfloat16* __restrict__ v_cache, int s_max, int hkv) {
@@ -179,26 +182,16 @@ rope_kernel(__nv_bfloat16* __restrict__ qkv, long long tokens, int row_stride, i
   if (pos_dev != nullptr) pos0 = *pos_dev;
   const long long in_batch = t / seq;
   const int in_seq = (int)(t - in_batch * seq);
-  float2* mine = angles + warp * half;
-  for (int i = lane; i < half; i += 32) {               // pair index in [0, D/2)
-    const float inv_freq = exp2f(-(2.0f * (float)i / (float)D) * log2_theta);
-    float ang = (float)(pos0 + in_seq) * inv_freq;
-    // bring the angle into [-pi, pi] before the fast sine / cosine
-    ang -= 6.283185307179586f * rintf(ang * 0.15915494309189535f);
-    float sn, cs;
-    __sincosf(ang, &sn, &cs);
-    mine[i] = make_float2(cs, sn);
-  }
-  __syncwarp();
   const int vecs = D / 16;                              // items of eight pairs per head
   const int n_items = (n_heads + (v_cache != nullptr ? hkv : 0)) * vecs;
   __nv_bfloat16* row = qkv + t * row_stride;
   const size_t cache_row = ((size_t)in_batch * s_max + in_seq) * hkv;   // the token's row of a cache, in heads
-  for (int item0 = lane; item0 < n_items; item0 += 64) {
-    Vec16 lo[2], hi[2];
-    int head[2], v[2];
+  constexpr int kPer = 3;                               // a lane's items in flight: a row of 12 heads of 128 in one go
+  Vec16 lo[kPer], hi[kPer];
+  int head[kPer], v[kPer];
+  auto load = [&](int item0) {
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < kPer; ++u) {
       const int item = item0 + 32 * u;
       head[u] = item / vecs;
       v[u] = (item - head[u] * vecs) * 8;
@@ -207,8 +200,23 @@ rope_kernel(__nv_bfloat16* __restrict__ qkv, long long tokens, int row_stride, i
         hi[u] = ld_16_stream(row + (size_t)head[u] * D + half + v[u]);
       }
     }
+  };
+  load(lane);
+  float2* mine = angles + warp * half;
+  for (int i = lane; i < half; i += 32) {               // pair index in [0, D/2)
+    const float inv_freq = exp2f(-(2.0f * (float)i / (float)D) * log2_theta);
+    float ang = (float)(pos0 + in_seq) * inv_freq;
+    // bring the angle into [-pi, pi] before the fast sine / cosine
+    ang -= 6.283185307179586f * rintf(ang * 0.15915494309189535f);
+    float sn, cs;
+    __sincosf(ang, &sn, &cs);
+    mine[(i & 7) * vecs + (i >> 3)] = make_float2(cs, sn);
+  }
+  __syncwarp();
+  for (int item0 = lane; item0 < n_items; item0 += 32 * kPer) {
+    if (item0 != lane) load(item0);
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < kPer; ++u) {
       if (item0 + 32 * u >= n_items) continue;
       if (head[u] >= n_heads) {                         // a value head: only copied
         __nv_bfloat16* dst = v_cache + (cache_row + (head[u] - n_heads)) * D + v[u];
@@ -221,7 +229,7 @@ rope_kernel(__nv_bfloat16* __restrict__ qkv, long long tokens, int row_stride, i
       unpack8(hi[u], x2);
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        const float2 c = mine[v[u] + q];
+        const float2 c = mine[q * vecs + (v[u] >> 3)];
         y1[q] = x1[q] * c.x - x2[q] * c.y;
         y2[q] = x2[q] * c.x + x1[q] * c.y;
       }

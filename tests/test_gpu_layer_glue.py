@@ -59,6 +59,22 @@ def test_rope(batch, seq, hq, hkv, D, pos0):
     assert torch.equal(got[:, (hq + hkv) * D:].cpu(), qkv[:, (hq + hkv) * D:])     # V untouched
 
 
+@pytest.mark.parametrize("tokens,heads,D", [(1, 1, 16), (9, 12, 128), (7, 13, 128), (33, 72, 128), (5, 25, 64), (3, 7, 256)])
+def test_rope_rows_of_one_and_of_several_passes(tokens, heads, D):
+    """A warp holds 96 items (heads x D / 16) of a row at a time: rows of fewer, of exactly as many and of more."""
+    from symm_mem_recipes_b200 import ops
+    from symm_mem_recipes_b200._ext import C
+
+    g = torch.Generator().manual_seed(heads + D)
+    qkv = torch.randn(tokens, (heads + 1) * D, generator=g).to(torch.bfloat16)
+    ref = C.oracle_rope_bf16(qkv, heads, D, tokens, 0, 500000.0)
+    got = ops.rope_(qkv.cuda(), heads, D, tokens, 500000.0)
+    # fp32 angles (the oracle's are fp64): position 32 x 2^-24 relative, far inside the 2e-4 rad of position 2048
+    ok, err = _ulp_close(got, ref, extra_abs=4e-3)
+    assert ok, err
+    assert torch.equal(got[:, heads * D:].cpu(), qkv[:, heads * D:])
+
+
 @pytest.mark.parametrize("rows,F", [(1, 8), (19, 48), (4096, 3584)])
 def test_silu_mul(rows, F):
     from symm_mem_recipes_b200 import ops
