@@ -718,6 +718,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
 
   m.def("check_push_schedule", &check_push_schedule);
   m.def("check_pair_work", &check_pair_work);
+  m.def("check_wide_work", &check_wide_work);
   m.def("check_rs_pair_schedule", &check_rs_pair_schedule);
   m.def("check_rs_progress", &check_rs_progress);
   m.def("gemv_batch_tile", &gemv_batch_tile);

@@ -58,30 +58,34 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-__device__ __forceinline__ void umma_bf16_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                                  uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Same for fp8 (e4m3) operands: kind::f8f6f4 multiplies 32 elements of K per
+// `kCollect`: what becomes of A in the tensor core's operand buffer.  Two MMAs with the same A and different B read A from
+// shared memory once if the first fills the buffer and the second is its last use.
+enum class CollectA { kDiscard, kFill, kLastUse };
+#define SMR_UMMA_PAIR(KIND, COLLECT)                                                              \
+  asm volatile(                                                                                   \
+      "{\n\t"                                                                                     \
+      ".reg .pred p;\n\t"                                                                         \
+      "setp.ne.b32 p, %4, 0;\n\t"                                                                 \
+      "tcgen05.mma.cta_group::2.kind::" KIND COLLECT " [%0], %1, %2, %3, p;\n\t"                  \
+      "}"                                                                                         \
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)                        \
+      : "memory")
+// kFp8: e4m3 operands.  kind::f8f6f4 multiplies 32 elements of K per
 // instruction, i.e. the same 32 bytes of every shared-memory row as kind::f16.
-__device__ __forceinline__ void umma_e4m3_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                                  uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t"
-      "}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
+template <bool kFp8, CollectA kCollect = CollectA::kDiscard>
+__device__ __forceinline__ void umma_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                             uint32_t accumulate) {
+  if constexpr (kFp8) {
+    if constexpr (kCollect == CollectA::kFill) SMR_UMMA_PAIR("f8f6f4", ".collector::a::fill");
+    else if constexpr (kCollect == CollectA::kLastUse) SMR_UMMA_PAIR("f8f6f4", ".collector::a::lastuse");
+    else SMR_UMMA_PAIR("f8f6f4", "");
+  } else {
+    if constexpr (kCollect == CollectA::kFill) SMR_UMMA_PAIR("f16", ".collector::a::fill");
+    else if constexpr (kCollect == CollectA::kLastUse) SMR_UMMA_PAIR("f16", ".collector::a::lastuse");
+    else SMR_UMMA_PAIR("f16", "");
+  }
 }
+#undef SMR_UMMA_PAIR
 // One arrival on the barrier at this offset in BOTH CTAs of the pair once all
 // MMAs issued so far have completed.
 __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {

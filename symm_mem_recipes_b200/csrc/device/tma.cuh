@@ -52,7 +52,10 @@ __device__ __forceinline__ void tma_load_4d_once(void* smem_dst, const CUtensorM
         "r"(x), "r"(y), "r"(z), "r"(w), "l"(policy)
       : "memory");
 }
-// The same box into L2 only.
+// The same boxes into L2 only.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int32_t c0, int32_t c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(c0), "r"(c1) : "memory");
+}
 __device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap* map, int32_t c0, int32_t c1, int32_t c2, int32_t c3) {
   asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];"
                ::"l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");

@@ -41,9 +41,12 @@
 // this library used to carry): 1940 µs against 705-724 µs on 4 GPUs at the
 // Llama-3-70B shape; an ordinary (non-symmetric) a_out is therefore served by this
 // kernel through the internal symmetric buffer plus one local copy.
+//
+// Without a gather, and where there are whole waves of them, two tiles at a time are multiplied by matmul_wide.cuh.
 #include "../device/pdl.cuh"
 #include "../device/tcgen05_pair.cuh"
 #include "ag_matmul_common.cuh"
+#include "matmul_wide.cuh"
 #include "residency.h"
 
 namespace smr {
@@ -260,12 +263,8 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,   // kRe
           const uint64_t db = umma_smem_desc_sw128(sa + L::kABytes);
 #pragma unroll
           for (int k = 0; k < kBK / kUmmaK; ++k) {
-            if constexpr (kFp8)
-              umma_e4m3_ss_pair(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc,
-                                (kb != w.kb0 || k != 0) ? 1u : 0u);
-            else
-              umma_bf16_ss_pair(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc,
-                                (kb != w.kb0 || k != 0) ? 1u : 0u);
+            umma_ss_pair<kFp8>(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc,
+                               (kb != w.kb0 || k != 0) ? 1u : 0u);
           }
           umma_commit_pair(&empty_bar[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -536,7 +535,7 @@ __global__ void __launch_bounds__(kMergeThreads) merge_tail_kernel(const AgMatmu
   if (tail_idx >= p.tail_tiles) return;
   const int n_pair_rows = (p.n_blocks_m + 1) >> 1;
   int prow, ni;
-  tile_coords(p, n_pair_rows, n_pair_rows * p.n_tiles_n - p.tail_tiles + tail_idx, prow, ni);
+  work_coords(p, n_pair_rows, n_pair_rows * p.n_tiles_n - 2 * p.wide_units - p.tail_tiles + tail_idx, 1, prow, ni);
   const int mi = prow * 2 + cta, n_out = kSwiGlu ? p.N >> 1 : p.N, col = ni * kOutCols + g * 8;
   if (mi >= p.n_blocks_m || col >= n_out) return;
   bool local_unused;
@@ -587,6 +586,29 @@ __global__ void __launch_bounds__(kMergeThreads) merge_tail_kernel(const AgMatmu
   }
 }
 
+cudaLaunchConfig_t overlapped(int grid, int threads, uint32_t smem, bool overlap, cudaLaunchAttribute (&attr)[1],
+                              cudaStream_t stream) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid, 1, 1);
+  cfg.blockDim = dim3((unsigned)threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cfg;
+}
+
+template <int BN, bool kFp8, bool kSwiGlu, bool kResidual>
+int launch_merge(const AgMatmulParams& p, cudaStream_t stream) {
+  constexpr int kWarpsPerBlock = kBM / 8 * (kSwiGlu ? BN / 2 : BN) / 32;
+  const int warps = p.tail_tiles * 2 * kWarpsPerBlock;
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = overlapped((warps + kMergeThreads / 32 - 1) / (kMergeThreads / 32), kMergeThreads, 0, true, attr, stream);
+  return (int)cudaLaunchKernelEx(&cfg, merge_tail_kernel<BN, kFp8, kSwiGlu, kResidual>, p);
+}
+
 template <int BN, int STAGES, bool kFp8, bool kSwiGlu = false, bool kResidual = false>
 int launch_pair_variant(const CUtensorMap& ta_shard, const CUtensorMap& ta_out, const CUtensorMap& tb,
                         const CUtensorMap& tc, const AgMatmulParams& p, int grid, bool overlap, cudaStream_t stream) {
@@ -598,25 +620,24 @@ int launch_pair_variant(const CUtensorMap& ta_shard, const CUtensorMap& ta_out, 
   // The pairs of a gather wait for one another's pieces: all of them must be resident.
   if (p.mode != 0)
     if (int rc = check_co_resident(kern, grid, kGemmThreads, L::kTotal, 2)) return rc;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)grid, 1, 1);
-  cfg.blockDim = dim3(kGemmThreads, 1, 1);
-  cfg.dynamicSmemBytes = L::kTotal;
-  cfg.stream = stream;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = overlap ? 1 : 0;
+  const cudaLaunchConfig_t cfg = overlapped(grid, kGemmThreads, L::kTotal, overlap, attr, stream);
   e = cudaLaunchKernelEx(&cfg, kern, ta_shard, ta_out, tb, tc, p);
   if (e != cudaSuccess || p.tail_tiles == 0) return (int)e;
-  constexpr int kWarpsPerBlock = kBM / 8 * (kSwiGlu ? BN / 2 : BN) / 32;
-  const int warps = p.tail_tiles * 2 * kWarpsPerBlock;
-  cfg.gridDim = dim3((unsigned)((warps + kMergeThreads / 32 - 1) / (kMergeThreads / 32)), 1, 1);
-  cfg.blockDim = dim3(kMergeThreads, 1, 1);
-  cfg.dynamicSmemBytes = 0;
-  cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, merge_tail_kernel<BN, kFp8, kSwiGlu, kResidual>, p);
+  return launch_merge<BN, kFp8, kSwiGlu, kResidual>(p, stream);
+}
+
+template <bool kSwiGlu, bool kResidual>
+int launch_wide(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tr,
+                const AgMatmulParams& p, int grid, bool overlap, cudaStream_t stream) {
+  auto kern = wide::matmul_wide_kernel<kSwiGlu, kResidual>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wide::kSmemBytes);
+  if (e != cudaSuccess) return (int)e;
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = overlapped(grid, wide::kThreads, wide::kSmemBytes, overlap, attr, stream);
+  e = cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, tr, p);
+  if (e != cudaSuccess || p.tail_tiles == 0) return (int)e;
+  return launch_merge<wide::kBN, false, kSwiGlu, kResidual>(p, stream);
 }
 
 }  // namespace
@@ -631,6 +652,24 @@ int tail_parts(int rem, int pairs, int k_blocks, int most) {
   if (most > 0 && splits > most) splits = most;
   while (splits > 1 && k_blocks < 2 * splits) --splits;
   return splits;
+}
+
+// Units of two tiles (matmul_wide.cuh) that a GEMM of `rows` x `cols` tiles of 256 x 256 is multiplied in: as many whole
+// waves of them as there are, the rest one tile at a time.  bf16 only: in fp8 the same loads feed twice the flops, and
+// 4096 and 16384 x 3584 x 8192 take 95 and 362 us either way.  The end of a unit costs about 4000 cycles more than that
+// of two single tiles (both accumulators have to be read before the next unit), so K has to be long.  Loops of calls,
+// one tile at a time / two, us:
+//     16384 x 8192 x  1024  2048    16384 x 4096 x  4096  6144    16384 x 3584 x 8192    4096 x 7168 x 8192
+//               218/228  410/413              400/397  642/605                767/700               384/360
+//     with SwiGLU 9000 x 8192 x 4096  2048 x 7168 x 8192  32768 x 7168 x 8192
+//                            444/449             196/186            3020/2790
+//     with residual 16384 x 8192 x 2048  32768 x 8192 x 3584  16384 x 8192 x 7168   (one stage less one tile at a time)
+//                               447/469            1640/1592            1570/1466
+// An odd column of tiles comes after all units and reads all of A again: 8192 x 1280 x 8192 (5 columns) 142/141 but
+// 32768 x 1280 x 8192 535/560 and 32768 x 1792 x 8192 (7) 741/750; 32768 x 2304 x 8192 (9) 952/945.
+int plan_wide_units(int rows, int cols, int pairs, int K, int elem_bytes, bool residual) {
+  if (elem_bytes != 2 || K < (residual ? 3072 : 5120) || (cols % 2 != 0 && cols < 9)) return 0;
+  return rows * (cols / 2) / pairs * pairs;
 }
 
 }  // namespace
@@ -803,6 +842,8 @@ int launch_ag_matmul_2cta(const AgMatmulArgs& a, cudaStream_t stream) {
       if (total_tiles < max_pairs) pairs = rem * splits;
     }
   }
+  if (!comm && bn == 256 && a.trace == nullptr)                    // the timing record is the other kernel's
+    p.wide_units = plan_wide_units((p.n_blocks_m + 1) / 2, p.n_tiles_n, max_pairs, a.K, es, a.residual != nullptr);
   const int grid = 2 * pairs;
   if (comm) {
     if (a.lead < 0) {
@@ -814,6 +855,11 @@ int launch_ag_matmul_2cta(const AgMatmulArgs& a, cudaStream_t stream) {
   }
   // the entry barrier of CTA i uses block slot (barrier_block_base + i): it must stay inside the block-slot region
   if (comm && ((size_t)a.barrier_block_base + grid) * a.world_size > kBlockSlots) return cudaErrorInvalidValue;
+  if (p.wide_units > 0) {
+    if (swiglu) return launch_wide<true, false>(ta_out, tb, tc, ta_shard, p, grid, a.overlap, stream);
+    if (p.residual != nullptr) return launch_wide<false, true>(ta_out, tb, tc, ta_shard, p, grid, a.overlap, stream);
+    return launch_wide<false, false>(ta_out, tb, tc, ta_shard, p, grid, a.overlap, stream);
+  }
   if (swiglu) return launch_pair_variant<256, 6, false, true>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
   if (fp8) {
     switch (bn) {

@@ -43,6 +43,7 @@ struct AgMatmulParams {
   int n_tiles_n;         // ceil(N / BN)
   int panel_w;           // N tiles per column panel of the tile order (n_tiles_n: one panel)
   int n_blocks_m;        // ceil(M / 128)
+  int wide_units;        // units of two neighbouring tiles at the front of the schedule, whole waves of them (0 = none)
   // gather
   int rank, world_size;
   int blocks_per_rank;   // 128-row blocks per shard
@@ -260,6 +261,37 @@ __host__ __device__ __forceinline__ bool pair_work(const AgMatmulParams& p, int 
   w.kb1 = w.kb0 + per < k_blocks ? w.kb0 + per : k_blocks;
   if (w.kb1 < w.kb0) w.kb1 = w.kb0;
   return true;
+}
+// The same with wide units first (`halves` 2: two neighbouring tiles of a row that share their rows of A); `tile` is then an
+// index into the units, or into the tiles they leave over.
+struct WideWork : PairWork {
+  int halves;
+};
+__host__ __device__ __forceinline__ bool wide_work(const AgMatmulParams& p, int pair, int n_pairs, int total_tiles, int k_blocks,
+                                                   int i, WideWork& w) {
+  w.tile = pair + i * n_pairs;
+  if (w.tile < p.wide_units) {
+    w.halves = 2; w.kb0 = 0; w.kb1 = k_blocks; w.part = -1; w.tail_idx = 0;
+    return true;
+  }
+  w.halves = 1;
+  return pair_work(p, pair, n_pairs, total_tiles - 2 * p.wide_units, k_blocks, i - p.wide_units / n_pairs, w);
+}
+// Row and (first) column of a piece of work in units of tiles.  With wide units the tiles are walked in pairs of columns;
+// the pairs that fill no whole wave are single tiles, and so is an odd last column, which comes after them.
+__host__ __device__ __forceinline__ void work_coords(const AgMatmulParams& p, int n_rows, int tile, int halves, int& row, int& ni) {
+  if (p.wide_units == 0) {
+    tile_coords(p, n_rows, tile, row, ni);
+    return;
+  }
+  const int n_wide = p.n_tiles_n >> 1, left = n_rows * n_wide - p.wide_units;
+  if (halves == 1 && tile >= 2 * left) {
+    row = tile - 2 * left;
+    ni = p.n_tiles_n - 1;
+    return;
+  }
+  panel_tile_coords(n_wide, p.panel_w > 1 ? p.panel_w >> 1 : 1, n_rows, halves == 2 ? tile : p.wide_units + (tile >> 1), row, ni);
+  ni = 2 * ni + (halves == 2 ? 0 : tile & 1);
 }
 
 // row-major [rows, cols] of bf16 (or of 1-byte elements) with a box of

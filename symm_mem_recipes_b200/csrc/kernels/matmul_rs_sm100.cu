@@ -182,7 +182,7 @@ matmul_rs_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           const uint64_t db = umma_smem_desc_sw128(sa + L::kABytes);
 #pragma unroll
           for (int k = 0; k < kBK / kUmmaK; ++k)
-            umma_bf16_ss_pair(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc,
+            umma_ss_pair<false>(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc,
                               (kb | k) != 0 ? 1u : 0u);
           umma_commit_pair(&empty_bar[stage]);
           if (++stage == kStages) { stage = 0; phase ^= 1; }

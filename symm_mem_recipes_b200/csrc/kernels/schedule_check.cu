@@ -112,6 +112,36 @@ int check_pair_work(int total_tiles, int n_pairs, int k_blocks, int tail_tiles, 
   return 0;
 }
 
+// The same with wide units at the front, through the places of the tiles: rows x cols tiles, panels of `panel_w` columns.
+int check_wide_work(int rows, int cols, int n_pairs, int k_blocks, int panel_w, int tail_tiles, int tail_splits) {
+  AgMatmulParams p{};
+  p.n_tiles_n = cols;
+  p.panel_w = panel_w;
+  p.wide_units = rows * (cols / 2) / n_pairs * n_pairs;
+  p.tail_tiles = tail_tiles;
+  p.tail_splits = tail_splits;
+  std::vector<int> cover((size_t)rows * cols * k_blocks, 0);
+  for (int pair = 0; pair < n_pairs; ++pair) {
+    WideWork w;
+    int last_halves = 2, units = 0;
+    for (int i = 0; wide_work(p, pair, n_pairs, rows * cols, k_blocks, i, w); ++i) {
+      int row, ni;
+      work_coords(p, rows, w.tile, w.halves, row, ni);
+      if (row < 0 || row >= rows || ni < 0 || ni + w.halves > cols) return 1;
+      if (w.halves > last_halves) return 2;              // the ring counts on wide units first
+      if (w.halves == 2) ++units;
+      last_halves = w.halves;
+      for (int h = 0; h < w.halves; ++h)
+        for (int kb = w.kb0; kb < w.kb1; ++kb) cover[((size_t)row * cols + ni + h) * k_blocks + kb]++;
+      if (i > rows * cols) return 3;
+    }
+    if (units != p.wide_units / n_pairs) return 5;       // and on this many of them
+  }
+  for (int v : cover)
+    if (v != 1) return 4;
+  return 0;
+}
+
 // CTA-pair reduce-scatter kernel: over all pairs, both CTAs and all tiles, every (destination, row
 // block, N tile) is produced exactly once, own rows last inside every column panel (a tile of the own
 // rows waits for the peers' tiles of the same panel, which therefore all come earlier in every

@@ -58,6 +58,37 @@ def test_swiglu_of_separate_and_interleaved_halves(M, F, K):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,sms,splits", [
+    (256, 1024, 5120, 4, 0),          # one wave of units, nothing left
+    (511, 1280, 5128, 8, 0),          # a ragged row, five columns (too few for an odd number: one tile at a time)
+    (700, 2312, 5184, 8, 0),          # ten columns, the last one 8 wide, tiles left over
+    (1290, 2304, 5120, 8, 2),         # nine columns: the odd one comes last, and the tail is cut
+    (769, 1040, 6200, 4, 1),          # no cut; three rows of tiles, the last with one row of C
+])
+def test_two_tiles_at_a_time(M, N, K, sms, splits):
+    from symm_mem_recipes_b200.parallel import symm_mem
+    from symm_mem_recipes_b200.utils.testing import guarded_empty
+
+    a, b = _operands(M, N, K)
+    ref = a.float() @ b.float().t()
+    res = (torch.randn(M, N, device="cuda")).to(torch.bfloat16)
+    gate, up = ref.split(N // 2, dim=1)
+    forms = [(0, None, ref), (0, res, ref + res.float())]
+    if N % 16 == 0:
+        forms.append((2, None, torch.nn.functional.silu(gate) * up))
+    for epilogue, residual, want in forms:
+        c, intact = guarded_empty(tuple(want.shape), torch.bfloat16, "cuda")
+        c.fill_(float("nan"))
+        assert _run(a, b, c, epilogue=epilogue, residual=residual, block_n=256, sms=sms, splits=splits) is not None
+        symm_mem.check_status("cuda")
+        # a bf16 rounding is 2^-9 of the value (two with a residual); the sums of 5000 products of 0.05 differ by 1e-4
+        assert bool(((c.float() - want).abs() <= want.abs() * 2.0 ** -6 + 2e-2).all())
+        assert intact(), "the kernel stored outside its output"
+        if splits == 1:                                  # same products in the same order: the same bits
+            assert torch.equal(c, _run(a, b, epilogue=epilogue, residual=residual, block_n=256, sms=64, splits=1))
+
+
+@pytest.mark.gpu
 def test_split_calls_on_several_streams():
     """Calls whose tiles are cut along K share neither scratch nor counters across streams."""
     from symm_mem_recipes_b200.parallel import symm_mem

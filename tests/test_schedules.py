@@ -76,6 +76,20 @@ def test_split_k_tail_covers_every_tile_once():
     assert not bad, bad[:10]
 
 
+def test_wide_units_cover_every_tile_once():
+    """Two neighbouring tiles at a time for whole waves, the rest one by one or cut, an odd last column at the end."""
+    bad = []
+    for rows, cols, pairs, kb in itertools.product((1, 3, 8, 64), (2, 5, 9, 14, 28), (1, 4, 37, 74), (1, 5, 128)):
+        rem = rows * cols % pairs
+        for panel_w, (tail, splits) in itertools.product({cols, (cols + 1) // 2, 1}, ((0, 1), (rem, pairs // max(rem, 1)))):
+            if tail and (rem * 2 > pairs or kb < 2 * min(splits, 8)):
+                continue
+            rc = C.check_wide_work(rows, cols, pairs, kb, panel_w, tail, min(splits, 8) if tail else 1)
+            if rc != 0:
+                bad.append((rows, cols, pairs, kb, panel_w, tail, splits, rc))
+    assert not bad, bad[:10]
+
+
 def test_reduce_scatter_pair_schedule_covers_every_tile_once():
     # decoder-layer shapes at TP8: 32 row blocks per rank, N = 8192 (32 tiles), 74 pairs
     for rank in range(8):
