@@ -654,6 +654,8 @@ int tail_parts(int rem, int pairs, int k_blocks, int most) {
   return splits;
 }
 
+size_t tail_scratch_bytes(int tiles, int parts, int bn) { return (size_t)tiles * parts * 2 * kBM * bn * sizeof(float); }
+
 // Units of two tiles (matmul_wide.cuh) that a GEMM of `rows` x `cols` tiles of 256 x 256 is multiplied in: as many whole
 // waves of them as there are, the rest one tile at a time.  bf16 only: in fp8 the same loads feed twice the flops, and
 // 4096 and 16384 x 3584 x 8192 take 95 and 362 us either way.  The end of a unit costs about 4000 cycles more than that
@@ -674,46 +676,46 @@ int plan_wide_units(int rows, int cols, int pairs, int K, int elem_bytes, bool r
 
 }  // namespace
 
-// Tile width and tail of a GEMM by a model of its time, fitted to measurements of every width and split on 21 shapes
-// (M 17 to 6000): a wave of n of the P pairs takes, per K block of 128 bytes, t1 with few pairs at work (the
-// tensor core's own rate) up to t1 + t2 with all of them (shared L2 and power), so narrow tiles win where tiles
-// are few and 256 columns where waves are full; cutting the last wave along K costs a pass through L2 (`merge`, fitted
-// when the parts were still added up inside the GEMM: merge_tail_kernel takes the same within 1 us).
-// Two more terms, fitted on 17 shapes (M 2048 to 16384).  Rows whose pitch is no multiple of 128 bytes make every
-// TMA row touch two L2 lines: `skew` more per K block (fp8 13201 x 880 x 7440: 83 us at 256 columns, 102 at
-// 128; with K = 7424 67 and 65).  And a tile cannot take less than its epilogue, `epi` in fp8, where K is short
-// (fp8 9000 x 7168 x 1024: 51 us at 256 columns, 74 at 192, 69 at 128).
-// Examples, before (always 256 columns, no cut below one wave) and after: 64 x 1280 x 8192 41 -> 13 us,
-// 129 x 7168 x 8192 45 -> 32 us, 509 x 1280 x 8192 42 -> 16 us, 300 x 2048 x 2048 15 -> 10 us.
+// Tile width and tail of a GEMM by a model of its time, fitted to loops of calls (so at the clocks the power limit leaves)
+// of every width on 35 bf16 and 28 fp8 shapes (M 131 to 32768): a wave of n of the P pairs takes, per K block of 128
+// bytes, t1 with few pairs at work (the tensor core's own rate) up to t1 + t2 with all of them (shared L2 and power),
+// so narrow tiles win where tiles are few and 256 columns where waves are full; cutting the last wave along K costs 2 us
+// and a pass of the parts through L2 (509 x 1280 x 8192: 128 columns in 3 parts are 2 us faster than 256 in 7).  Rows
+// whose pitch is no multiple of 128 bytes make every TMA row touch two L2 lines: `skew` more per K block.  A tile
+// cannot take less than its epilogue, `epi`, where K is short.  Whole waves of wide units take 0.94 of single tiles.
+// The widths the plan picks are on average 0.3 % slower than the best one of each shape, at worst 5 % (2992 x 6224 x
+// 704: 27.6 us at 192 columns, 26.3 at 256).
+// Examples, fp8, with the figures of before (fitted in short bursts) and now: 4096 x 3584 x 8192 103 -> 97 us (192 -> 256
+// columns), 16384 x 3584 x 8192 386 -> 362, 1024 x 8192 x 8192 65 -> 61; bf16 2992 x 6224 x 704 29.4 -> 27.6.
 MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int block_n, int num_sms, int max_splits) {
-  struct Width { int bn; double t1, t2, merge, skew, epi; };        // microseconds
-  constexpr Width kWidths[] = {{256, 0.285, 0.135, 6.4, 0.07, 3.5}, {192, 0.215, 0.115, 5.4, 0.08, 4.0},
-                               {128, 0.14, 0.095, 4.2, 0.115, 2.5}};
+  struct Width { int bn; double t1, t2, skew, epi; };               // microseconds
+  constexpr Width kBf16[] = {{256, 0.29, 0.15, 0.03, 3.0}, {192, 0.218, 0.135, 0.03, 1.5}, {128, 0.135, 0.12, 0.04, 2.3}};
+  constexpr Width kFp8[] = {{256, 0.29, 0.135, 0.04, 2.7}, {192, 0.225, 0.13, 0.065, 3.0}, {128, 0.125, 0.13, 0.08, 2.0}};
+  const Width(&widths)[3] = elem_bytes == 1 ? kFp8 : kBf16;
   const int pairs = num_sms < 4 ? 1 : num_sms / 2, rows = (M + 2 * kBM - 1) / (2 * kBM);
   const int k_blocks = (K * elem_bytes + 127) / 128;
   MatmulPlan best{block_n != 0 ? block_n : 256, 1, 0};
   double best_cost = -1;
-  for (const Width& w : kWidths) {
+  for (const Width& w : widths) {
     // a width the caller (or the SwiGLU epilogue) asks for is taken with the figures of the nearest one
     if (block_n != 0 || epilogue != 0) {
       if (w.bn != (block_n == 128 || block_n == 192 ? block_n : 256)) continue;
     }
     const int bn = block_n != 0 ? block_n : w.bn;
     const int tiles = rows * (epilogue != 0 ? (N / 2 + bn / 2 - 1) / (bn / 2) : (N + bn - 1) / bn);
-    // full waves of 256 columns lose more in fp8 (twice the MMA rate on the same operand bytes)
-    const double t2 = elem_bytes == 1 && w.bn == 256 ? 0.165 : w.t2;
-    const double t1 = w.t1 + (K * elem_bytes % 128 != 0 ? w.skew : 0.0), least = elem_bytes == 1 ? w.epi : 0.0;
+    const double t1 = w.t1 + (K * elem_bytes % 128 != 0 ? w.skew : 0.0);
     auto wave_us = [&](int n, int parts) {
-      const double us = k_blocks * (t1 + t2 * n * parts / pairs) / parts;
-      return us > least ? us : least;
+      const double us = k_blocks * (t1 + w.t2 * n * parts / pairs) / parts;
+      return us > w.epi ? us : w.epi;
     };
     const int rem = tiles % pairs;
-    double cost = tiles / pairs * wave_us(pairs, 1);
+    const bool wide = bn == 256 && plan_wide_units(rows, tiles / rows, pairs, K, elem_bytes, false) > 0;
+    double cost = tiles / pairs * wave_us(pairs, 1) * (wide ? 0.94 : 1.0);
     int parts = 1;
     if (rem > 0) {
       double tail = wave_us(rem, 1);
       for (int most = tail_parts(rem, pairs, k_blocks, max_splits); most >= 2; --most) {
-        const double cut = wave_us(rem, most) + w.merge;
+        const double cut = wave_us(rem, most) + 2.0 + 0.25e-6 * tail_scratch_bytes(rem, most, bn);
         if (cut < tail) { tail = cut; parts = most; }
       }
       cost += tail;
@@ -722,7 +724,7 @@ MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int bl
       best_cost = cost;
       best.block_n = bn;
       best.tail_splits = parts;
-      best.tail_bytes = parts > 1 ? (size_t)rem * parts * 2 * kBM * bn * sizeof(float) : 0;
+      best.tail_bytes = parts > 1 ? tail_scratch_bytes(rem, parts, bn) : 0;
     }
   }
   return best;
@@ -834,7 +836,7 @@ int launch_ag_matmul_2cta(const AgMatmulArgs& a, cudaStream_t stream) {
   const int rem = total_tiles % max_pairs;
   if (a.tail_scratch != nullptr && rem > 0 && rem * 2 <= max_pairs) {
     int splits = tail_parts(rem, max_pairs, k_blocks, a.tail_splits);
-    while (splits > 1 && (size_t)rem * splits * 2 * kBM * bn * sizeof(float) > a.tail_scratch_bytes) --splits;
+    while (splits > 1 && tail_scratch_bytes(rem, splits, bn) > a.tail_scratch_bytes) --splits;
     if (splits >= 2) {
       p.tail_tiles = rem;
       p.tail_splits = splits;
