@@ -60,7 +60,7 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* k_
   }
   const __nv_bfloat16* row = qkv + (size_t)b * (hq + 2 * hkv) * D;
   attn::State<D> st;
-  attn::attend<D>(kc, vc, pitch, pos, unit, n_units, G, scale, log2_theta != 0.f ? angles : nullptr, [] {},
+  attn::attend<D, false>(kc, vc, pitch, pos, unit, n_units, G, scale, log2_theta != 0.f ? angles : nullptr, [] {},
                   [&](int part, int head, int d) {
                     const int h = part == 0 ? kvh * G + head : (part == 1 ? hq + kvh : hq + hkv + kvh);
                     return ld_16(row + (size_t)h * D + d);

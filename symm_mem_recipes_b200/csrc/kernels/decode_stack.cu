@@ -258,7 +258,7 @@ __device__ __forceinline__ bool attend_item(const StackParams& p, uint8_t* smem,
     }
   };
   attn::State<D> st;
-  attn::attend<D>(L.k_cache + base, L.v_cache + base, (size_t)pitch, pos, unit, n_units, G, p.scale, nullptr, ready,
+  attn::attend<D, true>(L.k_cache + base, L.v_cache + base, (size_t)pitch, pos, unit, n_units, G, p.scale, nullptr, ready,
                   [&](int part, int head, int d) {
                     const int r = part == 0 ? head : G + part - 1;
                     return *reinterpret_cast<const Vec16*>(row + r * D + d);
@@ -689,22 +689,15 @@ __global__ void __launch_bounds__(kThreads, 1) decode_stack_kernel(const __grid_
       }
       return true;
     };
-    // The keys and values of this CTA's first share of the attention into L2, up to six tiles per warp, while the
-    // queries are still being made (DRAM idles at the meeting points: the weight ring is full by then).
+    // The keys and values of this CTA's first share of the attention into L2, two tiles per warp, while the queries are still
+    // being made (DRAM idles at the meeting points: the weight ring is full by then).
     auto prefetch_kv = [&](int l, int pos) {
       const int bh_total = p.batch * p.hkv, bh = cta % bh_total, split = cta / bh_total;
       if (split >= p.n_split) return;
       const int b = bh / p.hkv, kvh = bh - b * p.hkv, pitch = p.hkv * D, n_units = p.n_split * kWarps;
       const size_t base = ((size_t)b * p.s_max * p.hkv + kvh) * D;
-      const int row = D == 128 ? lane >> 1 : lane & 15, off = D == 128 ? (lane & 1) * 64 : 0;
-      int unit = cw * p.n_split + split;
-      for (int i = 0; i < 6; ++i, unit += n_units) {
-        const int at = (unit - 1) * attn::kTile + row;
-        if (unit > 0 && at < pos) {
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(p.layer[l].k_cache + base + (size_t)at * pitch + off));
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(p.layer[l].v_cache + base + (size_t)at * pitch + off));
-        }
-      }
+      for (int i = 0, unit = cw * p.n_split + split; i < 2; ++i, unit += n_units)
+        attn::prefetch_tile<D>(p.layer[l].k_cache + base, p.layer[l].v_cache + base, (size_t)pitch, pos, unit);
     };
 
     int pos = p.pos_dev != nullptr ? *p.pos_dev : p.pos0;
