@@ -115,7 +115,7 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,   // kRe
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cta_rank = cluster_ctarank();
   const bool leader = cta_rank == 0;
-  static_assert(!kSwiGlu || (BN == 256 && !kFp8), "the SwiGLU epilogue is built for bf16 tiles of 256 columns");
+  static_assert(!kSwiGlu || ((BN == 256 || BN == 224) && !kFp8), "the SwiGLU epilogue is built for bf16 tiles of 256 or 224 columns");
 
   uint32_t epoch = 0, flag_target = p.flag_target;
   if (p.mode == 2) {
@@ -442,6 +442,28 @@ ag_matmul_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a_shard,   // kRe
           }
           if constexpr (!kResidual) out_box ^= 1;
         }
+      } else if constexpr (kSwiGlu) {
+#pragma unroll 1
+        for (int c = 0; c < kOutCols / 16; ++c) {
+          uint32_t g[16], u[16];
+          tmem_ld_32x32b_x16(taddr + (uint32_t)(c * 16), g);
+          tmem_ld_32x32b_x16(taddr + (uint32_t)(BN / 2 + c * 16), u);
+          tmem_ld_wait();
+#pragma unroll
+          for (int v = 0; v < 2; ++v) {
+            if (row_ok && col0 + c * 16 + v * 8 < n_out) {
+              float y[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const float x = __uint_as_float(g[v * 8 + i]);
+                y[i] = x / (1.0f + __expf(-x)) * __uint_as_float(u[v * 8 + i]);
+              }
+              st_16(crow + (c * 16 + v * 8) * 2, Vec16{pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]),
+                                                       pack_bf16x2(y[4], y[5]), pack_bf16x2(y[6], y[7])});
+            }
+          }
+        }
+        release_accumulator();
       } else {
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
@@ -624,7 +646,8 @@ int launch_pair_variant(const CUtensorMap& ta_shard, const CUtensorMap& ta_out, 
   const cudaLaunchConfig_t cfg = overlapped(grid, kGemmThreads, L::kTotal, overlap, attr, stream);
   e = cudaLaunchKernelEx(&cfg, kern, ta_shard, ta_out, tb, tc, p);
   if (e != cudaSuccess || p.tail_tiles == 0) return (int)e;
-  return launch_merge<BN, kFp8, kSwiGlu, kResidual>(p, stream);
+  if constexpr (kSwiGlu && BN == 224) return cudaErrorInvalidValue;  // never cut: its columns are no whole groups of the merge
+  else return launch_merge<BN, kFp8, kSwiGlu, kResidual>(p, stream);
 }
 
 template <bool kSwiGlu, bool kResidual>
@@ -727,6 +750,17 @@ MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int bl
       best.tail_bytes = parts > 1 ? tail_scratch_bytes(rem, parts, bn) : 0;
     }
   }
+  // Gate and up in two halves of B: 112 columns of each, uncut, where that fills the pairs better (K 8192, us): 300 x 7168
+  // 50 -> 45, 509 x 7168 57 -> 53 (64 tiles on 74 pairs instead of 56), 509 x 14336 106 -> 103, 900 x 7168 113 -> 107, 1500 x
+  // 7168 150 -> 146; 385 x 4000 x 2048 24.5 -> 21.1.  Its rows of C are 224 bytes, so the lanes store them themselves.
+  if (epilogue == 2 && block_n == 0) {
+    const int tiles = rows * ((N / 2 + 111) / 112), rem = tiles % pairs;
+    auto wave_us = [&](int n) {
+      const double us = k_blocks * (0.254 + (K % kBK != 0 ? 0.03 : 0.0) + 0.143 * n / pairs);
+      return us > 4.0 ? us : 4.0;
+    };
+    if (tiles / pairs * wave_us(pairs) + (rem > 0 ? wave_us(rem) : 0.0) < 0.97 * best_cost) best = MatmulPlan{224, 1, 0};
+  }
   return best;
 }
 
@@ -754,8 +788,10 @@ int launch_ag_matmul_2cta(const AgMatmulArgs& a, cudaStream_t stream) {
   if (bn != 128 && bn != 192 && bn != 224 && bn != 256) return cudaErrorInvalidValue;
   const bool swiglu = a.epilogue != 0;
   if (a.epilogue < 0 || a.epilogue > 2) return cudaErrorInvalidValue;
-  // bf16, 256-column tiles; interleaved in groups of 128 rows of B: whole groups only
-  if (swiglu && (fp8 || bn != 256 || a.N % (a.epilogue == 1 ? 256 : 16) != 0)) return cudaErrorInvalidValue;
+  // bf16, 256-column tiles, or 224 uncut; interleaved in groups of 128 rows of B: whole groups of 256 columns only
+  if (swiglu && (fp8 || (bn != 256 && (bn != 224 || a.epilogue != 2 || a.tail_scratch != nullptr || comm)) ||
+                 a.N % (a.epilogue == 1 ? 256 : 16) != 0))
+    return cudaErrorInvalidValue;
   if (a.residual != nullptr && (swiglu || fp8 || comm || bn == 224 || (uintptr_t)a.residual % 16 != 0))
     return cudaErrorInvalidValue;
 
@@ -862,6 +898,7 @@ int launch_ag_matmul_2cta(const AgMatmulArgs& a, cudaStream_t stream) {
     if (p.residual != nullptr) return launch_wide<false, true>(ta_out, tb, tc, ta_shard, p, grid, a.overlap, stream);
     return launch_wide<false, false>(ta_out, tb, tc, ta_shard, p, grid, a.overlap, stream);
   }
+  if (swiglu && bn == 224) return launch_pair_variant<224, 7, false, true>(ta_shard, ta_out, tb, tc, p, grid, a.overlap, stream);
   if (swiglu) return launch_pair_variant<256, 6, false, true>(ta_shard, ta_out, tb, tc, p, grid, a.overlap && !comm, stream);
   if (fp8) {
     switch (bn) {

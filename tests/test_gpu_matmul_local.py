@@ -58,6 +58,24 @@ def test_swiglu_of_separate_and_interleaved_halves(M, F, K):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,F,K", [(129, 7168, 2048), (509, 3584, 2048), (385, 6984, 1032)])
+def test_swiglu_in_narrower_tiles(M, F, K):
+    """Sizes at which tiles of 112 gate and 112 up columns fill the pairs better; the last one ends inside a tile."""
+    from symm_mem_recipes_b200.parallel import symm_mem
+    from symm_mem_recipes_b200.utils.testing import guarded_empty
+
+    a, b = _operands(M, 2 * F, K)
+    g, u = (a.float() @ b.float().t()).split(F, dim=1)
+    want = torch.nn.functional.silu(g) * u
+    c, intact = guarded_empty((M, F), torch.bfloat16, "cuda")
+    c.fill_(float("nan"))
+    assert _run(a, b, c, epilogue=2) is not None
+    symm_mem.check_status("cuda")
+    assert bool(((c.float() - want).abs() <= want.abs() * 2.0 ** -6 + 2e-2).all())
+    assert intact(), "the kernel stored outside its output"
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("M,N,K,sms,splits", [
     (256, 1024, 5120, 4, 0),          # one wave of units, nothing left
     (511, 1280, 5128, 8, 0),          # a ragged row, five columns (too few for an odd number: one tile at a time)
