@@ -705,14 +705,14 @@ int plan_wide_units(int rows, int cols, int pairs, int K, int elem_bytes, bool r
 // so narrow tiles win where tiles are few and 256 columns where waves are full; cutting the last wave along K costs 2 us
 // and a pass of the parts through L2 (509 x 1280 x 8192: 128 columns in 3 parts are 2 us faster than 256 in 7).  Rows
 // whose pitch is no multiple of 128 bytes make every TMA row touch two L2 lines: `skew` more per K block.  A tile
-// cannot take less than its epilogue, `epi`, where K is short.  Whole waves of wide units take 0.94 of single tiles.
-// The widths the plan picks are on average 0.3 % slower than the best one of each shape, at worst 5 % (2992 x 6224 x
-// 704: 27.6 us at 192 columns, 26.3 at 256).
+// cannot take less than its epilogue, `epi`, where K is short (244 x 1024 x 640: 6.6 us at 128 columns, 7.5 at 192).
+// Whole waves of wide units take 0.94 of single tiles.  The widths the plan picks are on average 0.3 % slower than the best
+// one of each shape, at worst 5 % (2992 x 6224 x 704: 27.6 us at 192 columns, 26.3 at 256).
 // Examples, fp8, with the figures of before (fitted in short bursts) and now: 4096 x 3584 x 8192 103 -> 97 us (192 -> 256
 // columns), 16384 x 3584 x 8192 386 -> 362, 1024 x 8192 x 8192 65 -> 61; bf16 2992 x 6224 x 704 29.4 -> 27.6.
 MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int block_n, int num_sms, int max_splits) {
   struct Width { int bn; double t1, t2, skew, epi; };               // microseconds
-  constexpr Width kBf16[] = {{256, 0.29, 0.15, 0.03, 3.0}, {192, 0.218, 0.135, 0.03, 1.5}, {128, 0.135, 0.12, 0.04, 2.3}};
+  constexpr Width kBf16[] = {{256, 0.29, 0.15, 0.03, 3.2}, {192, 0.218, 0.135, 0.03, 2.6}, {128, 0.135, 0.12, 0.04, 2.3}};
   constexpr Width kFp8[] = {{256, 0.29, 0.135, 0.04, 2.7}, {192, 0.225, 0.13, 0.065, 3.0}, {128, 0.125, 0.13, 0.08, 2.0}};
   const Width(&widths)[3] = elem_bytes == 1 ? kFp8 : kBf16;
   const int pairs = num_sms < 4 ? 1 : num_sms / 2, rows = (M + 2 * kBM - 1) / (2 * kBM);
