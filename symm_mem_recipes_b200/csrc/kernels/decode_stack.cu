@@ -19,7 +19,7 @@
 //     the splits over (sequence, query head).  A layer has eight such round trips over the whole grid: six counters,
 //     and twice, before a norm, the exchange of the sums of squares.
 // The CTAs wait for one another, so the launch is cooperative.  Every wait is bounded.
-// Two layers of that share, against the five kernels: batch 1 at position 3000 133 -> 105 us, batch 16 at 6500 172 -> 145
+// Two layers of that share, against the five kernels: batch 1 at position 3000 133 -> 105 us, batch 16 at 6500 172 -> 139
 // us.  Their weights and caches at the measured copy rate take 66 and 82.
 // Of the 48 us a layer takes at batch 1 about 14 are attention with its meeting points, 12 the other meeting points
 // and first loads of x, the rest is the weight stream.
