@@ -299,8 +299,9 @@ c10::optional<torch::Tensor> matmul_local(const torch::Tensor& a, const torch::T
   args.panel_w = panel_w;
   args.overlap = true;
   const MatmulPlan plan = plan_matmul((int)M, (int)N, (int)K, args.elem_bytes, epilogue, block_n, args.num_sms,
-                                      split_k ? max_splits : 1);
+                                      split_k ? max_splits : 1, residual.has_value());
   args.block_n = plan.block_n;
+  args.wide_units = plan.wide_units;
   torch::Tensor scratch;
   if (plan.tail_bytes > 0) {
     scratch = new_tensor({(int64_t)plan.tail_bytes}, torch::kUInt8, dev);
@@ -712,6 +713,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("matmul_local", &matmul_local, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("epilogue"), py::arg("residual"),
         py::arg("block_n"), py::arg("num_sms"), py::arg("split_k"), py::arg("panel_w"), py::arg("timeout_ns"),
         py::arg("max_splits") = 0);
+
+  // (tile width, K parts of a tail tile, units of two tiles) of matmul_local's GEMM
+  m.def("matmul_plan", [](int M, int N, int K, int elem_bytes, int epilogue, int block_n, int num_sms, int max_splits, bool residual) {
+    const MatmulPlan p = plan_matmul(M, N, K, elem_bytes, epilogue, block_n, num_sms, max_splits, residual);
+    return py::make_tuple(p.block_n, p.tail_splits, p.wide_units);
+  }, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("elem_bytes") = 2, py::arg("epilogue") = 0, py::arg("block_n") = 0,
+     py::arg("num_sms") = 148, py::arg("max_splits") = 0, py::arg("residual") = false);
 
   m.def("gemm_kernels", &gemm_kernels, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("elem_bytes"), py::arg("num_sms"),
         py::arg("gather"));

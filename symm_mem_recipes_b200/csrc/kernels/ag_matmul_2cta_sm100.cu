@@ -706,18 +706,21 @@ int plan_wide_units(int rows, int cols, int pairs, int K, int elem_bytes, bool r
 // and a pass of the parts through L2 (509 x 1280 x 8192: 128 columns in 3 parts are 2 us faster than 256 in 7).  Rows
 // whose pitch is no multiple of 128 bytes make every TMA row touch two L2 lines: `skew` more per K block.  A tile
 // cannot take less than its epilogue, `epi`, where K is short (244 x 1024 x 640: 6.6 us at 128 columns, 7.5 at 192).
-// Whole waves of wide units take 0.94 of single tiles.  The widths the plan picks are on average 0.3 % slower than the best
+// Where there are units of two tiles and K is 5120 or more, whole waves are priced at 0.94.  All of them, not only those of
+// units: that choice differs in 33 of 120000 random shapes, half of which are faster either way (9750 x 1312 x 5280 124 us, with
+// only the units' waves 116; 16363 x 1296 x 9304 372, 428).  The shorter K that units with a residual take is priced at 1: they save 2 to 3 %
+// there, less than 192 columns do where those fill the waves (1240 x 8192 x 3584 66.5 us, 256 columns 69.6).  The widths the plan picks are on average 0.3 % slower than the best
 // one of each shape, at worst 5 % (2992 x 6224 x 704: 27.6 us at 192 columns, 26.3 at 256).
 // Examples, fp8, with the figures of before (fitted in short bursts) and now: 4096 x 3584 x 8192 103 -> 97 us (192 -> 256
 // columns), 16384 x 3584 x 8192 386 -> 362, 1024 x 8192 x 8192 65 -> 61; bf16 2992 x 6224 x 704 29.4 -> 27.6.
-MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int block_n, int num_sms, int max_splits) {
+MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int block_n, int num_sms, int max_splits, bool residual) {
   struct Width { int bn; double t1, t2, skew, epi; };               // microseconds
   constexpr Width kBf16[] = {{256, 0.29, 0.15, 0.03, 3.2}, {192, 0.218, 0.135, 0.03, 2.6}, {128, 0.135, 0.12, 0.04, 2.3}};
   constexpr Width kFp8[] = {{256, 0.29, 0.135, 0.04, 2.7}, {192, 0.225, 0.13, 0.065, 3.0}, {128, 0.125, 0.13, 0.08, 2.0}};
   const Width(&widths)[3] = elem_bytes == 1 ? kFp8 : kBf16;
   const int pairs = num_sms < 4 ? 1 : num_sms / 2, rows = (M + 2 * kBM - 1) / (2 * kBM);
   const int k_blocks = (K * elem_bytes + 127) / 128;
-  MatmulPlan best{block_n != 0 ? block_n : 256, 1, 0};
+  MatmulPlan best{block_n != 0 ? block_n : 256, 1, 0, 0};
   double best_cost = -1;
   for (const Width& w : widths) {
     // a width the caller (or the SwiGLU epilogue) asks for is taken with the figures of the nearest one
@@ -732,8 +735,8 @@ MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int bl
       return us > w.epi ? us : w.epi;
     };
     const int rem = tiles % pairs;
-    const bool wide = bn == 256 && plan_wide_units(rows, tiles / rows, pairs, K, elem_bytes, false) > 0;
-    double cost = tiles / pairs * wave_us(pairs, 1) * (wide ? 0.94 : 1.0);
+    const int wide_units = bn == 256 ? plan_wide_units(rows, tiles / rows, pairs, K, elem_bytes, residual) : 0;
+    double cost = tiles / pairs * wave_us(pairs, 1) * (wide_units > 0 && K >= 5120 ? 0.94 : 1.0);
     int parts = 1;
     if (rem > 0) {
       double tail = wave_us(rem, 1);
@@ -748,6 +751,7 @@ MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int bl
       best.block_n = bn;
       best.tail_splits = parts;
       best.tail_bytes = parts > 1 ? tail_scratch_bytes(rem, parts, bn) : 0;
+      best.wide_units = wide_units;
     }
   }
   // Gate and up in two halves of B: 112 columns of each, uncut, where that fills the pairs better (K 8192, us): 300 x 7168
@@ -759,13 +763,13 @@ MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int bl
       const double us = k_blocks * (0.254 + (K % kBK != 0 ? 0.03 : 0.0) + 0.143 * n / pairs);
       return us > 4.0 ? us : 4.0;
     };
-    if (tiles / pairs * wave_us(pairs) + (rem > 0 ? wave_us(rem) : 0.0) < 0.97 * best_cost) best = MatmulPlan{224, 1, 0};
+    if (tiles / pairs * wave_us(pairs) + (rem > 0 ? wave_us(rem) : 0.0) < 0.97 * best_cost) best = MatmulPlan{224, 1, 0, 0};
   }
   return best;
 }
 
 int gemm_kernels(int M, int N, int K, int elem_bytes, int num_sms, bool gather) {
-  if (!gather) return plan_matmul(M, N, K, elem_bytes, 0, 0, num_sms, 0).tail_splits > 1 ? 2 : 1;
+  if (!gather) return plan_matmul(M, N, K, elem_bytes, 0, 0, num_sms, 0, false).tail_splits > 1 ? 2 : 1;
   const int tiles = (M + 2 * kBM - 1) / (2 * kBM) * ((N + 255) / 256), pairs = num_sms < 4 ? 1 : num_sms / 2;
   return tail_parts(tiles % pairs, pairs, (K * elem_bytes + 127) / 128, 0) > 1 ? 2 : 1;
 }
@@ -880,8 +884,13 @@ int launch_ag_matmul_2cta(const AgMatmulArgs& a, cudaStream_t stream) {
       if (total_tiles < max_pairs) pairs = rem * splits;
     }
   }
-  if (!comm && bn == 256 && a.trace == nullptr)                    // the timing record is the other kernel's
-    p.wide_units = plan_wide_units((p.n_blocks_m + 1) / 2, p.n_tiles_n, max_pairs, a.K, es, a.residual != nullptr);
+  if (a.wide_units != 0) {
+    // whole waves of them (a second accumulator for each tile of a unit, so 256 columns of bf16); a pair's first work
+    if (comm || fp8 || bn != 256 || a.trace != nullptr || a.wide_units < 0 || a.wide_units % max_pairs != 0 ||
+        a.wide_units > (p.n_blocks_m + 1) / 2 * (p.n_tiles_n / 2))
+      return cudaErrorInvalidValue;
+    p.wide_units = a.wide_units;
+  }
   const int grid = 2 * pairs;
   if (comm) {
     if (a.lead < 0) {

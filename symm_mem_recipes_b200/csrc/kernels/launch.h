@@ -115,15 +115,19 @@ struct AgMatmulArgs {
   // N tiles per column panel of the tile order (0 = the launcher's choice: the widest even split of the
   // N tiles whose rows of B stay in L2)
   int panel_w;
+  // mode 0: units of two neighbouring tiles multiplied at a time, whole waves of them (MatmulPlan::wide_units)
+  int wide_units;
 };
 int launch_ag_matmul_2cta(const AgMatmulArgs& args, cudaStream_t stream);
-// Tile width and split-K tail of a GEMM without a gather (mode 0).  `block_n` / `max_splits`: 0 = the plan's choice.
+// Tile width, split-K tail and units of two tiles of a GEMM without a gather (mode 0).  `block_n` / `max_splits`: 0 = the
+// plan's choice.
 struct MatmulPlan {
   int block_n;
   int tail_splits;        // K parts of a tail tile (1 = no split)
   size_t tail_bytes;      // scratch for them
+  int wide_units;         // units of two neighbouring tiles at the front of the schedule (matmul_wide.cuh), 0 = none
 };
-MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int block_n, int num_sms, int max_splits);
+MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int block_n, int num_sms, int max_splits, bool residual);
 // Kernels that such a GEMM launches (bf16 or fp8, planned width; with `gather` the width and cut of the fused kernel): 1, or
 // 2 where tiles are cut and their parts added up.
 int gemm_kernels(int M, int N, int K, int elem_bytes, int num_sms, bool gather);
