@@ -238,11 +238,19 @@ py::tuple host_all_reduce(const std::shared_ptr<HostSymmAllocation>& a, int64_t 
   return py::make_tuple(code, rank, 0, peer, (int)kWhereTwoShotExit, 0);
 }
 
+// The per-CTA timing record that a GEMM on `num_sms` SMs fills.
+uint64_t* trace_words(const torch::Tensor& trace, int dev, int num_sms) {
+  TORCH_CHECK(trace.is_cuda() && trace.get_device() == dev && trace.is_contiguous() && trace.scalar_type() == torch::kInt64 &&
+              trace.numel() >= (int64_t)num_sms * 12, "trace must be a contiguous int64 CUDA tensor of num_sms x 12 words");
+  return reinterpret_cast<uint64_t*>(trace.data_ptr());
+}
+
 // The GEMM alone (no gather): checks, output, scratch and launch in one call.  Nothing when the operands are not what
 // the kernel takes: the caller's full path then says why.  epilogue: see AgMatmulArgs.
 c10::optional<torch::Tensor> matmul_local(const torch::Tensor& a, const torch::Tensor& b, const c10::optional<torch::Tensor>& out,
                                         int epilogue, const c10::optional<torch::Tensor>& residual, int block_n, int num_sms,
-                                        bool split_k, int panel_w, uint64_t timeout_ns, int max_splits) {
+                                        bool split_k, int panel_w, uint64_t timeout_ns, int max_splits,
+                                        const c10::optional<torch::Tensor>& trace = c10::nullopt) {
   const auto dtype = a.scalar_type();
   const bool fp8 = dtype == at::kFloat8_e4m3fn;
   if ((!fp8 && dtype != torch::kBFloat16) || !a.is_cuda()) return c10::nullopt;
@@ -266,10 +274,11 @@ c10::optional<torch::Tensor> matmul_local(const torch::Tensor& a, const torch::T
   // Few rows are a matter of streaming the weights.  Up to 64 of them the skinny kernel is the faster one (64 x 7168 x
   // 8192 with SwiGLU 36 -> 25 us, 64 x 1280 x 8192 14.1 -> 10.1, 32 x 8192 x 1024 10.2 -> 7.4); up to 128 where the
   // GEMM's narrowest tiles fill less than half of the SM pairs (128 x 7168 x 8192 with SwiGLU 37 -> 29; 128 x 8192 x
-  // 1024, 64 tiles, 9.0 against 12.1).  A caller who sets the GEMM's parameters gets the GEMM.
+  // 1024, 64 tiles, 9.0 against 12.1).  A caller who sets the GEMM's parameters or asks for its record gets the GEMM.
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   const bool few_tiles = (N + (swiglu ? 255 : 127)) / (swiglu ? 256 : 128) * 4 <= sms;
-  if (!fp8 && (M <= 64 || (M <= 128 && few_tiles)) && block_n == 0 && num_sms == 0 && max_splits == 0 && split_k) {
+  if (!fp8 && (M <= 64 || (M <= 128 && few_tiles)) && block_n == 0 && num_sms == 0 && max_splits == 0 && split_k &&
+      !trace.has_value()) {
     GemvLocalArgs skinny{};
     skinny.x = a.data_ptr();
     skinny.w = b.data_ptr();
@@ -309,6 +318,7 @@ c10::optional<torch::Tensor> matmul_local(const torch::Tensor& a, const torch::T
     args.tail_scratch_bytes = plan.tail_bytes;
     args.tail_splits = plan.tail_splits;
   }
+  if (trace.has_value()) args.trace = trace_words(*trace, dev, args.num_sms);
   rt_check(launch_ag_matmul_2cta(args, stream), "matmul");
   return c;
 }
@@ -696,12 +706,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     args.push_plain_stores = push_plain_stores ? 1 : 0;
     args.push_pieces = push_pieces;
     args.panel_w = panel_w;
-    if (trace.has_value()) {
-      TORCH_CHECK(trace->is_cuda() && trace->get_device() == dev && trace->is_contiguous() &&
-                  trace->scalar_type() == torch::kInt64 && trace->numel() >= (int64_t)num_sms * 12,
-                  "trace must be a contiguous int64 CUDA tensor of num_sms x 12 words");
-      args.trace = reinterpret_cast<uint64_t*>(trace->data_ptr());
-    }
+    if (trace.has_value()) args.trace = trace_words(*trace, dev, num_sms);
     rt_check(launch_ag_matmul_2cta(args, stream), "ag_matmul");
   }, py::arg("a"), py::arg("b"), py::arg("c"), py::arg("mode"), py::arg("aout_alloc"), py::arg("aout_offset"),
      py::arg("a_out"), py::arg("block_n"), py::arg("num_sms"), py::arg("timeout_ns"),
@@ -712,7 +717,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
 
   m.def("matmul_local", &matmul_local, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("epilogue"), py::arg("residual"),
         py::arg("block_n"), py::arg("num_sms"), py::arg("split_k"), py::arg("panel_w"), py::arg("timeout_ns"),
-        py::arg("max_splits") = 0);
+        py::arg("max_splits") = 0, py::arg("trace") = py::none());
 
   // (tile width, K parts of a tail tile, units of two tiles) of matmul_local's GEMM
   m.def("matmul_plan", [](int M, int N, int K, int elem_bytes, int epilogue, int block_n, int num_sms, int max_splits, bool residual) {

@@ -653,7 +653,7 @@ int launch_pair_variant(const CUtensorMap& ta_shard, const CUtensorMap& ta_out, 
 template <bool kSwiGlu, bool kResidual>
 int launch_wide(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tr,
                 const AgMatmulParams& p, int grid, bool overlap, cudaStream_t stream) {
-  auto kern = wide::matmul_wide_kernel<kSwiGlu, kResidual>;
+  auto kern = p.trace != nullptr ? wide::matmul_wide_kernel<kSwiGlu, kResidual, true> : wide::matmul_wide_kernel<kSwiGlu, kResidual, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wide::kSmemBytes);
   if (e != cudaSuccess) return (int)e;
   cudaLaunchAttribute attr[1];
@@ -886,7 +886,7 @@ int launch_ag_matmul_2cta(const AgMatmulArgs& a, cudaStream_t stream) {
   }
   if (a.wide_units != 0) {
     // whole waves of them (a second accumulator for each tile of a unit, so 256 columns of bf16); a pair's first work
-    if (comm || fp8 || bn != 256 || a.trace != nullptr || a.wide_units < 0 || a.wide_units % max_pairs != 0 ||
+    if (comm || fp8 || bn != 256 || a.wide_units < 0 || a.wide_units % max_pairs != 0 ||
         a.wide_units > (p.n_blocks_m + 1) / 2 * (p.n_tiles_n / 2))
       return cudaErrorInvalidValue;
     p.wide_units = a.wide_units;

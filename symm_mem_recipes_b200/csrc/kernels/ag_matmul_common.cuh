@@ -70,17 +70,17 @@ struct AgMatmulParams {
   // rows of B that tile ni takes: CTA c of the pair loads BN / 2 of them from ni * b_step + c * b_pair
   int b_step, b_pair;
   const __nv_bfloat16* residual;   // [M, N] added to the rounded product (plain bf16 epilogue), or nullptr
-  // optional per-CTA %globaltimer record (2-CTA kernel), kTraceSlots words per CTA; see ag_trace::
+  // optional per-CTA %globaltimer record, kTraceSlots words per CTA; see ag_trace::
   uint64_t* trace;
 };
 
-// Per-CTA timing record of the CTA-pair kernel (nanoseconds of %globaltimer).  Absolute stamps
+// Per-CTA timing record of the CTA-pair kernels, one tile or two at a time (nanoseconds of %globaltimer).  Absolute stamps
 // and accumulated waiting times of each warp role, enough to tell where a fused call loses time
 // against the GEMM alone.  Upstream has no counterpart (it reads kernel times from the profiler,
 // symm_mem_recipes/utils.py:74-82).
 namespace ag_trace {
 constexpr int kStart = 0;          // stamp: kernel entry
-constexpr int kEntered = 1;        // stamp: entry barrier of the push mode passed
+constexpr int kEntered = 1;        // stamp: epilogue warps begin (push mode: entry barrier passed)
 constexpr int kFlagWait = 2;       // producer: total wait for arrival flags of remote blocks
 constexpr int kPush = 3;           // epilogue warps: total time inside push_pieces
 constexpr int kAccWait = 4;        // epilogue warps: total wait for a complete accumulator

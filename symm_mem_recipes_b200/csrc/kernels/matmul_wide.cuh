@@ -58,8 +58,9 @@ __device__ __forceinline__ uint32_t chunk_at(uint32_t first, int i) {
   return c >= (uint32_t)kChunks ? c - kChunks : c;
 }
 
-// kSwiGlu, kResidual: as in ag_matmul_2cta_kernel.
-template <bool kSwiGlu, bool kResidual>
+// kSwiGlu, kResidual: as in ag_matmul_2cta_kernel.  kTraced: an instantiation of its own fills p.trace (ag_trace::), so that
+// the waits of the others are not timed.
+template <bool kSwiGlu, bool kResidual, bool kTraced>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 matmul_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                    const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_residual, const AgMatmulParams p) {
@@ -107,6 +108,19 @@ matmul_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   const int n_pair_rows = (p.n_blocks_m + 1) >> 1, total_tiles = n_pair_rows * p.n_tiles_n;
   const int k_blocks = (p.K + kBK - 1) / kBK;
   bool failed = false;
+  [[maybe_unused]] uint64_t* trc = kTraced ? p.trace + (size_t)blockIdx.x * ag_trace::kTraceSlots : nullptr;
+  if (kTraced && threadIdx.x == 0) trc[ag_trace::kStart] = globaltimer_ns();
+  // a wait on a barrier, with its time added to `total`
+  auto timed_wait = [&p](uint64_t* bar, uint32_t parity, [[maybe_unused]] uint64_t& total) {
+    if constexpr (kTraced) {
+      const uint64_t t0 = globaltimer_ns();
+      const bool ok = mbar_wait(bar, parity, p.timeout_ns);
+      total += globaltimer_ns() - t0;
+      return ok;
+    } else {
+      return mbar_wait(bar, parity, p.timeout_ns);
+    }
+  };
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
@@ -114,6 +128,7 @@ matmul_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
       Cursor at, oldest;                                         // oldest: the next K block to come back
       int free = kChunks, wide_left = p.wide_units / n_pairs * k_blocks;   // K blocks of three chunks not yet back
       WideWork w;
+      uint64_t t_stage = 0;
       pdl_wait();
       for (int wi = 0; !failed && wide_work(p, pair, n_pairs, total_tiles, k_blocks, wi, w); ++wi) {
         int prow, ni;
@@ -123,7 +138,7 @@ matmul_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
 #pragma unroll 1
         for (int kb = w.kb0; kb < w.kb1; ++kb) {
           while (free < need) {
-            if (!mbar_wait(&empty_bar[oldest.bar], oldest.phase, p.timeout_ns)) {
+            if (!timed_wait(&empty_bar[oldest.bar], oldest.phase, t_stage)) {
               report_status(p.status, kTimeoutMbarrier, p.rank, blockIdx.x, oldest.bar, kWhereGemmEmpty);
               failed = true;
               break;
@@ -144,6 +159,7 @@ matmul_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           at.next(need);
         }
       }
+      if constexpr (kTraced) trc[ag_trace::kStageWait] = t_stage;
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
@@ -153,8 +169,9 @@ matmul_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
       Cursor at;
       uint32_t acc = 0, acc_phase = 0;
       WideWork w;
+      uint64_t t_operand = 0, t_tmem = 0;
       auto wait_operands = [&](const Cursor& c) {
-        if (!mbar_wait(&full_bar[c.bar], c.phase, p.timeout_ns)) {
+        if (!timed_wait(&full_bar[c.bar], c.phase, t_operand)) {
           report_status(p.status, kTimeoutMbarrier, p.rank, blockIdx.x, c.bar, kWhereGemmFull);
           failed = true;
           return false;
@@ -163,7 +180,7 @@ matmul_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         return true;
       };
       auto wait_accumulator = [&](uint32_t which, uint32_t parity) {
-        if (!mbar_wait(&tmem_empty[which], parity, p.timeout_ns)) {
+        if (!timed_wait(&tmem_empty[which], parity, t_tmem)) {
           report_status(p.status, kTimeoutMbarrier, p.rank, blockIdx.x, which, kWhereGemmTmemEmpty);
           failed = true;
           return false;
@@ -230,6 +247,10 @@ matmul_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         umma_commit_pair(&tmem_full[acc ^ 1]);
         acc_phase ^= 1;
       }
+      if constexpr (kTraced) {
+        trc[ag_trace::kTmemWait] = t_tmem;
+        trc[ag_trace::kOperandWait] = t_operand;
+      }
     }
   } else {
     // ---------------- epilogue (eight warps of both CTAs) ----------------
@@ -245,6 +266,10 @@ matmul_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     uint32_t acc = 0, acc_phase = 0;
     [[maybe_unused]] uint32_t residual_phase = 0;
     pdl_wait();
+    const bool records = kTraced && warp == 2 && lane == 0;
+    uint64_t t_acc = 0;
+    [[maybe_unused]] uint64_t n_tiles = 0;
+    if (records) trc[ag_trace::kEntered] = globaltimer_ns();
     WideWork w;
     w.halves = 1;
     for (int wi = 0, half = 1;; ++half) {
@@ -271,11 +296,12 @@ matmul_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             }
         }
       }
-      if (!mbar_wait(&tmem_full[acc], acc_phase, p.timeout_ns)) {
+      if (!timed_wait(&tmem_full[acc], acc_phase, t_acc)) {
         if (lane == 0) report_status(p.status, kTimeoutMbarrier, p.rank, blockIdx.x, acc, kWhereGemmTmemFull);
         failed = true;
         break;
       }
+      if constexpr (kTraced) ++n_tiles;
       tcgen05_fence_after_thread_sync();
       const uint32_t taddr = tmem_base + acc * 256u + ((uint32_t)(quarter * 32) << 16);
       auto release_accumulator = [&] {
@@ -358,6 +384,11 @@ matmul_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
       if (failed) break;
     }
     if (lane == 0) bulk_wait_group<0>();                         // C is written before the kernel ends
+    if (records) {
+      trc[ag_trace::kAccWait] = t_acc;
+      trc[ag_trace::kTiles] = n_tiles;
+      trc[ag_trace::kTilesDone] = trc[ag_trace::kEnd] = globaltimer_ns();
+    }
   }
 
   // ---------------- teardown ----------------

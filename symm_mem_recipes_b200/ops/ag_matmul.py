@@ -165,10 +165,11 @@ def _epilogue_code(epilogue, dtype: torch.dtype, N: int, config: "AgMatmulConfig
     return code
 
 
-def _matmul_local(a, b, c_out, config: "AgMatmulConfig", epilogue: Optional[str]) -> Optional[torch.Tensor]:
+def _matmul_local(a, b, c_out, config: "AgMatmulConfig", epilogue: Optional[str],
+                  trace: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
     """The GEMM without a gather in one native call, or None when the operands are not for it."""
     return C.matmul_local(a, b, c_out, _EPILOGUES.get(epilogue, -1), None, config.block_n, config.num_sms,
-                          config.split_k_tail, config.panel_w, config.timeout_ms * 1_000_000)
+                          config.split_k_tail, config.panel_w, config.timeout_ms * 1_000_000, 0, trace)
 
 
 @traced("smr.matmul")
@@ -176,9 +177,11 @@ def matmul(a: torch.Tensor, b: torch.Tensor, c_out: Optional[torch.Tensor] = Non
            config: AgMatmulConfig = DEFAULT_CONFIG, epilogue: Optional[str] = None,
            trace: Optional[torch.Tensor] = None) -> torch.Tensor:
     """C[M, N] = A[M, K] @ B[N, K]^T on the tcgen05 kernel, no communication.
-    `epilogue="swiglu"`: see `all_gather_matmul`."""
-    if a.is_cuda and trace is None:
-        c = _matmul_local(a, b, c_out, config, epilogue)
+    `epilogue="swiglu"`: see `all_gather_matmul`.  `trace`: as there, the record of the GEMM kernel that the call takes
+    without it; only a few rows (up to 64, or 128 of a small N), which go to the weight-streaming kernel otherwise, take
+    the GEMM for the sake of the record.  The kernel that adds up a cut tail is not in it."""
+    if a.is_cuda:
+        c = _matmul_local(a, b, c_out, config, epilogue, trace)
         if c is not None:
             return c
     _check_2d("a", a)
@@ -253,7 +256,7 @@ def all_gather_matmul(a_shard: torch.Tensor, b: torch.Tensor, a_out: Optional[to
     accumulators before they leave the SM (bf16, push gather or no gather).
 
     `trace`: an int64 CUDA tensor [num_sms, 12] that receives the per-CTA timing
-    record of the CTA-pair kernel (`TRACE_FIELDS`; push gather or no gather).
+    record of the GEMM kernel (`TRACE_FIELDS`; push gather or no gather).
     """
     if a_shard.is_cuda and trace is None and not mm_only and \
             (not dist.is_initialized() or dist.get_world_size(group) == 1):

@@ -115,19 +115,29 @@ def test_cut_call_while_another_thread_captures():
 def test_calls_in_a_row_and_replayed(traced):
     """Both bindings, again and again on one scratch, eagerly and from a graph."""
     import symm_mem_recipes_b200 as smr
+    from symm_mem_recipes_b200._ext import C
     from symm_mem_recipes_b200.parallel import symm_mem
 
     a, b, want = _operands()
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    trace = torch.zeros(sms, 12, dtype=torch.int64, device="cuda") if traced else None   # a record takes the other binding
+    trace = torch.zeros(sms, 12, dtype=torch.int64, device="cuda") if traced else None
+    scratch = torch.empty(sms * 128 * 256 * 4, dtype=torch.uint8, device="cuda")
+
+    def call():
+        if not traced:
+            return smr.matmul(a, b)
+        c = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")          # the binding of the gather, with a record
+        C.ag_matmul(a, b, c, 0, None, 0, None, 128, sms, 2_000_000_000, scratch, 0, trace)
+        return c
+
     graph = torch.cuda.CUDAGraph()
-    smr.matmul(a, b, trace=trace)
+    call()
     with torch.cuda.graph(graph):
-        c = smr.matmul(a, b, trace=trace)
+        c = call()
     for _ in range(3):
         c.zero_()
         graph.replay()
-        assert _matches(c, want) and _matches(smr.matmul(a, b, trace=trace), want)
+        assert _matches(c, want) and _matches(call(), want)
     symm_mem.check_status("cuda")
 
 

@@ -107,6 +107,35 @@ def test_two_tiles_at_a_time(M, N, K, sms, splits):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,epilogue", [
+    (509, 1280, 8192, None),          # narrow tiles, all cut along K
+    (1240, 8192, 3584, None),         # 192 columns, three rounds
+    (2048, 5120, 5120, None), (2048, 5120, 5120, "swiglu"), (1100, 8200, 5120, None),   # two tiles at a time
+])
+def test_a_record_is_of_the_kernel_that_runs(M, N, K, epilogue):
+    """The CTAs and pieces of work in a timing record are those of the plan, and the result is the same to the bit."""
+    import symm_mem_recipes_b200 as smr
+    from symm_mem_recipes_b200._ext import C
+    from symm_mem_recipes_b200.ops.ag_matmul import TRACE_FIELDS
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    pairs = sms // 2
+    width, parts, units = C.matmul_plan(M, N, K, epilogue=1 if epilogue else 0, num_sms=sms)
+    assert (units > 0) == (K == 5120)
+    a, b = _operands(M, N, K)
+    trace = torch.zeros(sms, len(TRACE_FIELDS), dtype=torch.int64, device="cuda")
+    got = smr.matmul(a, b, epilogue=epilogue, trace=trace)
+    assert torch.equal(got, smr.matmul(a, b, epilogue=epilogue))
+    tiles = -(-M // 256) * -(-N // width)
+    cut = tiles % pairs if parts > 1 else 0
+    record = dict(zip(TRACE_FIELDS, trace.cpu().unbind(1)))
+    assert int((record["start"] > 0).sum()) == 2 * (tiles * parts if cut == tiles else min(tiles, pairs))
+    assert int(record["tiles"].sum()) == 2 * (tiles - cut + cut * parts)
+    ran = record["start"] > 0
+    assert bool((record["end"] >= record["tiles_done"])[ran].all()) and bool((record["tiles_done"] > record["start"])[ran].all())
+
+
+@pytest.mark.gpu
 def test_split_calls_on_several_streams():
     """Calls whose tiles are cut along K share neither scratch nor counters across streams."""
     from symm_mem_recipes_b200.parallel import symm_mem
