@@ -740,9 +740,10 @@ MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int bl
     int parts = 1;
     if (rem > 0) {
       double tail = wave_us(rem, 1);
-      for (int most = tail_parts(rem, pairs, k_blocks, max_splits); most >= 2; --most) {
+      for (int most = tail_parts(rem, pairs, k_blocks, max_splits < 0 ? -max_splits : max_splits); most >= 2; --most) {
         const double cut = wave_us(rem, most) + 2.0 + 0.25e-6 * tail_scratch_bytes(rem, most, bn);
-        if (cut < tail) { tail = cut; parts = most; }
+        if (cut < tail || max_splits < 0) { tail = cut; parts = most; }
+        if (max_splits < 0) break;
       }
       cost += tail;
     }
@@ -757,7 +758,7 @@ MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int bl
   // Gate and up in two halves of B: 112 columns of each, uncut, where that fills the pairs better (K 8192, us): 300 x 7168
   // 50 -> 45, 509 x 7168 57 -> 53 (64 tiles on 74 pairs instead of 56), 509 x 14336 106 -> 103, 900 x 7168 113 -> 107, 1500 x
   // 7168 150 -> 146; 385 x 4000 x 2048 24.5 -> 21.1.  Its rows of C are 224 bytes, so the lanes store them themselves.
-  if (epilogue == 2 && block_n == 0) {
+  if (epilogue == 2 && block_n == 0 && max_splits >= 0) {
     const int tiles = rows * ((N / 2 + 111) / 112), rem = tiles % pairs;
     auto wave_us = [&](int n) {
       const double us = k_blocks * (0.254 + (K % kBK != 0 ? 0.03 : 0.0) + 0.143 * n / pairs);

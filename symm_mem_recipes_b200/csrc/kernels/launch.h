@@ -120,7 +120,7 @@ struct AgMatmulArgs {
 };
 int launch_ag_matmul_2cta(const AgMatmulArgs& args, cudaStream_t stream);
 // Tile width, split-K tail and units of two tiles of a GEMM without a gather (mode 0).  `block_n` / `max_splits`: 0 = the
-// plan's choice.
+// plan's choice; max_splits > 0: parts at most; < 0: so many parts wherever the tail can be cut, whatever the model says.
 struct MatmulPlan {
   int block_n;
   int tail_splits;        // K parts of a tail tile (1 = no split)

@@ -163,14 +163,15 @@ def test_cut_calls_of_two_priorities_at_once():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("m,n,k,block_n,sms,epilogue,dtype", [
-    (129, 136, 1024, 128, 0, 0, torch.bfloat16), (300, 1000, 2048, 192, 24, 0, torch.bfloat16),
+    (129, 136, 1024, 128, 0, 0, torch.bfloat16), (300, 1000, 2048, 192, 0, 0, torch.bfloat16),
     (257, 520, 4096, 256, 0, 0, torch.bfloat16), (130, 464, 1160, 224, 0, 0, torch.bfloat16),
-    (300, 2000, 1024, 0, 0, 2, torch.bfloat16), (300, 768, 1024, 0, 0, 1, torch.bfloat16),
-    (129, 144, 4096, 128, 0, 0, torch.float8_e4m3fn), (300, 976, 2064, 192, 24, 0, torch.float8_e4m3fn),
+    (300, 2000, 1024, 256, 0, 2, torch.bfloat16), (300, 768, 1024, 0, 0, 1, torch.bfloat16),
+    (129, 144, 4096, 128, 0, 0, torch.float8_e4m3fn), (300, 976, 2064, 192, 0, 0, torch.float8_e4m3fn),
     (600, 464, 4096, 224, 0, 0, torch.float8_e4m3fn)])
 @pytest.mark.parametrize("splits", [2, 3, 8])
 def test_cut_tiles_equal_uncut_ones(m, n, k, block_n, sms, epilogue, dtype, splits):
-    """Every width, end and type of the cut path at ragged edges.  The same products in another order of fp32 sums: a
+    """Every width, end and type of the cut path at ragged edges, cut into as many parts as asked for or as there are
+    pairs (K 1160 in eight: the last part is empty).  The same products in another order of fp32 sums: a
     result may round to the neighbouring bf16 (2^-8 of it) or e4m3 (2^-3) number, and beside that differ by what
     cancels, k * 2^-24 of a sum of k terms of 0.05."""
     from symm_mem_recipes_b200._ext import C
@@ -180,15 +181,27 @@ def test_cut_tiles_equal_uncut_ones(m, n, k, block_n, sms, epilogue, dtype, spli
     gen = torch.Generator(device="cuda").manual_seed(m + n + k)
     a = (torch.randn(m, k, generator=gen, device="cuda") * 0.5).to(dtype)
     b = (torch.randn(n, k, generator=gen, device="cuda") * 0.1).to(dtype)
-    n_out = n // 2 if epilogue else n
-    if dtype == torch.bfloat16:
-        c, intact = guarded_empty((m, n_out), dtype, "cuda")
-    else:
-        c, intact = torch.empty(m, n_out, dtype=dtype, device="cuda"), lambda: True
-    whole = C.matmul_local(a, b, None, epilogue, None, block_n, sms, False, 0, 2_000_000_000, 1)
-    assert C.matmul_local(a, b, c, epilogue, None, block_n, sms, True, 0, 2_000_000_000, splits) is not None
-    symm_mem.check_status("cuda")
-    ulp = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -3
-    x, y = c.float(), whole.float()
-    assert bool(((x - y).abs() <= torch.maximum(x.abs(), y.abs()) * ulp + 0.05 * k * 2.0 ** -22).all())
-    assert intact(), "the kernel stored outside its output"
+    n_out, es = n // 2 if epilogue else n, a.element_size()
+    width = block_n or 256
+    tiles, pairs = -(-m // 256) * -(-n_out // (width // 2 if epilogue else width)), torch.cuda.get_device_properties(0).multi_processor_count // 2
+    parts = min(splits, pairs // tiles)            # every tile is cut: they are fewer than half of the pairs
+    assert C.matmul_plan(m, n, k, es, epilogue, block_n, 2 * pairs, -splits) == (width, parts, 0) and parts >= 2
+    residuals = [None]
+    if dtype == torch.bfloat16 and not epilogue and block_n != 224:
+        residuals.append(torch.randn(m, n, generator=gen, device="cuda").to(dtype))
+    for residual in residuals:
+        if dtype == torch.bfloat16:
+            c, intact = guarded_empty((m, n_out), dtype, "cuda")
+            c.fill_(float("nan"))
+        else:
+            c, intact = torch.empty(m, n_out, dtype=dtype, device="cuda"), lambda: True
+        whole = C.matmul_local(a, b, None, epilogue, residual, block_n, sms, False, 0, 2_000_000_000, 1)
+        assert C.matmul_local(a, b, c, epilogue, residual, block_n, sms, True, 0, 2_000_000_000, -splits) is not None
+        symm_mem.check_status("cuda")
+        ulp = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -3
+        x, y = c.float(), whole.float()
+        product = torch.maximum(x.abs(), y.abs())
+        if residual is not None:                   # rounded before the residual is added, and once more after
+            product = torch.maximum(product, torch.maximum((x - residual.float()).abs(), (y - residual.float()).abs())) * 2
+        assert bool(((x - y).abs() <= product * ulp + 0.05 * k * 2.0 ** -22).all())
+        assert intact(), "the kernel stored outside its output"
