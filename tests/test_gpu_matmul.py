@@ -80,7 +80,7 @@ def test_matmul_split_k_tail(shape, num_sms):
     outs = []
     for split in (True, False):
         c = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
-        for _ in range(2):       # second call reuses the scratch and its counters
+        for _ in range(2):       # second call may find the scratch of the first
             matmul(a, b, c, AgMatmulConfig(num_sms=num_sms, split_k_tail=split, timeout_ms=2000))
         symm_mem.check_status("cuda")
         outs.append(c)

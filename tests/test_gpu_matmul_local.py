@@ -31,7 +31,7 @@ def test_tiles_splits_and_residual(M, N, K, block_n, sms):
         if r is not None and block_n == 224:
             continue                                     # the launcher refuses it: no whole boxes of C
         c, intact = guarded_empty((M, N), torch.bfloat16, "cuda")
-        for _ in range(2):                               # the second call finds the counters as the first left them
+        for _ in range(2):                               # the second call finds the scratch as the first left it
             c.fill_(float("nan"))
             assert _run(a, b, c, residual=r, block_n=block_n, sms=sms) is not None
         symm_mem.check_status("cuda")
@@ -76,14 +76,16 @@ def test_swiglu_in_narrower_tiles(M, F, K):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("M,N,K,sms,splits", [
-    (256, 1024, 5120, 4, 0),          # one wave of units, nothing left
-    (511, 1280, 5128, 8, 0),          # a ragged row, five columns (too few for an odd number: one tile at a time)
-    (700, 2312, 5184, 8, 0),          # ten columns, the last one 8 wide, tiles left over
-    (1290, 2304, 5120, 8, 2),         # nine columns: the odd one comes last, and the tail is cut
-    (769, 1040, 6200, 4, 1),          # no cut; three rows of tiles, the last with one row of C
+@pytest.mark.parametrize("M,N,K,sms,units,left", [
+    (256, 1024, 5120, 4, 2, 0),       # one wave of units, nothing left
+    (511, 1520, 5128, 8, 4, 4),       # a ragged row and column; a wave of single tiles after the units
+    (700, 2320, 5184, 8, 12, 6),      # three rows of ten columns, the last one 16 wide
+    (1290, 2304, 5120, 8, 24, 6),     # nine columns: the odd one comes last, and its last two tiles are the tail
+    (769, 1296, 6200, 4, 12, 0),      # the last row of tiles with one row of C, the last column 16 wide
 ])
-def test_two_tiles_at_a_time(M, N, K, sms, splits):
+def test_two_tiles_at_a_time(M, N, K, sms, units, left):
+    """Uncut, the same products in the same order as one tile at a time: the same bits.  And with the tail cut in two."""
+    from symm_mem_recipes_b200._ext import C
     from symm_mem_recipes_b200.parallel import symm_mem
     from symm_mem_recipes_b200.utils.testing import guarded_empty
 
@@ -91,19 +93,23 @@ def test_two_tiles_at_a_time(M, N, K, sms, splits):
     ref = a.float() @ b.float().t()
     res = (torch.randn(M, N, device="cuda")).to(torch.bfloat16)
     gate, up = ref.split(N // 2, dim=1)
-    forms = [(0, None, ref), (0, res, ref + res.float())]
-    if N % 16 == 0:
-        forms.append((2, None, torch.nn.functional.silu(gate) * up))
-    for epilogue, residual, want in forms:
-        c, intact = guarded_empty(tuple(want.shape), torch.bfloat16, "cuda")
-        c.fill_(float("nan"))
-        assert _run(a, b, c, epilogue=epilogue, residual=residual, block_n=256, sms=sms, splits=splits) is not None
-        symm_mem.check_status("cuda")
-        # a bf16 rounding is 2^-9 of the value (two with a residual); the sums of 5000 products of 0.05 differ by 1e-4
-        assert bool(((c.float() - want).abs() <= want.abs() * 2.0 ** -6 + 2e-2).all())
-        assert intact(), "the kernel stored outside its output"
-        if splits == 1:                                  # same products in the same order: the same bits
-            assert torch.equal(c, _run(a, b, epilogue=epilogue, residual=residual, block_n=256, sms=64, splits=1))
+    tail = left % (sms // 2)
+    for epilogue, residual, want in [(0, None, ref), (0, res, ref + res.float()), (2, None, torch.nn.functional.silu(gate) * up)]:
+        def plan(sms, splits):
+            return C.matmul_plan(M, N, K, 2, epilogue, 256, sms, splits, residual is not None)
+
+        one = _run(a, b, epilogue=epilogue, residual=residual, block_n=256, sms=64, splits=1)
+        assert plan(64, 1) == (256, 1, 0)                # 32 pairs: no whole wave of units
+        for splits in (1, -2):
+            c, intact = guarded_empty(tuple(want.shape), torch.bfloat16, "cuda")
+            c.fill_(float("nan"))
+            assert plan(sms, splits) == (256, 2 if splits < 0 and tail else 1, units)
+            assert _run(a, b, c, epilogue=epilogue, residual=residual, block_n=256, sms=sms, splits=splits) is not None
+            symm_mem.check_status("cuda")
+            # a bf16 rounding is 2^-9 of the value (two with a residual); the sums of 5000 products of 0.05 differ by 1e-4
+            assert bool(((c.float() - want).abs() <= want.abs() * 2.0 ** -6 + 2e-2).all())
+            assert intact(), "the kernel stored outside its output"
+            assert splits < 0 or torch.equal(c, one)
 
 
 @pytest.mark.gpu
@@ -137,7 +143,7 @@ def test_a_record_is_of_the_kernel_that_runs(M, N, K, epilogue):
 
 @pytest.mark.gpu
 def test_split_calls_on_several_streams():
-    """Calls whose tiles are cut along K share neither scratch nor counters across streams."""
+    """Calls whose tiles are cut along K share no scratch across streams."""
     from symm_mem_recipes_b200.parallel import symm_mem
 
     cases = [_operands(M, 1280, 4096) for M in (64, 200, 500)]
