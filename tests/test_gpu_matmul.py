@@ -42,6 +42,7 @@ def test_matmul_small(block_n, shape):
 def test_matmul_column_panels(panel_w, shape):
     """The tile order in column panels (whole, uneven and single-tile panels, with and without the
     split-K tail) computes every tile exactly once: same bits as the one-panel order."""
+    from symm_mem_recipes_b200._ext import C
     from symm_mem_recipes_b200.ops.ag_matmul import AgMatmulConfig, matmul
     from symm_mem_recipes_b200.parallel import symm_mem
 
@@ -49,27 +50,38 @@ def test_matmul_column_panels(panel_w, shape):
     torch.manual_seed(M + N + K)
     a = (torch.randn(M, K, device="cuda") * 0.5).to(torch.bfloat16)
     b = (torch.randn(N, K, device="cuda") * 0.5).to(torch.bfloat16)
+
+    def run(c, split, panel_w):
+        if split:                                  # in two parts, for which K is too short otherwise
+            C.matmul_local(a, b, c, 0, None, 256, 12, True, panel_w, 2_000_000_000, -2)
+        else:
+            matmul(a, b, c, AgMatmulConfig(block_n=256, num_sms=12, split_k_tail=False, panel_w=panel_w, timeout_ms=2000))
+
+    assert C.matmul_plan(M, N, K, block_n=256, num_sms=12, max_splits=-2)[1] == 2    # 6 pairs: 15 and 20 tiles leave 3 and 2
     for split in (False, True):
         want = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
-        matmul(a, b, want, AgMatmulConfig(block_n=256, num_sms=8, split_k_tail=split, panel_w=1000, timeout_ms=2000))
+        run(want, split, 1000)
         c, intact = guarded_empty((M, N), torch.bfloat16, "cuda")
         c.fill_(float("nan"))
-        matmul(a, b, c, AgMatmulConfig(block_n=256, num_sms=8, split_k_tail=split, panel_w=panel_w, timeout_ms=2000))
+        run(c, split, panel_w)
         symm_mem.check_status("cuda")
         ok, err = _close(c, _ref(a, b), K)
         assert ok, f"max abs error {err}"
         assert intact(), "the kernel stored outside its output"
         if not split:
             assert torch.equal(c, want), "whole tiles: the order of the tiles must not change a bit"
+        else:                                      # which tiles are the last ones, and so cut, depends on the order
+            assert _close(c, want.float(), K)[0]
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("shape,num_sms", [((768, 768, 1024), 8), ((1280, 512, 512), 8), ((768, 768, 4096), 8),
-                                           ((16384, 3584, 1024), 0)])
+@pytest.mark.parametrize("shape,num_sms", [((768, 768, 4096), 8), ((1280, 512, 8192), 8), ((768, 768, 8192), 8),
+                                           ((16384, 3584, 8192), 0)])
 def test_matmul_split_k_tail(shape, num_sms):
     """Tile counts that leave a thin last wave: its tiles are cut along K and
     reduced through scratch memory; the result must not differ from the plain
     schedule by more than summation order."""
+    from symm_mem_recipes_b200._ext import C
     from symm_mem_recipes_b200.ops.ag_matmul import AgMatmulConfig, matmul
     from symm_mem_recipes_b200.parallel import symm_mem
 
@@ -78,6 +90,7 @@ def test_matmul_split_k_tail(shape, num_sms):
     a = (torch.randn(M, K, device="cuda") * 0.5).to(torch.bfloat16)
     b = (torch.randn(N, K, device="cuda") * 0.5).to(torch.bfloat16)
     outs = []
+    assert C.matmul_plan(M, N, K, num_sms=num_sms or torch.cuda.get_device_properties(0).multi_processor_count)[1] > 1
     for split in (True, False):
         c = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
         for _ in range(2):       # second call may find the scratch of the first

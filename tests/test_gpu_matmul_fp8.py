@@ -46,8 +46,11 @@ def test_matmul_fp8_small(block_n, shape):
     spawn_ranks(_mm_worker, 1, "nccl", (*shape, block_n, 0, True))
 
 
-@pytest.mark.parametrize("shape,num_sms", [((768, 768, 2048), 8), ((1280, 512, 1024), 8)])
+@pytest.mark.parametrize("shape,num_sms", [((768, 768, 8192), 8), ((1280, 512, 16384), 8)])
 def test_matmul_fp8_split_k_tail(shape, num_sms):
+    from symm_mem_recipes_b200._ext import C
+
+    assert C.matmul_plan(*shape, 1, num_sms=num_sms)[1] > 1
     spawn_ranks(_mm_worker, 1, "nccl", (*shape, 0, num_sms, True))
 
 

@@ -146,7 +146,10 @@ def test_split_calls_on_several_streams():
     """Calls whose tiles are cut along K share no scratch across streams."""
     from symm_mem_recipes_b200.parallel import symm_mem
 
-    cases = [_operands(M, 1280, 4096) for M in (64, 200, 500)]
+    from symm_mem_recipes_b200._ext import C
+
+    cases = [_operands(M, 1280, 4096) for M in (64, 200, 250)]
+    assert all(C.matmul_plan(*a.shape[:1], 1280, 4096, num_sms=48)[1] > 1 for a, _ in cases)
     want = [a.float() @ b.float().t() for a, b in cases]
     streams = [torch.cuda.Stream() for _ in cases]
     torch.cuda.synchronize()
