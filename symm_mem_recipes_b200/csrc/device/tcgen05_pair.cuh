@@ -75,15 +75,11 @@ enum class CollectA { kDiscard, kFill, kLastUse };
 template <bool kFp8, CollectA kCollect = CollectA::kDiscard>
 __device__ __forceinline__ void umma_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                                              uint32_t accumulate) {
-  if constexpr (kFp8) {
-    if constexpr (kCollect == CollectA::kFill) SMR_UMMA_PAIR("f8f6f4", ".collector::a::fill");
-    else if constexpr (kCollect == CollectA::kLastUse) SMR_UMMA_PAIR("f8f6f4", ".collector::a::lastuse");
-    else SMR_UMMA_PAIR("f8f6f4", "");
-  } else {
-    if constexpr (kCollect == CollectA::kFill) SMR_UMMA_PAIR("f16", ".collector::a::fill");
-    else if constexpr (kCollect == CollectA::kLastUse) SMR_UMMA_PAIR("f16", ".collector::a::lastuse");
-    else SMR_UMMA_PAIR("f16", "");
-  }
+  static_assert(!kFp8 || kCollect == CollectA::kDiscard, "two tiles at a time are bf16");
+  if constexpr (kFp8) SMR_UMMA_PAIR("f8f6f4", "");
+  else if constexpr (kCollect == CollectA::kFill) SMR_UMMA_PAIR("f16", ".collector::a::fill");
+  else if constexpr (kCollect == CollectA::kLastUse) SMR_UMMA_PAIR("f16", ".collector::a::lastuse");
+  else SMR_UMMA_PAIR("f16", "");
 }
 #undef SMR_UMMA_PAIR
 // One arrival on the barrier at this offset in BOTH CTAs of the pair once all
