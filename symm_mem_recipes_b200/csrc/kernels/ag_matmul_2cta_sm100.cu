@@ -682,16 +682,23 @@ size_t tail_scratch_bytes(int tiles, int parts, int bn) { return (size_t)tiles *
 // Units of two tiles (matmul_wide.cuh) that a GEMM of `rows` x `cols` tiles of 256 x 256 is multiplied in: as many whole
 // waves of them as there are, the rest one tile at a time.  bf16 only: in fp8 the same loads feed twice the flops, and
 // 4096 and 16384 x 3584 x 8192 take 95 and 362 us either way.  The end of a unit costs about 4000 cycles more than that
-// of two single tiles (both accumulators have to be read before the next unit), so K has to be long.  Loops of calls,
-// one tile at a time / two, us:
-//     16384 x 8192 x  1024  2048    16384 x 4096 x  4096  6144    16384 x 3584 x 8192    4096 x 7168 x 8192
-//               218/228  410/413              400/397  642/605                767/700               384/360
-//     with SwiGLU 9000 x 8192 x 4096  2048 x 7168 x 8192  32768 x 7168 x 8192
-//                            444/449             196/186            3020/2790
-//     with residual 16384 x 8192 x 2048  32768 x 8192 x 3584  16384 x 8192 x 7168   (one stage less one tile at a time)
-//                               447/469            1640/1592            1570/1466
-// An odd column of tiles comes after all units and reads all of A again: 8192 x 1280 x 8192 (5 columns) 142/141 but
-// 32768 x 1280 x 8192 535/560 and 32768 x 1792 x 8192 (7) 741/750; 32768 x 2304 x 8192 (9) 952/945.
+// of two single tiles (both accumulators have to be read before the next unit), so K has to be long.  Loops of calls at
+// 1000 W, all in one session, in turn: us (median SM clock, MHz) one tile at a time / two:
+//     16384 x 8192 x 1024    218 (1166) / 224 (1485)      16384 x 3584 x 8192    748 (1162) / 701 (1327)
+//     16384 x 8192 x 2048    404 (1297) / 410 (1402)       4096 x 7168 x 8192    377 (1237) / 359 (1342)
+//     16384 x 4096 x 4096    399 (1297) / 401 (1365)      16384 x 4096 x 6144    634 (1181) / 605 (1327)
+//   with SwiGLU (columns of C)
+//      9000 x 8192 x 4096    889 (1275) / 915 (1357)       2048 x 7168 x 8192    383 (1162) / 366 (1327)
+//                                                         32768 x 7168 x 8192   5830 (1095) / 5657 (1282)
+//   with residual (one stage less one tile at a time)
+//     16384 x 8192 x 2048    441 (1162) / 466 (1327)      32768 x 8192 x 3584   1617 (1027) / 1578 (1271)
+//                                                         16384 x 8192 x 7168   1539 (1087) / 1453 (1286)
+// An odd column of tiles comes after all units and reads all of A again:
+//      8192 x 1280 x 8192 (5 columns)  140 / 140          32768 x 1280 x 8192 (5)  530 / 549
+//     32768 x 1792 x 8192 (7)          736 / 740          32768 x 2304 x 8192 (9)  941 / 935
+// Single calls at a high clock (4 ms of pause before each, L2 cold), where power does not limit, lose nothing: 2048 x 5120
+// x 8192 118 / 118, 4096 x 3584 x 8192 159 / 159, 2048 x 8192 x 5120 120 / 119, 1024 x 7168 x 8192 with SwiGLU 165 / 161, with
+// residual 1280 x 8192 x 3584 71 / 69 and 2048 x 8192 x 3584 99 / 95, 16384 x 3584 x 8192 605 / 585.
 int plan_wide_units(int rows, int cols, int pairs, int K, int elem_bytes, bool residual) {
   if (elem_bytes != 2 || K < (residual ? 3072 : 5120) || (cols % 2 != 0 && cols < 9)) return 0;
   return rows * (cols / 2) / pairs * pairs;
@@ -709,8 +716,9 @@ int plan_wide_units(int rows, int cols, int pairs, int K, int elem_bytes, bool r
 // Where there are units of two tiles and K is 5120 or more, whole waves are priced at 0.94.  All of them, not only those of
 // units: that choice differs in 33 of 120000 random shapes, half of which are faster either way (9750 x 1312 x 5280 124 us, with
 // only the units' waves 116; 16363 x 1296 x 9304 372, 428).  The shorter K that units with a residual take is priced at 1: they save 2 to 3 %
-// there, less than 192 columns do where those fill the waves (1240 x 8192 x 3584 66.5 us, 256 columns 69.6).  The widths the plan picks are on average 0.3 % slower than the best
-// one of each shape, at worst 5 % (2992 x 6224 x 704: 27.6 us at 192 columns, 26.3 at 256).
+// there, less than 192 columns do where those fill the waves (1240 x 8192 x 3584 66.5 us, 256 columns 69.6).  On the shapes of
+// the fit and ten more the width that the plan picks is on average 0.1 % slower than the best one, at worst 3.8 % (148 x 1856 x
+// 7008: 13.2 us at 192 columns in parts, 12.7 at 128; then 2992 x 6224 x 704 with 1.6 %: 26.9 at 192, 26.5 at 256).
 // Examples, fp8, with the figures of before (fitted in short bursts) and now: 4096 x 3584 x 8192 103 -> 97 us (192 -> 256
 // columns), 16384 x 3584 x 8192 386 -> 362, 1024 x 8192 x 8192 65 -> 61; bf16 2992 x 6224 x 704 29.4 -> 27.6.
 MatmulPlan plan_matmul(int M, int N, int K, int elem_bytes, int epilogue, int block_n, int num_sms, int max_splits, bool residual) {

@@ -5,7 +5,8 @@
 // a time), so what counts is the energy of a flop and not the cycles.  Two tiles at once load 96 KB per 2 x 256 x 256 x 64
 // products instead of 128 (A once), and the tensor core takes A from its operand buffer for the second MMA
 // (`.collector::a`, 0.5 %).  Energy per flop at 16384 x 3584 x 8192, one tile of 128 columns at a time: 0.86 pJ, 192
-// columns 0.81, 256 columns 0.76, here 0.72.  At the full clock (operands of zeros) it takes 462 us against 458.
+// columns 0.81, 256 columns 0.76, here 0.72.  At the full clock (operands of zeros) it takes 462 us against 458; a single
+// call after a pause is no slower than one tile at a time (see plan_wide_units).
 //
 // Both accumulators (2 x 256 columns) fill TMEM, so there is no spare one to write while a tile is read.  Instead the two
 // are skewed against one another (kSkew): at either end of the K loop the first gets a few K blocks alone and the

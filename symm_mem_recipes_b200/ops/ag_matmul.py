@@ -254,6 +254,9 @@ def all_gather_matmul(a_shard: torch.Tensor, b: torch.Tensor, a_out: Optional[to
     `epilogue="swiglu"`: `b` is `interleave_gate_up(w_gate, w_up)` ([2F, K]) and
     the result is `SiLU(A @ w_gate^T) * (A @ w_up^T)`, [M, F], computed on the
     accumulators before they leave the SM (bf16, push gather or no gather).
+    Groups of 128 rows mean tiles of 256 columns.  The decoder layer on one rank
+    keeps gate and up as two halves instead, which a prompt of some hundred
+    tokens multiplies in narrower tiles (509 rows, K 8192, F 3584: 57 -> 53 µs).
 
     `trace`: an int64 CUDA tensor [num_sms, 12] that receives the per-CTA timing
     record of the GEMM kernel (`TRACE_FIELDS`; push gather or no gather).
