@@ -32,7 +32,8 @@ def test_gemv_tile_edges(B, K, N, nk):
 @pytest.mark.parametrize("n_layers,B,hidden,heads,kv,D,ffn,s_max,pos", [
     (1, 1, 512, 4, 1, 64, 512, 32, 0), (2, 3, 512, 8, 1, 128, 576, 40, 15), (1, 16, 1024, 8, 2, 128, 1536, 300, 257),
     (3, 5, 256, 3, 1, 64, 320, 4096, 4095), (1, 16, 512, 64, 16, 64, 512, 64, 40), (9, 2, 512, 4, 1, 128, 512, 64, 33),
-    (2, 2, 8192, 8, 1, 128, 3584, 2048, 1000)])
+    (2, 2, 8192, 8, 1, 128, 3584, 2048, 1000),
+    (1, 16, 512, 8, 1, 128, 512, 4100, 4097), (1, 16, 512, 2, 1, 64, 512, 4100, 4090)])   # five tiles of positions a warp
 def test_decode_step_matches_the_composition(n_layers, B, hidden, heads, kv, D, ffn, s_max, pos):
     """The persistent step against the layers composed of library GEMMs and PyTorch attention."""
     from symm_mem_recipes_b200.models.llama_tp_layer import LlamaTPConfig, LlamaTPDecoderLayer, decode_local

@@ -61,9 +61,11 @@ def test_swiglu_of_separate_and_interleaved_halves(M, F, K):
 @pytest.mark.parametrize("M,F,K", [(129, 7168, 2048), (509, 3584, 2048), (385, 6984, 1032)])
 def test_swiglu_in_narrower_tiles(M, F, K):
     """Sizes at which tiles of 112 gate and 112 up columns fill the pairs better; the last one ends inside a tile."""
+    from symm_mem_recipes_b200._ext import C
     from symm_mem_recipes_b200.parallel import symm_mem
     from symm_mem_recipes_b200.utils.testing import guarded_empty
 
+    assert C.matmul_plan(M, 2 * F, K, epilogue=2) == (224, 1, 0)
     a, b = _operands(M, 2 * F, K)
     g, u = (a.float() @ b.float().t()).split(F, dim=1)
     want = torch.nn.functional.silu(g) * u
