@@ -147,7 +147,7 @@ FUNCTIONS = [
     ("test_gpu_gemv", "test_gemv_world_of_one", {"B": 8, "K": 256, "N": 64, "algo": "simt"}),
     ("test_gpu_matmul_rs", "test_matmul_reduce_scatter_world_of_one", {}),
     ("test_gpu_llama_layer", "test_layer_world_of_one", {}),
-    ("test_gpu_matmul", "test_matmul_split_k_tail", {"shape": (768, 768, 1024), "num_sms": 8}),
+    ("test_gpu_matmul", "test_matmul_split_k_tail", {"shape": (768, 768, 4096), "num_sms": 8}),
 ]
 
 
